@@ -20,33 +20,9 @@
 // cut are added in the order of k by the CTA that finishes last (fp32 partials and an arrival counter in the scratch; no
 // CTA waits for another). Two accumulators in tensor memory: the
 // epilogue of a tile runs under the MMAs of the next. At decode sizes the kernel is a plain stream of W at HBM rate.
-#include "tpx_hybrid.cuh"
-#include "tpx_tc_ptx.cuh"
+#include "tpx_bf16_pair.cuh"
 
 namespace tpx {
-
-// Epilogue of tpx_linear: fp32 bias, row stride, fp32 or bf16 result, activation from a column on; gated units from pairs of
-// columns; or the residual sum with the norm of its next reader.
-struct BfEx {
-  const float *bias, *ap;
-  void* y;
-  long long ldy;
-  int on, out_f32, act, act_from;
-  uint16_t* z;
-  const float *res, *add, *nw, *nb;
-  float* x_out;
-  uint16_t* h;
-  long long ldz, ldr, ldh;
-  float limit, nalpha;
-};
-
-struct BfParams {
-  TcParams t;   // epilogue fields (bias, act, mul_in, res, res_scale, y, M, N, err)
-  int ksteps;   // k steps of 64 (K rounded up)
-  int TN, TM;   // feature tiles, token tiles
-  int split;    // 1: the CTAs share all pipeline stages of all tiles evenly; a tile cut between CTAs is put together by the last of them
-  BfEx ex;
-};
 
 // The stages a CTA works on, as pieces of tiles: piece = stages [g0, g1) of one tile.
 struct BfPieces {
@@ -360,7 +336,7 @@ linear_bf16_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
 }
 
 // 2-D bf16 tensor [rows][cols] (row stride ld elements), box = 64 columns x box_rows, 128-byte swizzle.
-static int bf_make_map(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows) {
+int bf_make_map(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows) {
   typedef CUresult (*Fn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
                          const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
   static Fn fn = nullptr;
@@ -415,6 +391,7 @@ static size_t bf_split_bytes(int64_t M, int grid) { return (size_t)grid * 2 * (M
 // Tiles, tensor maps and launch for a filled epilogue.
 static int bf_run(BfParams& p, const void* w, const void* x, int64_t M, int64_t N, int64_t K, int64_t ldw, int64_t ldx, void* scratch,
                   size_t scratch_bytes, cudaStream_t st) {
+  if (bf_pair_serves(p, M, N, K)) return bf_pair_run(p, w, x, M, N, K, ldw, ldx, st);
   p.split = bf_split_ctas(M, N, K);
   if (p.split && scratch_bytes < kTcCounterBytes + bf_split_bytes(M, p.split)) p.split = 0;
   p.t.counters = reinterpret_cast<unsigned*>(scratch);
