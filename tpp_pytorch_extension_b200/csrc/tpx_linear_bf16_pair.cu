@@ -4,13 +4,13 @@
 // 128 tokens. There a CTA multiplied 128 features by 256 tokens with three stages in flight, fetched 48 KB per 64 values of
 // k, and its lanes held features, so that every result left as a 2-byte store.
 // Here tokens are the rows of the MMA: a cluster of two CTAs computes 256 tokens x 256 features, each CTA holding its own 128
-// tokens of x and HALF of the weight tile (the hardware reads both halves for both CTAs), 32 KB per 64 values of k, six
+// tokens of x and HALF of the weight tile (the hardware reads both halves for both CTAs), 32 KB per 64 values of k, seven
 // stages deep. A lane of the epilogue owns one token and consecutive features: 16-byte loads and stores, gated units without
-// an exchange between lanes. Two accumulators of 256 columns fill tensor memory: the eight epilogue warps of a CTA work
-// under the next tile's MMAs. Clusters walk the tiles in blocks of eight token tiles, so that the tiles in flight at a time
+// an exchange between lanes. Two accumulators of 256 columns fill tensor memory: the sixteen epilogue warps of a CTA work
+// under the next tile's MMAs. Clusters walk the tiles in blocks of sixteen token tiles, so that the tiles in flight at a time
 // share their operands through L2.
 //   warp 0: TMA producer (both CTAs; copies complete on the first CTA's barrier)   warp 1: MMA issuer (first CTA)
-//   warps 2-9: epilogue, two per 32-lane quarter of tensor memory
+//   warps 2-17: epilogue, four per 32-lane quarter of tensor memory
 #include "tpx_bf16_pair.cuh"
 
 namespace tpx {
@@ -18,10 +18,11 @@ namespace tpx {
 struct BpCfg {
   static constexpr int HALF_BYTES = 128 * 128;  // 128 rows x 64 bf16
   static constexpr int STAGE_BYTES = 2 * HALF_BYTES;
-  static constexpr int STAGES = 6;
-  static constexpr int THREADS = 64 + 256;
-  static constexpr int EPI_WARPS = 8;
-  static constexpr int GROUP = 8;  // token tiles walked side by side
+  static constexpr int STAGES = 7;
+  static constexpr int EPI_WARPS = 16;             // four per 32-lane quarter of tensor memory
+  static constexpr int EPI_COLS = 1024 / EPI_WARPS;  // features per warp
+  static constexpr int THREADS = 64 + 32 * EPI_WARPS;
+  static constexpr int GROUP = 16;  // token tiles walked side by side (16384 x 14336 x 4096: 1210 us, with 8: 1231, with 4: 1270)
   static constexpr size_t SMEM = (size_t)STAGES * STAGE_BYTES + 1024;
 };
 
@@ -73,7 +74,8 @@ __device__ __forceinline__ void bp_ld8(const float* p, float (&o)[8]) {
   o[0] = a.x; o[1] = a.y; o[2] = a.z; o[3] = a.w; o[4] = b.x; o[5] = b.y; o[6] = b.z; o[7] = b.w;
 }
 __device__ __forceinline__ uint32_t bp_pack(float a, float b) {
-  return (uint32_t)f32_to_bf16_bits(a) | ((uint32_t)f32_to_bf16_bits(b) << 16);
+  const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<const uint32_t*>(&v);
 }
 __device__ __forceinline__ void bp_st8(uint16_t* p, const float (&v)[8]) {
   *reinterpret_cast<uint4*>(p) = make_uint4(bp_pack(v[0], v[1]), bp_pack(v[2], v[3]), bp_pack(v[4], v[5]), bp_pack(v[6], v[7]));
@@ -209,64 +211,74 @@ linear_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_co
   pdl_trigger();
 
   if (warp == 0) {
-    // ------------------------------------------------------------ producer (one thread in each CTA)
-    if (lane == 0) {
-      pdl_wait();
-      long long it = 0;
-      bool dead = false;
-      for (int t = cid; t < T && !dead; t += G) {
-        int tn, tm;
-        bp_tile(p, t, tn, tm);
-        const int row = tm * 256 + crank * 128, col = tn * 256 + crank * 128;
-        for (int g = 0; g < p.ksteps; g++, it++) {
-          const int s = (int)(it % C::STAGES);
-          if (it >= C::STAGES && !tc_wait(tc_smem_u32(&bar_empty[s]), (uint32_t)((it / C::STAGES - 1) & 1))) {
-            atomicExch(p.t.err, 2u);
-            dead = true;
-            break;
-          }
+    // ------------------------------------------------------------ producer (both CTAs)
+    pdl_wait();
+    int s = 0;
+    uint32_t phase = 1;  // parity to wait for on bar_empty: the first round over the ring finds every stage free
+    bool dead = false;
+    for (int t = cid; t < T && !dead; t += G) {
+      int tn, tm;
+      bp_tile(p, t, tn, tm);
+      const int row = tm * 256 + crank * 128, col = tn * 256 + crank * 128;
+      for (int g = 0; g < p.ksteps; g++) {
+        if (!tc_wait(tc_smem_u32(&bar_empty[s]), phase)) {
+          if (tc_elect()) atomicExch(p.t.err, 2u);
+          dead = true;
+          break;
+        }
+        if (tc_elect()) {
           const uint32_t st = smem_base + (uint32_t)s * C::STAGE_BYTES;
           const uint32_t lbar = tc_mapa(tc_smem_u32(&bar_full[s]), 0u);  // the first CTA's barrier
           if (crank == 0) tc_mbar_expect_tx(tc_smem_u32(&bar_full[s]), 2u * C::STAGE_BYTES);
           bp_tma_2d(st, &tmX, g * 64, row, lbar);
           bp_tma_2d(st + C::HALF_BYTES, &tmW, g * 64, col, lbar);
         }
+        __syncwarp();
+        if (++s == C::STAGES) s = 0, phase ^= 1u;
       }
     }
-    __syncwarp();
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (first CTA only)
-    if (lane == 0 && crank == 0) {
+    if (crank == 0) {
       // kind::f16: D = F32 (1), A = B = BF16 (1), both K-major, N = 256, M = 256 over the pair
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(256 >> 3) << 17) | ((256u >> 4) << 24);
-      long long it = 0;
+      const uint64_t desc0 = tc_smem_desc(smem_base);
+      int s = 0, i = 0;
+      uint32_t phase = 0;
       bool dead = false;
-      int i = 0;
       for (int t = cid; t < T && !dead; t += G, i++) {
         const int buf = i & 1;
         if (i >= 2) {  // both CTAs' epilogue warps have drained this accumulator
-          if (!bp_wait_cluster(tc_smem_u32(&acc_empty[buf]), (uint32_t)((i / 2 - 1) & 1))) { atomicExch(p.t.err, 3u); break; }
+          if (!bp_wait_cluster(tc_smem_u32(&acc_empty[buf]), (uint32_t)((i / 2 - 1) & 1))) {
+            if (tc_elect()) atomicExch(p.t.err, 3u);
+            break;
+          }
           tc_fence_after();
         }
-        for (int g = 0; g < p.ksteps; g++, it++) {
-          const int s = (int)(it % C::STAGES);
-          if (!tc_wait(tc_smem_u32(&bar_full[s]), (uint32_t)((it / C::STAGES) & 1))) { atomicExch(p.t.err, 4u); dead = true; break; }
+        for (int g = 0; g < p.ksteps; g++) {
+          if (!tc_wait(tc_smem_u32(&bar_full[s]), phase)) {
+            if (tc_elect()) atomicExch(p.t.err, 4u);
+            dead = true;
+            break;
+          }
           tc_fence_after();
-          const uint32_t st = smem_base + (uint32_t)s * C::STAGE_BYTES;
+          if (tc_elect()) {
+            const uint64_t desc = desc0 + (uint64_t)(s * (C::STAGE_BYTES >> 4));  // descriptors count 16-byte units
 #pragma unroll
-          for (int j = 0; j < 4; j++)
-            bp_mma(tmem + buf * 256, tc_smem_desc(st) + (uint64_t)(2 * j), tc_smem_desc(st + C::HALF_BYTES) + (uint64_t)(2 * j), idesc,
-                   (g == 0 && j == 0) ? 0u : 1u);
-          bp_commit_both(tc_smem_u32(&bar_empty[s]));
+            for (int j = 0; j < 4; j++)
+              bp_mma(tmem + buf * 256, desc + (uint64_t)(2 * j), desc + (uint64_t)((C::HALF_BYTES >> 4) + 2 * j), idesc, (g | j) ? 1u : 0u);
+            bp_commit_both(tc_smem_u32(&bar_empty[s]));
+            if (g == p.ksteps - 1) bp_commit_both(tc_smem_u32(&acc_full[buf]));
+          }
+          __syncwarp();
+          if (++s == C::STAGES) s = 0, phase ^= 1u;
         }
-        if (!dead) bp_commit_both(tc_smem_u32(&acc_full[buf]));
       }
     }
-    __syncwarp();
   } else {
-    // ------------------------------------------------------------ epilogue (warps 2 .. 9 of both CTAs)
+    // ------------------------------------------------------------ epilogue (warps 2 .. 17 of both CTAs)
     const int sub = warp & 3;  // tensor-memory lanes 32*sub .. 32*sub+31 belong to this warp
-    const int c_first = ((warp - 2) >> 2) * 128;
+    const int c_first = ((warp - 2) >> 2) * C::EPI_COLS;
     const uint32_t lane_base = ((uint32_t)(sub * 32)) << 16;
     pdl_wait();  // residual and multiplier inputs belong to earlier grids
     int i = 0;
@@ -282,7 +294,7 @@ linear_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_co
       const long long row = (long long)tm * 256 + crank * 128 + sub * 32 + lane;
       const int n0 = tn * 256 + c_first;
 #pragma unroll 1
-      for (int c = 0; c < 128 && n0 + c < p.t.N; c += 16) {
+      for (int c = 0; c < C::EPI_COLS && n0 + c < p.t.N; c += 16) {
         uint32_t a[16];
         tc_ld_x16(tmem + lane_base + (uint32_t)(buf * 256 + c_first + c), a);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");

@@ -67,6 +67,15 @@ __device__ __forceinline__ void tc_stamp(const TcParams&, int) {}
 // ---------------------------------------------------------------- PTX wrappers
 __device__ __forceinline__ uint32_t tc_smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
+// True in one lane of a converged warp. A warp that issues tcgen05.mma or TMA copies runs its loops with all lanes and issues
+// under this predicate: the compiler then knows loop state and descriptors to be warp-uniform and keeps them in uniform
+// registers. Behind `if (lane == 0)` every operand of every MMA is moved there one by one, and the issuing thread, not the tensor
+// core, sets the pace (bf16 pair kernel, 16384 x 14336 x 4096: 1463 us with the branch, 1231 us with the predicate).
+__device__ __forceinline__ bool tc_elect() {
+  uint32_t p;
+  asm volatile("{ .reg .pred p; elect.sync _|p, 0xffffffff; selp.u32 %0, 1, 0, p; }" : "=r"(p));
+  return p != 0;
+}
 __device__ __forceinline__ void tc_mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
 }
