@@ -141,7 +141,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
 
   if (warp == 0) {
     // ------------------------------------------------------------ producer
-    if (lane == 0) {
+    if (tc_elect()) {
       tc_mbar_expect_tx(tc_smem_u32(&q_full), C::Q_BYTES);
 #pragma unroll
       for (int h = 0; h < C::HALVES; h++) tc_tma_2d(q_s + h * C::HALF_BYTES, &tmQ, h * 64, bn * rows_total + row0, tc_smem_u32(&q_full));
@@ -161,7 +161,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     __syncwarp();
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (tc_elect()) {
       const uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((128u >> 3) << 17) | ((128u >> 4) << 24);
       const uint32_t idesc_t = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((uint32_t)(H >> 3) << 17) | ((128u >> 4) << 24);
       bool ok = tc_wait(tc_smem_u32(&q_full), 0);

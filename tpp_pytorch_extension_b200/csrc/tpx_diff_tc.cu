@@ -189,7 +189,7 @@ diff_attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   const int ntiles = last_r >= first ? last_r / 128 + 1 - j0 : 0;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (tc_elect()) {
       tc_mbar_expect_tx(tc_smem_u32(&q_full), C::Q_BYTES);
 #pragma unroll
       for (int m = 0; m < 2; m++)
@@ -216,7 +216,7 @@ diff_attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0 && ntiles > 0) {
+    if (ntiles > 0 && tc_elect()) {
       const uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((128u >> 3) << 17) | ((128u >> 4) << 24);
       const uint32_t idesc_o = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((uint32_t)(VS * 64 >> 3) << 17) | ((128u >> 4) << 24);
       bool ok = tc_wait(tc_smem_u32(&q_full), 0);

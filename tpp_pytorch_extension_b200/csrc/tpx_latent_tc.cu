@@ -135,7 +135,7 @@ latent_attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   const int ntiles = kmax > kmin ? (kmax + 127) / 128 - j0 : 0;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (tc_elect()) {
       tc_mbar_expect_tx(tc_smem_u32(&q_full), C::Q_BYTES);
 #pragma unroll
       for (int h = 0; h < QS; h++)
@@ -160,7 +160,7 @@ latent_attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (tc_elect()) {
       const uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((128u >> 3) << 17) | ((128u >> 4) << 24);
       const uint32_t idesc_t = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((uint32_t)(VS * 64 >> 3) << 17) | ((128u >> 4) << 24);
       bool ok = tc_wait(tc_smem_u32(&q_full), 0);

@@ -172,7 +172,7 @@ linear_bf16_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
 
   if (warp == 0) {
     // ------------------------------------------------------------ producer
-    if (lane == 0) {
+    if (tc_elect()) {
       // at decode sizes W is a model's weight, not the output of a kernel in flight: its copies for the first stages need not
       // wait for the kernels that make x (many rows may come with a weight unpacked for the call)
       auto copy_w = [&](int tile, int g, int s) {
@@ -214,7 +214,7 @@ linear_bf16_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     __syncwarp();
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (tc_elect()) {
       // kind::f16: D = F32 (1), A = B = BF16 (1), both K-major, N = TOK, M = 128
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TOK >> 3) << 17) | ((128u >> 4) << 24);
       long long it = 0;

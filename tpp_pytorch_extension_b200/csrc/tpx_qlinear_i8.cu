@@ -273,7 +273,7 @@ qlinear_i8_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
 
   if (warp == 0) {
     // ------------------------------------------------------------ producer
-    if (lane == 0) {
+    if (tc_elect()) {
       auto fetch_w = [&](int s, int ks) {
         const uint32_t st = smem_base + (uint32_t)s * C::STAGE_BYTES;
         tc_mbar_expect_tx(tc_smem_u32(&bar_full[s]), C::A_BYTES + C::B_BYTES);
@@ -294,7 +294,7 @@ qlinear_i8_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
     __syncwarp();
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (tc_elect()) {
       // kind::i8: D = S32 (2), A = B = S8 (1), both K-major, N = TOK, M = 128
       const uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TOK >> 3) << 17) | ((128u >> 4) << 24);
       int buf = 0, inblk = 0;  // accumulator in use, k32 steps already in the current scale block

@@ -288,7 +288,7 @@ qlinear_tc4_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
 
   if (warp == 0) {
     // ------------------------------------------------------------ producer
-    if (lane == 0) {
+    if (tc_elect()) {
       auto fetch_w = [&](int s, int tn, int ks) {  // weight tiles and their scale blocks: independent of the split kernel
         const uint32_t st = smem_base + (uint32_t)s * C::STAGE_BYTES;
         const uint32_t bar = tc_smem_u32(&bar_full[s]);
@@ -349,7 +349,7 @@ qlinear_tc4_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     __syncwarp();
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (tc_elect()) {
       // instruction descriptor: A = B = E2M1 (1 in this kind), both K-major, N = 4*TOK, UE8M0 scales, M = 128, K = 64
       const uint32_t idesc0 = (1u << 7) | (1u << 10) | ((uint32_t)(C::NCOL >> 3) << 17) | (1u << 23) | ((128u >> 4) << 24);
       int ks = ks0;
@@ -409,7 +409,7 @@ qlinear_tc4_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     // ------------------------------------------------------------ scale-factor copies (shared -> tensor memory)
     // Issued by their own thread so that they are not queued in order between the MMAs; a stage's tensor-memory
     // columns are free again once its shared memory has been refilled (the refill waits for the stage's MMAs).
-    if (lane == 0 && !(TPX_DBG(p) & 48)) {
+    if (!(TPX_DBG(p) & 48) && tc_elect()) {
       for (int it = 0; it < nunits; it++) {
         const int s = it % C::STAGES;
         const uint32_t ph = (uint32_t)((it / C::STAGES) & 1);

@@ -94,7 +94,7 @@ qlinear_tcp_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
 
   if (warp == 0) {
     // ------------------------------------------------------------ producer
-    if (lane == 0) {
+    if (tc_elect()) {
       auto fetch_w = [&](int s, int tn, int d, int ku) {  // weights and their scale blocks: independent of earlier kernels
         const uint32_t st = smem_base + (uint32_t)s * C::STAGE_BYTES;
         const uint32_t bar = tc_smem_u32(&bar_full[s]);
@@ -154,7 +154,7 @@ qlinear_tcp_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     __syncwarp();
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (tc_elect()) {
       // instruction descriptor: A = E2M1 (5), B = E4M3 (0), both K-major, N = 128, UE8M0 scales, M = 128
       const uint32_t idesc0 = (5u << 7) | (0u << 10) | ((uint32_t)(128 >> 3) << 17) | (1u << 23) | ((128u >> 4) << 24);
       for (int it = 0; it < nunits; it++) {

@@ -277,7 +277,7 @@ qlinear_tcp2_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
     // ------------------------------------------------------------ weight producer (one thread in each CTA)
     // Issuing a stage's copies takes one thread about as long as the stage's MMAs run, so the weights and the
     // activation terms have a producer thread each.
-    if (lane == 0) {
+    if (tc_elect()) {
       for (int it = 0; it < nunits; it++) {
         const int s = it % C::STAGES;
         int tn, tm, d, ku;
@@ -309,7 +309,7 @@ qlinear_tcp2_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
     __syncwarp();
   } else if (warp == 2) {
     // ------------------------------------------------------------ activation producer (one thread in each CTA)
-    if (lane == 0) {
+    if (tc_elect()) {
       pdl_wait();  // the activation terms belong to the split kernel until it has completed
       for (int it = 0; it < nunits; it++) {
         const int s = it % C::STAGES;
@@ -333,7 +333,7 @@ qlinear_tcp2_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
     __syncwarp();
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (first CTA only)
-    if (lane == 0 && crank == 0) {
+    if (crank == 0 && tc_elect()) {
       // instruction descriptor: A = E2M1 (5), B = E4M3 (0), both K-major, N = 256, UE8M0 scales, M = 256 over the pair
       const uint32_t idesc0 = ((p.wfmt == 0 ? 5u : p.wfmt == 1 ? 0u : 1u) << 7) | (0u << 10) | ((uint32_t)(256 >> 3) << 17) | (1u << 23) | ((256u >> 4) << 24);
       for (int it = 0; it < nunits; it++) {

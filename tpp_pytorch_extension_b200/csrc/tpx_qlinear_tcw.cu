@@ -210,7 +210,7 @@ qlinear_tcw_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
 
   if (warp == 0) {
     // ------------------------------------------------------------ producer
-    if (lane == 0) {
+    if (tc_elect()) {
       auto fetch_w = [&](int s, int t, int ks) {
         const uint32_t st = smem_base + (uint32_t)s * C::STAGE_BYTES;
         const uint32_t bar = tc_smem_u32(&bar_full[s]);
@@ -283,7 +283,7 @@ qlinear_tcw_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     __syncwarp();
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (tc_elect()) {
       // A = E4M3 (0), B = E2M1 (5), both K-major, N = 256, UE8M0 scales, M = 128
       const uint32_t idesc0 = (0u << 7) | ((p.wfmt == 0 ? 5u : p.wfmt == 1 ? 0u : 1u) << 10) | ((256u >> 3) << 17) | (1u << 23) | ((128u >> 4) << 24);
       int ks = ks0;

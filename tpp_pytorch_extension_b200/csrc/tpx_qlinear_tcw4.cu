@@ -396,7 +396,7 @@ qlinear_tcw4_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
 
   if (warp == 0) {
     // ------------------------------------------------------------ producer
-    if (lane == 0) {
+    if (tc_elect()) {
       auto fetch_w = [&](int s, int t, int ks) {
         const uint32_t st = stage0 + (uint32_t)s * C::STAGE_BYTES;
         const uint32_t bar = tc_smem_u32(&bar_full[s]);
@@ -449,7 +449,7 @@ qlinear_tcw4_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
     __syncwarp();
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (tc_elect()) {
       // kind::mxf4: A = B = E2M1 (1), both K-major, N = 256, UE8M0 scales, M = 128, K = 64
       const uint32_t idesc0 = (1u << 7) | (1u << 10) | ((256u >> 3) << 17) | (1u << 23) | ((128u >> 4) << 24);
       bool ok = true;
