@@ -88,11 +88,13 @@ def _int8_tc(x, y, w, w2, bias, act, mul_in, res, res_scale, norm=None):
 
 def bf16_linear_scratch(M):
     """Scratch of the bf16 linear for M rows and any weight: one size for all shapes, so that the buffer does not grow
-    between the layers of a step."""
-    key = ("bf16", 64 if M <= 64 else 0)
+    between the layers of a step. (The many-token kernel's buffer for cut tiles has one size, and 129 rows, one tile, cut it.)"""
+    rows = 64 if M <= 64 else 128 if M <= 128 else 0
+    key = ("bf16", rows)
     nb = _SCRATCH_BYTES.get(key)
     if nb is None:
-        nb = _SCRATCH_BYTES[key] = max(_lib.lib().tpx_linear_bf16_tc_scratch_bytes(key[1] or 65, n, 4096) for n in (128, 128 * 149))
+        f = _lib.lib().tpx_linear_bf16_tc_scratch_bytes
+        nb = _SCRATCH_BYTES[key] = max(f(rows, n, 4096) for n in (128, 128 * 149)) if rows else f(129, 256, 4096)
     return nb
 
 

@@ -36,11 +36,24 @@ def _call(name, st):
         _lib.check(rc)
 
 
+_F32_SCRATCH = {}
+
+
+def _f32_linear_scratch(M, N, K):
+    key = (M, N, K)
+    nb = _F32_SCRATCH.get(key)
+    if nb is None:
+        if len(_F32_SCRATCH) > 4096:
+            _F32_SCRATCH.clear()
+        nb = _F32_SCRATCH[key] = max(_lib.lib().tpx_linear_f32_scratch_bytes(M, N, K), 65536)
+    return nb
+
+
 def _linear_call(x, w, y, bias=None, **fields):
     M, (N, K) = x.shape[0], w.shape
     if x.dtype != w.dtype or x.shape[1] != K:
         raise _lib.TpxError(f"linear: input {tuple(x.shape)} {x.dtype} does not fit the weight {tuple(w.shape)} {w.dtype}")
-    sc = _lib.scratch(bf16_linear_scratch(M), x.device)
+    sc = _lib.scratch(_f32_linear_scratch(M, N, K) if w.dtype == torch.float32 else bf16_linear_scratch(M), x.device)
     _call("tpx_linear", _lib.LinearStruct(
         w=w.data_ptr(), x=x.data_ptr(), bias=_lib.ptr(bias), y=_lib.ptr(y), M=M, N=N, K=K, ldw=w.stride(0), ldx=x.stride(0),
         ldy=y.stride(0) if y is not None else 0, f32=int(w.dtype == torch.float32), out_f32=int(y is not None and y.dtype == torch.float32),

@@ -42,6 +42,7 @@ _SIGS = {
     "tpx_qlinear_qint8_tc": (c_int, [c_vp, c_vp, c_vp, c_vp, c_int, c_f32, c_i64, c_i64, c_i64, c_i64, c_int, c_vp, c_int, c_vp, c_vp, c_f32,
                                      c_vp, c_vp, c_sz, c_vp]),
     "tpx_linear_bf16_tc_scratch_bytes": (c_sz, [c_i64, c_i64, c_i64]),
+    "tpx_linear_f32_scratch_bytes": (c_sz, [c_i64, c_i64, c_i64]),
     "tpx_linear_bf16_tc": (c_int, [c_vp, c_vp, c_i64, c_i64, c_i64, c_vp, c_int, c_vp, c_vp, c_f32, c_vp, c_vp, c_sz, c_vp]),
     "tpx_allreduce_flag_bytes": (c_sz, []),
     "tpx_allreduce_bf16": (c_int, [c_vp, c_i64, c_int, c_int, c_vp, c_vp, c_vp, c_i64, c_vp]),
@@ -236,11 +237,13 @@ _scratch = {}
 
 
 def scratch(nbytes, device):
-    """Per-device, per-stream zero-initialised scratch for split-K partial sums, grown on demand."""
+    """Per-device, per-stream scratch of the linears, grown on demand: arrival counters and the error word in its first
+    64 KiB, which start at zero, then partial sums and the like, which need no initial state."""
     key = (device.index, stream())
     buf = _scratch.get(key)
     if buf is None or buf.numel() < nbytes:
-        buf = torch.zeros(max(nbytes, 1 << 20), dtype=torch.uint8, device=device)
+        buf = torch.empty(max(nbytes, 1 << 20), dtype=torch.uint8, device=device)
+        buf[:65536].zero_()
         _scratch[key] = buf
     return buf
 

@@ -391,7 +391,7 @@ static size_t bf_split_bytes(int64_t M, int grid) { return (size_t)grid * 2 * (M
 // Tiles, tensor maps and launch for a filled epilogue.
 static int bf_run(BfParams& p, const void* w, const void* x, int64_t M, int64_t N, int64_t K, int64_t ldw, int64_t ldx, void* scratch,
                   size_t scratch_bytes, cudaStream_t st) {
-  if (bf_pair_serves(p, M, N, K)) return bf_pair_run(p, w, x, M, N, K, ldw, ldx, st);
+  if (bf_pair_serves(p, M, N, K)) return bf_pair_run(p, w, x, M, N, K, ldw, ldx, scratch, scratch_bytes, st);
   p.split = bf_split_ctas(M, N, K);
   if (p.split && scratch_bytes < kTcCounterBytes + bf_split_bytes(M, p.split)) p.split = 0;
   p.t.counters = reinterpret_cast<unsigned*>(scratch);
@@ -434,6 +434,7 @@ using namespace tpx;
 
 extern "C" size_t tpx_linear_bf16_tc_scratch_bytes(int64_t M, int64_t N, int64_t K) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
+  if (M > 128) return bf_pair_scratch_bytes(M, N, K);
   const int grid = bf_split_ctas(M, N, K);
   return kTcCounterBytes + (grid ? bf_split_bytes(M, grid) : 0);
 }

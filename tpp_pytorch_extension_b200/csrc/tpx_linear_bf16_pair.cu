@@ -19,71 +19,9 @@ struct BpCfg {
   static constexpr int HALF_BYTES = 128 * 128;  // 128 rows x 64 bf16
   static constexpr int STAGE_BYTES = 2 * HALF_BYTES;
   static constexpr int STAGES = 7;
-  static constexpr int EPI_WARPS = 16;             // four per 32-lane quarter of tensor memory
-  static constexpr int EPI_COLS = 1024 / EPI_WARPS;  // features per warp
-  static constexpr int THREADS = 64 + 32 * EPI_WARPS;
-  static constexpr int GROUP = 16;  // token tiles walked side by side (16384 x 14336 x 4096: 1210 us, with 8: 1231, with 4: 1270)
+  static constexpr int THREADS = 64 + 32 * kBpEpiWarps;
   static constexpr size_t SMEM = (size_t)STAGES * STAGE_BYTES + 1024;
 };
-
-__device__ __forceinline__ void bp_tma_2d(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t cluster_bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
-      "l"(map), "r"(c0), "r"(c1), "r"(cluster_bar)
-      : "memory");
-}
-__device__ __forceinline__ void bp_mma(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{ .reg .pred p; setp.ne.b32 p, %4, 0;\n"
-      "  tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p; }" ::"r"(d_tmem),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-__device__ __forceinline__ void bp_commit_both(uint32_t bar) {  // arrives on the barrier at this offset in both CTAs
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
-               "h"((uint16_t)3)
-               : "memory");
-}
-__device__ __forceinline__ void bp_arrive_cluster(uint32_t cluster_bar) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
-}
-__device__ __forceinline__ bool bp_wait_cluster(uint32_t bar, uint32_t parity) {  // arrivals come from both CTAs
-  for (unsigned spins = 0; spins < kTcSpinLimit; spins++) {
-    uint32_t ok;
-    asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
-                 : "=r"(ok)
-                 : "r"(bar), "r"(parity)
-                 : "memory");
-    if (ok) return true;
-  }
-  return false;
-}
-
-// Eight consecutive values; the caller guarantees 16-byte alignment.
-__device__ __forceinline__ void bp_ld8(const uint16_t* p, float (&o)[8]) {
-  const uint4 v = *reinterpret_cast<const uint4*>(p);
-  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-  for (int j = 0; j < 4; j++) {
-    o[2 * j] = __uint_as_float(w[j] << 16);
-    o[2 * j + 1] = __uint_as_float(w[j] & 0xffff0000u);
-  }
-}
-__device__ __forceinline__ void bp_ld8(const float* p, float (&o)[8]) {
-  const float4 a = reinterpret_cast<const float4*>(p)[0], b = reinterpret_cast<const float4*>(p)[1];
-  o[0] = a.x; o[1] = a.y; o[2] = a.z; o[3] = a.w; o[4] = b.x; o[5] = b.y; o[6] = b.z; o[7] = b.w;
-}
-__device__ __forceinline__ uint32_t bp_pack(float a, float b) {
-  const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
-  return *reinterpret_cast<const uint32_t*>(&v);
-}
-__device__ __forceinline__ void bp_st8(uint16_t* p, const float (&v)[8]) {
-  *reinterpret_cast<uint4*>(p) = make_uint4(bp_pack(v[0], v[1]), bp_pack(v[2], v[3]), bp_pack(v[4], v[5]), bp_pack(v[6], v[7]));
-}
-__device__ __forceinline__ void bp_st8(float* p, const float (&v)[8]) {
-  reinterpret_cast<float4*>(p)[0] = make_float4(v[0], v[1], v[2], v[3]);
-  reinterpret_cast<float4*>(p)[1] = make_float4(v[4], v[5], v[6], v[7]);
-}
 
 // Features n .. n+7 of one token.
 __device__ __forceinline__ void bp_finish8(const BfParams& p, long long row, int n, float (&x)[8]) {
@@ -164,15 +102,6 @@ __device__ __forceinline__ void bp_finish8(const BfParams& p, long long row, int
   else bp_st8(reinterpret_cast<uint16_t*>(e.y) + row * e.ldy + n, x);
 }
 
-// Tile t of the walk: blocks of GROUP token tiles, inside a block the token tiles of one feature tile are neighbours.
-__device__ __forceinline__ void bp_tile(const BfParams& p, int t, int& tn, int& tm) {
-  const int per = BpCfg::GROUP * p.TN;
-  const int g0 = t / per * BpCfg::GROUP, in = t % per;
-  const int rows = min(BpCfg::GROUP, p.TM - g0);
-  tn = in / rows;
-  tm = g0 + in % rows;
-}
-
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(BpCfg::THREADS, 1)
 linear_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, BfParams p) {
   using C = BpCfg;
@@ -180,11 +109,11 @@ linear_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_co
   __shared__ __align__(8) unsigned long long bar_full[C::STAGES], bar_empty[C::STAGES];
   __shared__ __align__(8) unsigned long long acc_full[2], acc_empty[2];
   __shared__ uint32_t tmem_holder;
+  __shared__ int last_piece;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t smem_base = (tc_smem_u32(bp_smem_raw) + 1023u) & ~1023u;
   const int crank = (int)tc_cluster_rank();  // 0: issues the MMAs and owns the barriers the copies complete on
-  const int T = p.TN * p.TM, G = gridDim.x / 2, cid = blockIdx.x / 2;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::STAGES; s++) {
@@ -193,7 +122,7 @@ linear_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_co
     }
     for (int b = 0; b < 2; b++) {
       tc_mbar_init(tc_smem_u32(&acc_full[b]), 1);
-      tc_mbar_init(tc_smem_u32(&acc_empty[b]), 2 * C::EPI_WARPS);  // the epilogue warps of both CTAs
+      tc_mbar_init(tc_smem_u32(&acc_empty[b]), 2 * kBpEpiWarps);  // the epilogue warps of both CTAs
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -216,11 +145,9 @@ linear_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_co
     int s = 0;
     uint32_t phase = 1;  // parity to wait for on bar_empty: the first round over the ring finds every stage free
     bool dead = false;
-    for (int t = cid; t < T && !dead; t += G) {
-      int tn, tm;
-      bp_tile(p, t, tn, tm);
-      const int row = tm * 256 + crank * 128, col = tn * 256 + crank * 128;
-      for (int g = 0; g < p.ksteps; g++) {
+    for (BpWork k(p); !dead && k.next();) {
+      const int row = k.tm * 256 + crank * 128, col = k.tn * 256 + crank * 128;
+      for (int g = k.g0; g < k.g1; g++) {
         if (!tc_wait(tc_smem_u32(&bar_empty[s]), phase)) {
           if (tc_elect()) atomicExch(p.t.err, 2u);
           dead = true;
@@ -246,7 +173,7 @@ linear_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_co
       int s = 0, i = 0;
       uint32_t phase = 0;
       bool dead = false;
-      for (int t = cid; t < T && !dead; t += G, i++) {
+      for (BpWork k(p); !dead && k.next(); i++) {
         const int buf = i & 1;
         if (i >= 2) {  // both CTAs' epilogue warps have drained this accumulator
           if (!bp_wait_cluster(tc_smem_u32(&acc_empty[buf]), (uint32_t)((i / 2 - 1) & 1))) {
@@ -255,7 +182,7 @@ linear_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_co
           }
           tc_fence_after();
         }
-        for (int g = 0; g < p.ksteps; g++) {
+        for (int g = k.g0; g < k.g1; g++) {
           if (!tc_wait(tc_smem_u32(&bar_full[s]), phase)) {
             if (tc_elect()) atomicExch(p.t.err, 4u);
             dead = true;
@@ -266,9 +193,10 @@ linear_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_co
             const uint64_t desc = desc0 + (uint64_t)(s * (C::STAGE_BYTES >> 4));  // descriptors count 16-byte units
 #pragma unroll
             for (int j = 0; j < 4; j++)
-              bp_mma(tmem + buf * 256, desc + (uint64_t)(2 * j), desc + (uint64_t)((C::HALF_BYTES >> 4) + 2 * j), idesc, (g | j) ? 1u : 0u);
+              bp_mma(tmem + buf * 256, desc + (uint64_t)(2 * j), desc + (uint64_t)((C::HALF_BYTES >> 4) + 2 * j), idesc,
+                     (g > k.g0 || j) ? 1u : 0u);
             bp_commit_both(tc_smem_u32(&bar_empty[s]));
-            if (g == p.ksteps - 1) bp_commit_both(tc_smem_u32(&acc_full[buf]));
+            if (g == k.g1 - 1) bp_commit_both(tc_smem_u32(&acc_full[buf]));
           }
           __syncwarp();
           if (++s == C::STAGES) s = 0, phase ^= 1u;
@@ -278,40 +206,60 @@ linear_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_co
   } else {
     // ------------------------------------------------------------ epilogue (warps 2 .. 17 of both CTAs)
     const int sub = warp & 3;  // tensor-memory lanes 32*sub .. 32*sub+31 belong to this warp
-    const int c_first = ((warp - 2) >> 2) * C::EPI_COLS;
+    const int c_first = ((warp - 2) >> 2) * kBpEpiCols;
     const uint32_t lane_base = ((uint32_t)(sub * 32)) << 16;
     pdl_wait();  // residual and multiplier inputs belong to earlier grids
     int i = 0;
-    for (int t = cid; t < T; t += G, i++) {
+    bool dead = false;  // a warp that gave up still meets the others at their barriers
+    for (BpWork k(p); k.next(); i++) {
       const int buf = i & 1;
-      if (!tc_wait(tc_smem_u32(&acc_full[buf]), (uint32_t)((i / 2) & 1))) {
+      if (!dead && !tc_wait(tc_smem_u32(&acc_full[buf]), (uint32_t)((i / 2) & 1))) {
         if (lane == 0) atomicExch(p.t.err, 6u);
-        break;
+        dead = true;
       }
       tc_fence_after();
-      int tn, tm;
-      bp_tile(p, t, tn, tm);
-      const long long row = (long long)tm * 256 + crank * 128 + sub * 32 + lane;
-      const int n0 = tn * 256 + c_first;
+      const long long row = (long long)k.tm * 256 + crank * 128 + sub * 32 + lane;
+      const int n0 = k.tn * 256 + c_first;
+      const bool whole = k.whole();
+      float* part = bp_part(p, blockIdx.x, warp - 2) + lane;
+      auto finish = [&](int c, float (&v)[16]) {
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          float x[8];
+#pragma unroll
+          for (int j = 0; j < 8; j++) x[j] = v[h * 8 + j];
+          if (row < p.t.M && n0 + c + h * 8 < p.t.N) bp_finish8(p, row, n0 + c + h * 8, x);
+        }
+      };
 #pragma unroll 1
-      for (int c = 0; c < C::EPI_COLS && n0 + c < p.t.N; c += 16) {
+      for (int c = 0; c < kBpEpiCols && n0 + c < p.t.N && !dead; c += 16) {
         uint32_t a[16];
+        float v[16];
         tc_ld_x16(tmem + lane_base + (uint32_t)(buf * 256 + c_first + c), a);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        if (row < p.t.M) {
 #pragma unroll
-          for (int h = 0; h < 2; h++) {
-            float x[8];
+        for (int j = 0; j < 16; j++) v[j] = __uint_as_float(a[j]);
+        if (whole) finish(c, v);
+        else {
 #pragma unroll
-            for (int j = 0; j < 8; j++) x[j] = __uint_as_float(a[h * 8 + j]);
-            if (n0 + c + h * 8 < p.t.N) bp_finish8(p, row, n0 + c + h * 8, x);
-          }
+          for (int j = 0; j < 16; j++) part[(c + j) * 32] = v[j];
         }
         __syncwarp();
       }
       tc_fence_before();
       __syncwarp();
       if (lane == 0) bp_arrive_cluster(tc_mapa(tc_smem_u32(&acc_empty[buf]), 0u));
+      if (!whole && bp_last(p, k, crank, &last_piece)) {
+        float sum[kBpEpiCols];
+        bp_sum(p, k, crank, warp - 2, lane, sum);
+#pragma unroll
+        for (int c = 0; c < kBpEpiCols; c += 16) {
+          float v[16];
+#pragma unroll
+          for (int j = 0; j < 16; j++) v[j] = sum[c + j];
+          finish(c, v);
+        }
+      }
     }
   }
   tc_fence_before();
@@ -342,9 +290,38 @@ bool bf_pair_serves(const BfParams& p, int64_t M, int64_t N, int64_t K) {
   return at % 16 == 0 && ld % 8 == 0;
 }
 
-int bf_pair_run(BfParams& p, const void* w, const void* x, int64_t M, int64_t N, int64_t K, int64_t ldw, int64_t ldx, cudaStream_t st) {
+// The last round of tiles leaves clusters idle where it is at most half full: its tiles are then cut along k into up to four pieces,
+// if the k steps saved are worth more than 1.2 us per piece (written to L2 by one CTA, read by another) and 2 us.
+int bf_pair_split(int64_t M, int64_t N, int64_t K, double us_per_step) {
+  const int64_t T = ((M + 255) / 256) * ((N + 255) / 256), ks = (K + 63) / 64, G = sm_count() / 2;
+  const int64_t R = T % G;
+  if (R == 0) return 1;
+  int best = 1;
+  double gain = 0.0;
+  for (int S = 2; S <= 4 && S * R <= G && S * 4 <= ks; S++) {
+    const double g = (double)(ks - (ks + S - 1) / S) * us_per_step - 1.2 * S - 2.0;
+    if (g > gain) gain = g, best = S;
+  }
+  return best;
+}
+int bf_pair_clusters(int64_t M, int64_t N, int split) {
+  const int64_t T = ((M + 255) / 256) * ((N + 255) / 256), G = sm_count() / 2;
+  return (int)(T >= G ? G : T * split);
+}
+size_t bf_pair_split_bytes() { return (size_t)(sm_count() / 2) * 2 * 128 * 256 * 4; }
+
+constexpr double kBpUsPerStep = 0.27;
+size_t bf_pair_scratch_bytes(int64_t M, int64_t N, int64_t K) {
+  return kTcCounterBytes + (bf_pair_split(M, N, K, kBpUsPerStep) > 1 ? bf_pair_split_bytes() : 0);
+}
+
+int bf_pair_run(BfParams& p, const void* w, const void* x, int64_t M, int64_t N, int64_t K, int64_t ldw, int64_t ldx, void* scratch,
+                size_t scratch_bytes, cudaStream_t st) {
   using C = BpCfg;
-  p.split = 0;
+  p.split = bf_pair_split(M, N, K, kBpUsPerStep);
+  if (p.split > 1 && scratch_bytes < kTcCounterBytes + bf_pair_split_bytes()) p.split = 1;
+  p.t.counters = reinterpret_cast<unsigned*>(scratch);
+  p.t.partial = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(scratch) + kTcCounterBytes);
   p.t.M = (int)M; p.t.N = (int)N; p.t.K = (int)K;
   p.ksteps = (int)((K + 63) / 64);
   p.TN = (int)((N + 255) / 256);
@@ -361,9 +338,7 @@ int bf_pair_run(BfParams& p, const void* w, const void* x, int64_t M, int64_t N,
     TPX_CUDA_OK(cudaFuncSetAttribute(linear_bf16_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM));
     if (dev >= 0 && dev < 16) opted[dev] = true;
   }
-  const long long T = (long long)p.TN * p.TM;
-  const long long pairs = sm_count() / 2;
-  const int grid = 2 * (int)(T < pairs ? T : pairs);
+  const int grid = 2 * bf_pair_clusters(M, N, p.split);
   TPX_CUDA_OK(launch_pdl(linear_bf16_pair_kernel, dim3((unsigned)grid), dim3(C::THREADS), C::SMEM, st, mw, mx, p));
   return TPX_OK;
 }

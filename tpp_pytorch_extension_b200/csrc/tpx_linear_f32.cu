@@ -1,26 +1,15 @@
 // Linear in true 32-bit: fp32 operands, fp32 products and sums on the CUDA cores (no reduced-precision tensor-core mode),
-// for models that are run in float32; and the tpx_linear entry point that chooses between it and the tcgen05 kernel.
+// for models that are run in float32; and the tpx_linear entry point that chooses between it, the tensor-core form for many rows
+// (tpx_linear_f32_pair.cu) and the bf16 kernels.
 //
 // 64 x 64 output tiles, 16 k values per step in shared memory, 4 x 4 outputs per thread. A decode step (few rows) takes
 // one warp per output feature instead: a 64-row tile would be mostly empty.
-#include "tpx_hybrid.cuh"
+#include "tpx_bf16_pair.cuh"
 
 namespace tpx {
 
 constexpr int kF32Tile = 64, kF32K = 16;
 
-struct F32Epi {
-  const float* bias;
-  void* y;
-  long long ldy;
-  int out_f32, act, act_from;
-  const float* ap;
-  float* z;  // gated units
-  const float *res, *add, *nw, *nb;
-  float *x_out, *h;
-  long long ldz, ldr, ldh;
-  float limit, nalpha;
-};
 __device__ __forceinline__ bool f32_pairs(const F32Epi& e, int n) { return e.act == TPX_ACT_CLAMPED_GLU && n >= e.act_from; }
 
 __device__ __forceinline__ void f32_finish(const F32Epi& e, long long m, int n, float v) {
@@ -43,13 +32,15 @@ __device__ __forceinline__ void f32_finish_pair(const F32Epi& e, long long m, in
   e.z[m * e.ldz + (n - e.act_from) / 2] = hy_clamped_glu(g, u, e.limit);
 }
 
-__global__ void __launch_bounds__(256) linear_f32_kernel(const float* __restrict__ w, const float* __restrict__ x, long long M, int N, int K,
-                                                         long long ldw, long long ldx, F32Epi e) {
+// row0: first row; M: end of the rows. flags: see f32_fma_run.
+__global__ void __launch_bounds__(256) linear_f32_kernel(const float* __restrict__ w, const float* __restrict__ x, long long row0, long long M, int N,
+                                                         int K, long long ldw, long long ldx, F32Epi e, const unsigned* __restrict__ flags, int slab) {
   __shared__ float xs[kF32K][kF32Tile + 4], ws[kF32K][kF32Tile + 4];
   pdl_trigger();
   pdl_wait();
-  const long long m0 = (long long)blockIdx.y * kF32Tile;
+  const long long m0 = row0 + (long long)blockIdx.y * kF32Tile;
   const int n0 = blockIdx.x * kF32Tile;
+  if (flags && !flags[0] && !flags[1 + n0 / slab]) return;  // a slab is a whole number of tiles
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
   float acc[4][4] = {};
   for (int k0 = 0; k0 < K; k0 += kF32K) {
@@ -115,6 +106,13 @@ __global__ void __launch_bounds__(256) linear_f32_rows_kernel(const float* __res
   }
 }
 
+int f32_fma_run(const TpxLinear& a, const F32Epi& e, int64_t m0, int64_t rows, const unsigned* flags, int64_t slab, cudaStream_t st) {
+  TPX_CUDA_OK(launch_pdl(linear_f32_kernel, dim3((unsigned)((a.N + kF32Tile - 1) / kF32Tile), (unsigned)((rows + kF32Tile - 1) / kF32Tile)), dim3(256),
+                         0, st, (const float*)a.w, (const float*)a.x, (long long)m0, (long long)(m0 + rows), (int)a.N, (int)a.K, (long long)a.ldw,
+                         (long long)a.ldx, e, flags, (int)slab));
+  return TPX_OK;
+}
+
 }  // namespace tpx
 
 using namespace tpx;
@@ -144,10 +142,9 @@ extern "C" int tpx_linear(const TpxLinear* a, void* stream) {
     TPX_CUDA_OK(launch_pdl(linear_f32_rows_kernel, dim3((unsigned)((a->N + 7) / 8), (unsigned)((a->M + kF32Rows - 1) / kF32Rows)), dim3(256), 0, st,
                            w, x, (long long)a->M, (int)a->N, (int)a->K, (long long)a->ldw, (long long)a->ldx, e));
   } else {
-    const int64_t my = (a->M + kF32Tile - 1) / kF32Tile;
-    TPX_REQUIRE(my <= 65535, TPX_ERR_UNSUPPORTED, "linear: too many rows for one 32-bit call");
-    TPX_CUDA_OK(launch_pdl(linear_f32_kernel, dim3((unsigned)((a->N + kF32Tile - 1) / kF32Tile), (unsigned)my), dim3(256), 0, st, w, x,
-                           (long long)a->M, (int)a->N, (int)a->K, (long long)a->ldw, (long long)a->ldx, e));
+    TPX_REQUIRE((a->M + kF32Tile - 1) / kF32Tile <= 65535, TPX_ERR_UNSUPPORTED, "linear: too many rows for one 32-bit call");
+    if (f32_pair_serves(*a)) return f32_pair_run(*a, e, st);
+    return f32_fma_run(*a, e, 0, a->M, nullptr, 1, st);
   }
   return TPX_OK;
 }
