@@ -23,6 +23,47 @@ struct BpCfg {
   static constexpr size_t SMEM = (size_t)STAGES * STAGE_BYTES + 1024;
 };
 
+__device__ __forceinline__ void bp_activate8(int act, float (&x)[8]) {
+  switch (act) {
+    case TPX_ACT_GELU:
+#pragma unroll
+      for (int j = 0; j < 8; j++) x[j] = 0.5f * x[j] * (1.0f + erff(x[j] * 0.70710678118654752f));
+      break;
+    case TPX_ACT_SILU:
+#pragma unroll
+      for (int j = 0; j < 8; j++) x[j] = __fdividef(x[j], 1.0f + __expf(-x[j]));
+      break;
+    case TPX_ACT_RELU:
+#pragma unroll
+      for (int j = 0; j < 8; j++) x[j] = fmaxf(x[j], 0.0f);
+      break;
+    default: break;
+  }
+}
+
+// Units n .. n+7 of one token from sixteen features (BfParams::glu; the features are a multiple of 64).
+__device__ __forceinline__ void bp_finish_glu8(const BfParams& p, long long row, int n, const float (&v)[16]) {
+  const TcParams& c = p.t;
+  const size_t o = (size_t)row * (c.N / 2) + n;
+  float x[8], t[8];
+#pragma unroll
+  for (int j = 0; j < 8; j++) x[j] = v[2 * j];
+  if (c.bias) {
+    bp_ld8(c.bias + n, t);
+#pragma unroll
+    for (int j = 0; j < 8; j++) x[j] += t[j];
+  }
+  bp_activate8(c.act, x);
+#pragma unroll
+  for (int j = 0; j < 8; j++) x[j] *= v[2 * j + 1];
+  if (c.res) {
+    bp_ld8(c.res + o, t);
+#pragma unroll
+    for (int j = 0; j < 8; j++) x[j] += t[j] * c.res_scale;
+  }
+  bp_st8(c.y + o, x);
+}
+
 // Features n .. n+7 of one token.
 __device__ __forceinline__ void bp_finish8(const BfParams& p, long long row, int n, float (&x)[8]) {
   float t[8];
@@ -34,21 +75,7 @@ __device__ __forceinline__ void bp_finish8(const BfParams& p, long long row, int
 #pragma unroll
       for (int j = 0; j < 8; j++) x[j] += t[j];
     }
-    switch (c.act) {
-      case TPX_ACT_GELU:
-#pragma unroll
-        for (int j = 0; j < 8; j++) x[j] = 0.5f * x[j] * (1.0f + erff(x[j] * 0.70710678118654752f));
-        break;
-      case TPX_ACT_SILU:
-#pragma unroll
-        for (int j = 0; j < 8; j++) x[j] = __fdividef(x[j], 1.0f + __expf(-x[j]));
-        break;
-      case TPX_ACT_RELU:
-#pragma unroll
-        for (int j = 0; j < 8; j++) x[j] = fmaxf(x[j], 0.0f);
-        break;
-      default: break;
-    }
+    bp_activate8(c.act, x);
     if (c.mul_in) {
       bp_ld8(c.mul_in + o, t);
 #pragma unroll
@@ -223,6 +250,10 @@ linear_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_co
       const bool whole = k.whole();
       float* part = bp_part(p, blockIdx.x, warp - 2) + lane;
       auto finish = [&](int c, float (&v)[16]) {
+        if (p.glu) {
+          if (row < p.t.M && n0 + c < p.t.N) bp_finish_glu8(p, row, (n0 + c) / 2, v);
+          return;
+        }
 #pragma unroll
         for (int h = 0; h < 2; h++) {
           float x[8];

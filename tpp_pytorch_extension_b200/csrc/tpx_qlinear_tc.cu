@@ -29,7 +29,9 @@
 // (one slot per contributor); a small second kernel, launched as a programmatic dependent so that its launch
 // latency hides behind the GEMM, adds them in CTA order and runs the epilogue. Doing this inside the GEMM (last
 // arriver per tile) cost a store -> atomic -> load chain at loaded-memory latency (~2 us per hop).
+#include "tpx_mxfp4_dense.cuh"
 #include "tpx_tc_ptx.cuh"
+#include <algorithm>
 #include <cuda_fp8.h>
 
 namespace tpx {
@@ -1066,7 +1068,9 @@ static size_t tc_scratch_need(int64_t M, int64_t N, int64_t K, bool pair, int ki
 
 extern "C" size_t tpx_qlinear_mxfp4_tc_scratch_bytes(int64_t M, int64_t N, int64_t K, int pair) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
-  return tc_scratch_need(M, N, K, pair != 0, tc_kind(M, N, K, pair != 0));
+  const int kind = tc_kind(M, N, K, pair != 0);
+  const size_t need = tc_scratch_need(M, N, K, pair != 0, kind);  // also where less than the dense form wants is given
+  return kind == 5 && mxfp4_dense_serves(M, N, K, pair != 0) ? std::max(need, mxfp4_dense_scratch_bytes(M, N, K, pair != 0)) : need;
 }
 
 // ---- hand-over between two decode-shaped linears (see TcEmit)
@@ -1108,6 +1112,8 @@ static int tc_run(const uint8_t* wq, const uint8_t* sfa, int pair, const uint16_
     b.bias = bias; b.mul_in = mul_in; b.res = res; b.res_scale = res_scale; b.y = y; b.act = act; b.tl = g_tc_timeline;
     b.dbg = knobs().dbg;
     b.wfmt = wfmt;
+    if (!wfmt && mxfp4_dense_takes(x, M, N, K, dual, b, scratch_bytes, norm))
+      return mxfp4_dense_run(wq, sfa, dual, x, M, N, K, b, scratch, scratch_bytes, (cudaStream_t)stream, norm);
     return tcp2_run(wq, sfa, dual, x, M, N, K, b, scratch, scratch_bytes, (cudaStream_t)stream, norm);
   }
   if (kind == 4) {
