@@ -4,8 +4,8 @@
 // one scale per (token, K block) (quantize_int8sym, :1249), every K block is an int8 x int8 -> int32 product
 // (:1134-1137, :1197-1198) and the output accumulates tmp * s_x[token, block] * s_w[block, feature]
 // (DequantTPP, :1200-1204). Here:
-//   quantize_act_i8_kernel   x bf16 [M][K] -> xq int8 [TOKP][Kp] (padding tokens zero), sx fp32 [K/B][TOKP]
-//   qlinear_i8_kernel<TOK>   A = 128 weight rows (int8, TMA, 128-byte swizzle), B = TOK tokens, tcgen05.mma kind::i8,
+//   quantize_act_i8_kernel   x bf16 [M][K] -> int8 and scales as the GEMM's stages hold them (I8Act; padding tokens zero)
+//   qlinear_i8_kernel<TOK, BS>   A = 128 weight rows (int8, TMA, 128-byte swizzle), B = TOK tokens, tcgen05.mma kind::i8,
 //                            one int32 accumulator per K block in tensor memory (a ring of them); the four epilogue
 //                            warps pull each finished block, scale it and add it to fp32 registers
 // Difference to the reference, inside the parity tolerance: the running output is kept in fp32, where the reference
@@ -13,7 +13,8 @@
 //
 // Work split: one output tile (128 features x TOK tokens, TOK = 16, 32, 64 or, for more than 64 tokens, 128) per CTA;
 // when tiles are few, a thread-block cluster per tile cuts K between its CTAs, which add their parts over distributed
-// shared memory.
+// shared memory. (Sharing the k units of all tiles evenly between the CTAs, 86 tiles of 11008 features on 148 SMs, brought nothing
+// up to 64 tokens: a CTA's chain of copy, MMA, drain is short enough, and putting cut tiles together costs what it saves.)
 #include "tpx_tc_ptx.cuh"
 
 namespace tpx {
@@ -23,13 +24,29 @@ constexpr int kI8MaxStages = 8;
 struct I8Params {
   TcParams t;          // epilogue fields (bias, act, mul_in, res, res_scale, y, M, N, err, cluster)
   const float* swT;    // [K/B][Np] weight scales, feature-contiguous
-  const float* sx;     // [K/B][TOKP] activation scales
+  const uint8_t* xq;   // quantised activations (I8Act)
   int ksteps;          // k steps of 128 (K padded)
-  int bsteps;          // k32 steps per scale block (B / 32)
   int Np;              // features padded to 128
   int nblk;            // scale blocks of the real K (the k padding of the last step has none)
   int tilesN;          // feature tiles; CTA (or cluster) t works on feature tile t % tilesN, token tile t / tilesN
-  int Mp;              // tokens padded to whole token tiles: row stride of sx
+};
+
+// The quantised activations of a token tile and k step (128 values) are one run of memory, fetched by one untiled copy: TOK rows of 128
+// bytes, their 16-byte units in the order of the 128-byte swizzle, then the scales of the step's blocks, [1 or 2][TOK] (a block that
+// spans several steps: with its last one). As plain rows of K bytes the 16 pieces of a step lay a power of two apart, and all CTAs
+// asking for them at once was what bounded the kernel (11008 x 4096, 16 tokens: 20 us, 19.4 without any weight traffic).
+struct I8Act {
+  int TOK, ksteps, B, bytes;  // bytes per (token tile, step)
+  __host__ __device__ I8Act(int tok, int ks, int block) : TOK(tok), ksteps(ks), B(block), bytes(tok * 128 + (block == 64 ? 2 : 1) * tok * 4) {}
+  __device__ __forceinline__ uint8_t* step(uint8_t* xq, int tok, int k) const { return xq + ((size_t)(tok / TOK) * ksteps + k / 128) * bytes; }
+  __device__ __forceinline__ uint8_t* value(uint8_t* xq, int tok, int k) const {  // up to the next 16 values
+    const int r = tok % TOK;
+    return step(xq, tok, k) + r * 128 + (((k % 128) / 16) ^ (r & 7)) * 16 + k % 16;
+  }
+  __device__ __forceinline__ float* scale(uint8_t* xq, int tok, int blk) const {
+    const int k = blk * B + B - 1;
+    return reinterpret_cast<float*>(step(xq, tok, k) + TOK * 128) + (B == 64 ? blk & 1 : 0) * TOK + tok % TOK;
+  }
 };
 
 __device__ __forceinline__ void i8_mma(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
@@ -40,20 +57,29 @@ __device__ __forceinline__ void i8_mma(uint32_t d_tmem, uint64_t adesc, uint64_t
       : "memory");
 }
 
+__device__ __forceinline__ float i8_ld_shared(uint32_t a) {
+  float v;
+  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ float4 i8_ld_shared4(uint32_t a) {
+  float4 v;
+  asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
+  return v;
+}
+
 // One thread per (token row of the padded tile, K block): scale = max|x| / 127 in double as the reference does
 // (src/csrc/qtypes.cpp:153-197), q = clamp(rint(x / scale)).
-__global__ void quantize_act_i8_kernel(const uint16_t* __restrict__ x, int M, int K, int Kp, int B, int TOKP, int8_t* __restrict__ xq,
-                                       float* __restrict__ sx) {
+__global__ void quantize_act_i8_kernel(const uint16_t* __restrict__ x, int M, int K, int rows, I8Act L, uint8_t* __restrict__ xq) {
   pdl_trigger();
   pdl_wait();
-  const int nb = K / B;
+  const int B = L.B, nb = K / B;
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= TOKP * nb) return;
+  if (idx >= rows * nb) return;
   const int tok = idx / nb, blk = idx % nb;
-  int8_t* dst = xq + (size_t)tok * Kp + (size_t)blk * B;
   if (tok >= M) {
-    for (int i = 0; i < B; i += 16) *reinterpret_cast<uint4*>(dst + i) = make_uint4(0, 0, 0, 0);
-    sx[(size_t)blk * TOKP + tok] = 0.0f;
+    for (int i = 0; i < B; i += 16) *reinterpret_cast<uint4*>(L.value(xq, tok, blk * B + i)) = make_uint4(0, 0, 0, 0);
+    *L.scale(xq, tok, blk) = 0.0f;
     return;
   }
   const uint16_t* src = x + (size_t)tok * K + (size_t)blk * B;
@@ -82,38 +108,43 @@ __global__ void quantize_act_i8_kernel(const uint16_t* __restrict__ x, int M, in
       }
       o[q] = word;
     }
-    *reinterpret_cast<uint4*>(dst + i) = make_uint4(o[0], o[1], o[2], o[3]);
+    *reinterpret_cast<uint4*>(L.value(xq, tok, blk * B + i)) = make_uint4(o[0], o[1], o[2], o[3]);
   }
-  sx[(size_t)blk * TOKP + tok] = scale;
+  *L.scale(xq, tok, blk) = scale;
 }
 
-// The same quantisation with one CTA per token row, vectorised, for blocks of up to 256 values, optionally behind an
-// RMSNorm of the row (y = bf16(x * rsqrt(mean(x^2) + eps) * gamma), llama_rms_norm of the reference, rows of up to
-// 8192 values then): eight consecutive values per thread, the B/8 threads of a block reduce its maximum with shuffles.
+// The same quantisation vectorised, for blocks of up to 256 values, optionally behind an RMSNorm of the row
+// (y = bf16(x * rsqrt(mean(x^2) + eps) * gamma), llama_rms_norm of the reference, rows of up to 8192 values then): eight consecutive
+// values per thread and vector, the B/8 threads of a block reduce its maximum with shuffles. With the norm a CTA has a whole row in
+// VECS vectors per thread, without it a row is spread over gridDim.y CTAs: the kernel is latency, and one CTA that goes round
+// over a row of 11008 values took 9 us.
 constexpr int kQaThreads = 256;
+template <int VECS>
 __global__ void __launch_bounds__(kQaThreads) quantize_act_i8_row_kernel(const uint16_t* __restrict__ x, const void* __restrict__ gamma,
-                                                                         int gamma_f32, float eps, int M, int K, int Kp, int B, int TOKP,
-                                                                         int8_t* __restrict__ xq, float* __restrict__ sx) {
+                                                                         int gamma_f32, float eps, int M, int K, I8Act L, uint8_t* __restrict__ xq) {
   __shared__ float red[kQaThreads / 32];
   pdl_trigger();
   pdl_wait();
   const int tok = blockIdx.x;
   const int nv = K / 8;
-  const int lanes = B / 8;  // threads per scale block: 8, 16 or 32
+  const int lanes = L.B / 8;  // threads per scale block: 8, 16 or 32
   const bool live = tok < M;
   const uint4* xr = reinterpret_cast<const uint4*>(x + (size_t)tok * K);
-  float inv = 1.0f;
-  if (gamma && live) {
-    float ss = 0.0f;
-    for (int i = threadIdx.x; i < nv; i += kQaThreads) {
-      const uint4 v = xr[i];
-      const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+  float f[VECS][8];
+  float ss = 0.0f;
 #pragma unroll
-      for (int j = 0; j < 4; j++) {
-        const float a = bf16_bits_to_f32((uint16_t)(w[j] & 0xffff)), b = bf16_bits_to_f32((uint16_t)(w[j] >> 16));
-        ss += a * a + b * b;
-      }
+  for (int q = 0; q < VECS; q++) {
+    const int i = threadIdx.x + (blockIdx.y * VECS + q) * kQaThreads;
+    const uint4 v = live && i < nv ? xr[i] : make_uint4(0, 0, 0, 0);
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      f[q][2 * j] = bf16_bits_to_f32((uint16_t)(w[j] & 0xffff));
+      f[q][2 * j + 1] = bf16_bits_to_f32((uint16_t)(w[j] >> 16));
+      ss += f[q][2 * j] * f[q][2 * j] + f[q][2 * j + 1] * f[q][2 * j + 1];
     }
+  }
+  if (gamma) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
@@ -121,43 +152,34 @@ __global__ void __launch_bounds__(kQaThreads) quantize_act_i8_row_kernel(const u
     float tot = 0.0f;
 #pragma unroll
     for (int w = 0; w < kQaThreads / 32; w++) tot += red[w];
-    inv = rsqrtf(tot / (float)K + eps);
-  }
-  for (int i0 = 0; i0 < nv; i0 += kQaThreads) {
-    const int i = i0 + threadIdx.x;
-    const bool in = i < nv;
-    float f[8];
+    const float inv = rsqrtf(tot / (float)K + eps);
 #pragma unroll
-    for (int j = 0; j < 8; j++) f[j] = 0.0f;
-    if (in && live) {
-      const uint4 v = xr[i];
-      const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+    for (int q = 0; q < VECS; q++) {
+      const int i = threadIdx.x + q * kQaThreads;
+      if (i >= nv) continue;
+      float g[8];
+      if (gamma_f32) {
+        const float4 g0 = reinterpret_cast<const float4*>(gamma)[2 * i], g1 = reinterpret_cast<const float4*>(gamma)[2 * i + 1];
+        g[0] = g0.x; g[1] = g0.y; g[2] = g0.z; g[3] = g0.w; g[4] = g1.x; g[5] = g1.y; g[6] = g1.z; g[7] = g1.w;
+      } else {
+        const uint4 gv = reinterpret_cast<const uint4*>(gamma)[i];
+        const uint32_t gw[4] = {gv.x, gv.y, gv.z, gv.w};
 #pragma unroll
-      for (int j = 0; j < 4; j++) {
-        f[2 * j] = bf16_bits_to_f32((uint16_t)(w[j] & 0xffff));
-        f[2 * j + 1] = bf16_bits_to_f32((uint16_t)(w[j] >> 16));
-      }
-      if (gamma) {
-        float g[8];
-        if (gamma_f32) {
-          const float4 g0 = reinterpret_cast<const float4*>(gamma)[2 * i], g1 = reinterpret_cast<const float4*>(gamma)[2 * i + 1];
-          g[0] = g0.x; g[1] = g0.y; g[2] = g0.z; g[3] = g0.w; g[4] = g1.x; g[5] = g1.y; g[6] = g1.z; g[7] = g1.w;
-        } else {
-          const uint4 gv = reinterpret_cast<const uint4*>(gamma)[i];
-          const uint32_t gw[4] = {gv.x, gv.y, gv.z, gv.w};
-#pragma unroll
-          for (int j = 0; j < 4; j++) {
-            g[2 * j] = bf16_bits_to_f32((uint16_t)(gw[j] & 0xffff));
-            g[2 * j + 1] = bf16_bits_to_f32((uint16_t)(gw[j] >> 16));
-          }
+        for (int j = 0; j < 4; j++) {
+          g[2 * j] = bf16_bits_to_f32((uint16_t)(gw[j] & 0xffff));
+          g[2 * j + 1] = bf16_bits_to_f32((uint16_t)(gw[j] >> 16));
         }
-#pragma unroll
-        for (int j = 0; j < 8; j++) f[j] = bf16_bits_to_f32(f32_to_bf16_bits(f[j] * inv * g[j]));
       }
+#pragma unroll
+      for (int j = 0; j < 8; j++) f[q][j] = bf16_bits_to_f32(f32_to_bf16_bits(f[q][j] * inv * g[j]));
     }
+  }
+#pragma unroll
+  for (int q = 0; q < VECS; q++) {
+    const int i = threadIdx.x + (blockIdx.y * VECS + q) * kQaThreads;
     float amax = 0.0f;
 #pragma unroll
-    for (int j = 0; j < 8; j++) amax = fmaxf(amax, fabsf(f[j]));
+    for (int j = 0; j < 8; j++) amax = fmaxf(amax, fabsf(f[q][j]));
     for (int o = 1; o < lanes; o <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
     const float scale = (float)((double)amax / 127.0);
     const float iscale = scale != 0.0f ? 1.0f / scale : 0.0f;
@@ -167,15 +189,15 @@ __global__ void __launch_bounds__(kQaThreads) quantize_act_i8_row_kernel(const u
       uint32_t word = 0;
 #pragma unroll
       for (int e = 0; e < 4; e++) {
-        float q = nearbyintf(f[4 * h + e] * iscale);
-        q = fminf(fmaxf(q, -127.0f), 127.0f);
-        word |= ((uint32_t)(uint8_t)(int8_t)(int)q) << (8 * e);
+        float r = nearbyintf(f[q][4 * h + e] * iscale);
+        r = fminf(fmaxf(r, -127.0f), 127.0f);
+        word |= ((uint32_t)(uint8_t)(int8_t)(int)r) << (8 * e);
       }
       o2[h] = word;
     }
-    if (in) {
-      *reinterpret_cast<uint2*>(xq + (size_t)tok * Kp + (size_t)i * 8) = make_uint2(o2[0], o2[1]);
-      if ((i % lanes) == 0) sx[(size_t)(i / lanes) * TOKP + tok] = live ? scale : 0.0f;
+    if (i < nv) {
+      *reinterpret_cast<uint2*>(L.value(xq, tok, i * 8)) = make_uint2(o2[0], o2[1]);
+      if ((i % lanes) == 0) *L.scale(xq, tok, i / lanes) = live ? scale : 0.0f;
     }
   }
 }
@@ -198,33 +220,47 @@ __global__ void repack_qint8_tc_kernel(const int8_t* __restrict__ q, const float
   }
 }
 
-template <int TOK>
+// BS: k32 steps per scale block (block / 32)
+template <int TOK, int BS>
 struct I8Cfg {
   static constexpr int A_BYTES = 128 * 128;   // 128 features x 128 k values
   static constexpr int B_BYTES = TOK * 128;   // TOK tokens x 128 k values
-  static constexpr int STAGE_BYTES = (A_BYTES + B_BYTES + 1023) / 1024 * 1024;
+  // Scales of the blocks of a step travel with it: read from global memory group by group they cost the epilogue a memory
+  // latency per 256 k values.
+  static constexpr int ROWS = BS == 2 ? 2 : 1;  // scale rows per step (a block that spans several steps: its row with each of them)
+  static constexpr int SX_BYTES = ROWS * TOK * 4, SW_BYTES = ROWS * 128 * 4;  // behind the activations, in this order
+  static constexpr int STAGE_BYTES = (A_BYTES + B_BYTES + SW_BYTES + SX_BYTES + 1023) / 1024 * 1024;
   static constexpr int STAGES_FIT = (227 * 1024 - 3072) / STAGE_BYTES;   // as many stages as shared memory holds: the bytes in
   static constexpr int STAGES = STAGES_FIT > kI8MaxStages ? kI8MaxStages : STAGES_FIT;  // flight bound the stream, not the MMAs
-  static constexpr int GROUP = TOK >= 128 ? 2 : 4;  // accumulators per group; a group (up to GROUP K blocks, 256 k values or one
-                                                    // larger block) is handed to the epilogue per barrier round trip
+  static constexpr int GROUP = TOK >= 128 ? 2 : 4;  // accumulators per group
   static constexpr int NBUF = 512 / TOK > 16 ? 16 : 512 / TOK;  // int32 accumulators (one per K block) in tensor memory
+  static constexpr int NGRP = NBUF / GROUP;
+  // K blocks that are handed to the epilogue per barrier round trip: 256 k values, or one larger block; their k steps
+  static constexpr int GS = BS >= 8 ? 1 : (8 / BS < GROUP ? 8 / BS : GROUP);
+  static constexpr int SG = GS * BS / 4;
+  static constexpr int ALIGN = BS > 4 ? BS / 4 : 1;  // k steps per scale block when a block spans several
   // Draining a K block (tensor memory -> int32 -> * s_x * s_w -> fp32 sum) is a chain of dependent scalar instructions;
   // with one warp per 32-row quarter it, not the MMAs, bounds the kernel as soon as there are many tokens. Every quarter
   // has EPI_SPLIT warps, each owning TW = TOK / EPI_SPLIT tokens (columns) of the tile.
   static constexpr int EPI_SPLIT = TOK >= 64 ? 4 : TOK / 16;
   static constexpr int TW = TOK / EPI_SPLIT;
   static constexpr int THREADS = 64 + 128 * EPI_SPLIT;
-  static constexpr int NGRP = NBUF / GROUP;
   static constexpr int TMEM_COLS = NBUF * TOK < 32 ? 32 : NBUF * TOK;
   static constexpr size_t SMEM = (size_t)STAGES * STAGE_BYTES + 1024;
   static_assert(NBUF * TOK <= 512, "tensor memory");
+  static_assert(SG >= 1 && SG <= STAGES, "a group's stages are held until it is drained");
   static_assert(128 * TOK * 4 <= STAGES * STAGE_BYTES, "the partial tile of a cluster member fits in the stages");
 };
 
-template <int TOK>
-__global__ void __launch_bounds__(I8Cfg<TOK>::THREADS, 1)
-qlinear_i8_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, I8Params p) {
-  using C = I8Cfg<TOK>;
+// One warp copies and one issues MMAs, for tens of steps of a few hundred cycles: everything in their loops that depends on the
+// block size is a constant, loop state is the same in all lanes, and only the issue itself is under an elected lane. (With the
+// bookkeeping of blocks and groups per MMA in one thread, the empty loops alone took 0.35 us per step.) 11008 x 4096, block 64, with the
+// quantisation of x, before and after this form: 1 token 27.4 / 16.3 us, 32: 30.1 / 18.8, 64: 38.0 / 26.3, 128: 81 / 43. What is left is a
+// chain per 256 k values (copies, eight MMAs, drain) that no single part of sets the pace: leaving one out takes 1 to 2 us off.
+template <int TOK, int BS>
+__global__ void __launch_bounds__(I8Cfg<TOK, BS>::THREADS, 1)
+qlinear_i8_kernel(const __grid_constant__ CUtensorMap tmW, I8Params p) {
+  using C = I8Cfg<TOK, BS>;
   extern __shared__ unsigned char i8_smem_raw[];
   __shared__ __align__(8) unsigned long long bar_full[C::STAGES], bar_empty[C::STAGES];
   __shared__ __align__(8) unsigned long long d_full[C::NGRP], d_free[C::NGRP];
@@ -236,16 +272,15 @@ qlinear_i8_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
   const int crank = csize > 1 ? (int)tc_cluster_rank() : 0;
   const int tile = (int)(blockIdx.x / csize) % p.tilesN;  // feature tile
   const int tm = (int)(blockIdx.x / csize) / p.tilesN;    // token tile
-  // K range of this CTA in k steps, aligned to whole scale blocks
-  const int align = p.bsteps > 4 ? p.bsteps / 4 : 1;  // k steps per scale block when a block spans several
-  const int groups = p.ksteps / align;
-  const int ks0 = (int)((long long)crank * groups / csize) * align, ks1 = (int)((long long)(crank + 1) * groups / csize) * align;
+  // K range of this CTA in k steps, whole scale blocks
+  const int groups = p.ksteps / C::ALIGN;
+  const int ks0 = (int)((long long)crank * groups / csize) * C::ALIGN, ks1 = (int)((long long)(crank + 1) * groups / csize) * C::ALIGN;
   const int nsteps = ks1 - ks0;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::STAGES; s++) {
       tc_mbar_init(tc_smem_u32(&bar_full[s]), 1);
-      tc_mbar_init(tc_smem_u32(&bar_empty[s]), 1);
+      tc_mbar_init(tc_smem_u32(&bar_empty[s]), 4 * C::EPI_SPLIT);
     }
     for (int b = 0; b < C::NGRP; b++) {
       tc_mbar_init(tc_smem_u32(&d_full[b]), 1);
@@ -267,153 +302,164 @@ qlinear_i8_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
   pdl_trigger();
 
   constexpr int TW = C::TW;
-  float acc[TW];  // this thread's tokens of its feature row
-#pragma unroll
-  for (int i = 0; i < TW; i++) acc[i] = 0.0f;
-
   if (warp == 0) {
     // ------------------------------------------------------------ producer
-    if (tc_elect()) {
-      auto fetch_w = [&](int s, int ks) {
-        const uint32_t st = smem_base + (uint32_t)s * C::STAGE_BYTES;
-        tc_mbar_expect_tx(tc_smem_u32(&bar_full[s]), C::A_BYTES + C::B_BYTES);
-        tc_tma_2d(st, &tmW, ks * 128, tile * 128, tc_smem_u32(&bar_full[s]));
-      };
-      const int early = nsteps < C::STAGES ? nsteps : C::STAGES;
-      for (int it = 0; it < early; it++) fetch_w(it, ks0 + it);  // weights do not depend on the quantisation kernel
-      pdl_wait();
-      for (int it = 0; it < nsteps; it++) {
-        const int s = it % C::STAGES;
-        if (it >= C::STAGES) {
-          if (!tc_wait(tc_smem_u32(&bar_empty[s]), (uint32_t)((it / C::STAGES - 1) & 1))) { atomicExch(p.t.err, 2u); break; }
-          fetch_w(s, ks0 + it);
-        }
-        tc_tma_2d(smem_base + (uint32_t)s * C::STAGE_BYTES + C::A_BYTES, &tmX, (ks0 + it) * 128, tm * TOK, tc_smem_u32(&bar_full[s]));
+    constexpr uint32_t kScales = C::A_BYTES + C::B_BYTES + C::SX_BYTES;
+    auto first_row = [](int ks) { return BS == 2 ? 2 * ks : ks / C::ALIGN; };
+    auto rows = [&](int ks) { return min(C::ROWS, max(0, p.nblk - first_row(ks))); };  // the k padding of the last step has no scales
+    auto fetch_w = [&](int s, int ks) {
+      if (tc_elect()) {
+        const uint32_t st = smem_base + (uint32_t)s * C::STAGE_BYTES, bar = tc_smem_u32(&bar_full[s]);
+        const int n = rows(ks);
+        tc_mbar_expect_tx(bar, kScales + n * 512);
+        tc_tma_2d(st, &tmW, ks * 128, tile * 128, bar);
+        const float* src = p.swT + (size_t)first_row(ks) * p.Np + tile * 128;
+#pragma unroll
+        for (int r = 0; r < C::ROWS; r++)
+          if (r < n) tc_bulk_g2s(st + kScales + r * 512, src + (size_t)r * p.Np, 512, bar);
       }
+      __syncwarp();
+    };
+    const int early = nsteps < C::STAGES ? nsteps : C::STAGES;
+    for (int it = 0; it < early; it++) fetch_w(it, ks0 + it);  // weights do not depend on the quantisation kernel
+    pdl_wait();
+    int s = 0;
+    uint32_t phase = 1;  // parity to wait for on bar_empty: the first round over the ring finds every stage free
+    for (int it = 0; it < nsteps; it++) {
+      if (it >= C::STAGES) {
+        if (!tc_wait(tc_smem_u32(&bar_empty[s]), phase)) {
+          if (tc_elect()) atomicExch(p.t.err, 2u);
+          break;
+        }
+        fetch_w(s, ks0 + it);
+      }
+      if (tc_elect()) {
+        const uint32_t st = smem_base + (uint32_t)s * C::STAGE_BYTES, bar = tc_smem_u32(&bar_full[s]);
+        tc_bulk_g2s(st + C::A_BYTES, p.xq + ((size_t)tm * p.ksteps + ks0 + it) * (C::B_BYTES + C::SX_BYTES), C::B_BYTES + C::SX_BYTES, bar);
+      }
+      __syncwarp();
+      if (++s == C::STAGES) s = 0, phase ^= 1u;
     }
-    __syncwarp();
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (tc_elect()) {
-      // kind::i8: D = S32 (2), A = B = S8 (1), both K-major, N = TOK, M = 128
-      const uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TOK >> 3) << 17) | ((128u >> 4) << 24);
-      int buf = 0, inblk = 0;  // accumulator in use, k32 steps already in the current scale block
-      uint32_t free_phase = 0;  // bit g: parity to wait for on d_free[g]
-      unsigned used = 0;        // bit g: group g has been handed out before
-      const int nblocks = nsteps * 4 / p.bsteps;
-      const int gsize = p.bsteps >= 8 ? 1 : (8 / p.bsteps < C::GROUP ? 8 / p.bsteps : C::GROUP);  // blocks per group: 256 k values, or one larger block
-      int done_blocks = 0;
-      for (int it = 0; it < nsteps; it++) {
-        const int s = it % C::STAGES;
-        if (!tc_wait(tc_smem_u32(&bar_full[s]), (uint32_t)((it / C::STAGES) & 1))) { atomicExch(p.t.err, 4u); break; }
-        tc_fence_after();
-        const uint32_t st = smem_base + (uint32_t)s * C::STAGE_BYTES;
-        bool dead = false;
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-          const int grp = buf / C::GROUP;
-          if (inblk == 0 && buf % C::GROUP == 0 && ((used >> grp) & 1u)) {  // a recycled group: the epilogue must have read it
-            if (!tc_wait(tc_smem_u32(&d_free[grp]), (free_phase >> grp) & 1u)) { atomicExch(p.t.err, 3u); dead = true; break; }
-            free_phase ^= 1u << grp;
-            tc_fence_after();
-          }
-          i8_mma(tmem + buf * TOK, tc_smem_desc(st) + (uint64_t)(2 * j), tc_smem_desc(st + C::A_BYTES) + (uint64_t)(2 * j), idesc,
-                 inblk == 0 ? 0u : 1u);
-          if (++inblk == p.bsteps) {  // block complete
-            inblk = 0;
-            done_blocks++;
-            if (buf % C::GROUP + 1 == gsize || done_blocks == nblocks) {
-              // group complete: hand its accumulators to the epilogue. This one commit also tells that the stages the
-              // group read are free again (the epilogue passes that on to the producer), so stages need none of their own.
-              tc_commit(tc_smem_u32(&d_full[grp]));
-              used |= 1u << grp;
-              buf = (grp + 1) * C::GROUP % C::NBUF;
-            } else {
-              buf++;
-            }
-          }
+    // kind::i8: D = S32 (2), A = B = S8 (1), both K-major, N = TOK, M = 128
+    constexpr uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TOK >> 3) << 17) | ((128u >> 4) << 24);
+    const uint64_t desc0 = tc_smem_desc(smem_base);
+    int s = 0, g = 0;  // g: groups handed out
+    uint32_t phase = 0;
+    bool dead = false;
+    for (int left = nsteps; !dead && left > 0; left -= C::SG, g++) {
+      const int grp = g % C::NGRP;
+      if (g >= C::NGRP) {  // a recycled group: the epilogue must have read it
+        if (!tc_wait(tc_smem_u32(&d_free[grp]), (uint32_t)((g / C::NGRP - 1) & 1))) {
+          if (tc_elect()) atomicExch(p.t.err, 3u);
+          dead = true;
+          break;
         }
-        if (dead) break;
+        tc_fence_after();
       }
+      const uint32_t d = tmem + grp * (C::GROUP * TOK);
+#pragma unroll
+      for (int t = 0; t < C::SG; t++) {
+        if (t >= left || dead) continue;
+        if (!tc_wait(tc_smem_u32(&bar_full[s]), phase)) {
+          if (tc_elect()) atomicExch(p.t.err, 4u);
+          dead = true;
+          continue;
+        }
+        tc_fence_after();
+        if (tc_elect()) {
+          const uint64_t desc = desc0 + (uint64_t)(s * (C::STAGE_BYTES >> 4));  // descriptors count 16-byte units
+#pragma unroll
+          for (int j = 0; j < 4; j++)
+            i8_mma(d + (4 * t + j) / BS * TOK, desc + (uint64_t)(2 * j), desc + (uint64_t)((C::A_BYTES >> 4) + 2 * j), idesc, (4 * t + j) % BS ? 1u : 0u);
+        }
+        __syncwarp();
+        if (++s == C::STAGES) s = 0, phase ^= 1u;
+      }
+      // the epilogue also frees the stages that the group read, once it has used their scales
+      if (!dead && tc_elect()) tc_commit(tc_smem_u32(&d_full[grp]));
+      __syncwarp();
     }
-    __syncwarp();
   } else {
     // ------------------------------------------------------------ epilogue: thread = feature row of the tile
     const int sub = warp & 3;
     const uint32_t lane_base = ((uint32_t)(sub * 32)) << 16;
     const int row = sub * 32 + lane;
-    const int n = tile * 128 + row;
+    const int cpart = (warp - 2) >> 2;  // this warp's tokens: [cpart * TW, +TW) of the tile
     pdl_wait();
-    const int nblocks = nsteps * 4 / p.bsteps;
-    const int blk0 = ks0 * 4 / p.bsteps;
-    uint32_t full_phase = 0;
-    constexpr bool kPrefetchSx = TW * C::GROUP <= 128;  // activation scales of a whole group in registers
-    const int cpart = (warp - 2) >> 2;                   // this warp's tokens: [cpart * TW, +TW) of the tile
-    const int gsize = p.bsteps >= 8 ? 1 : (8 / p.bsteps < C::GROUP ? 8 / p.bsteps : C::GROUP);
-    const float* sx_tile = p.sx + (size_t)tm * TOK + (size_t)cpart * TW;  // this warp's columns of sx [K/B][Mp]
-    int b = 0, buf = 0;
-    bool dead = false;
-    while (b < nblocks && !dead) {
-      const int grp = buf / C::GROUP;
-      const int cnt = nblocks - b < gsize ? nblocks - b : gsize;
-      // scales of the group's blocks are fetched before the wait (a block of pure k padding has none: zeros)
-      float sw[C::GROUP];
-      float sxg[kPrefetchSx ? C::GROUP : 1][kPrefetchSx ? TW : 1];
+    // The conversion instruction runs at a quarter of the rate of an addition. Sums of at most 256 products stay below 2^22: added to
+    // the bits of 1.5 * 2^23 they are that float's low bits, exact either way.
+    auto to_float = [](uint32_t d) { return BS <= 8 ? __uint_as_float(d + 0x4B400000u) - 12582912.0f : (float)(int)d; };
+    int s = 0, g = 0;
+    uint32_t phase = 0;
+    bool dead = false;  // a warp that gave up still meets the others at their barriers
+    const int n = tile * 128 + row;
+    float acc[TW];  // this thread's tokens of its feature row
 #pragma unroll
-      for (int q = 0; q < C::GROUP; q++) {
-        const int blk = blk0 + b + q;
-        const bool real = q < cnt && blk < p.nblk;
-        sw[q] = real ? p.swT[(size_t)blk * p.Np + n] : 0.0f;
-        if (kPrefetchSx) {
-          const float4* sxp = reinterpret_cast<const float4*>(sx_tile + (size_t)(real ? blk : 0) * p.Mp);
+    for (int i = 0; i < TW; i++) acc[i] = 0.0f;
+    int blk = BS == 2 ? 2 * ks0 : ks0 / C::ALIGN;
+    for (int left = nsteps; left > 0 && !dead; left -= C::SG, g++, blk += C::GS) {
+      const int grp = g % C::NGRP;
+      const int steps = left < C::SG ? left : C::SG, cnt = BS == 2 ? 2 * steps : steps / C::ALIGN;
+      uint32_t at[C::SG];  // the steps' stages: their scales were copied there
+      const int s_first = s;
+      bool ok = true;
 #pragma unroll
-          for (int i = 0; i < TW / 4; i++) {
-            const float4 v = sxp[i];
-            sxg[q][4 * i] = v.x; sxg[q][4 * i + 1] = v.y; sxg[q][4 * i + 2] = v.z; sxg[q][4 * i + 3] = v.w;
-          }
-        }
+      for (int t = 0; t < C::SG; t++) {
+        at[t] = smem_base + (uint32_t)s * C::STAGE_BYTES + C::A_BYTES + C::B_BYTES;
+        if (t >= steps) continue;
+        ok = ok && tc_wait(tc_smem_u32(&bar_full[s]), phase);
+        if (++s == C::STAGES) s = 0, phase ^= 1u;
       }
-      if (!tc_wait(tc_smem_u32(&d_full[grp]), (full_phase >> grp) & 1u)) {
+      if (!ok || !tc_wait(tc_smem_u32(&d_full[grp]), (uint32_t)((g / C::NGRP) & 1))) {
         if (lane == 0) atomicExch(p.t.err, 6u);
         dead = true;
         break;
       }
-      full_phase ^= 1u << grp;
       tc_fence_after();
-      if (sub == 0 && lane == 0 && cpart == 0) {  // the MMAs of this group are complete: the stages they read may be refilled
-        const int it_lo = b * p.bsteps / 4, it_hi = (b + cnt) * p.bsteps / 4;
-        for (int it = it_lo; it < it_hi; it++) tc_mbar_arrive(tc_smem_u32(&bar_empty[it % C::STAGES]));
-      }
+      constexpr int BATCH = C::EPI_SPLIT <= 2 ? C::GS : 1;  // blocks per round trip to tensor memory
 #pragma unroll
-      for (int q = 0; q < C::GROUP; q++) {
-        if (q < cnt) {
-          const int blk = blk0 + b + q;
-          const float4* sxp = reinterpret_cast<const float4*>(sx_tile + (size_t)(blk < p.nblk ? blk : 0) * p.Mp);
+      for (int q0 = 0; q0 < C::GS; q0 += BATCH) {
 #pragma unroll
-          for (int c0 = 0; c0 < TW; c0 += 16) {
-            float sxc[16];
-            if (!kPrefetchSx) {  // many tokens: the scales of 16 tokens at a time (they sit in L1 after the first warp's read)
+        for (int c0 = 0; c0 < TW; c0 += 16) {
+          uint32_t d[BATCH][16];
 #pragma unroll
-              for (int i = 0; i < 4; i++) {
-                const float4 v = sxp[c0 / 4 + i];
-                sxc[4 * i] = v.x; sxc[4 * i + 1] = v.y; sxc[4 * i + 2] = v.z; sxc[4 * i + 3] = v.w;
-              }
+          for (int q = 0; q < BATCH; q++)
+            if (q0 + q < cnt) tc_ld_x16(tmem + lane_base + (grp * C::GROUP + q0 + q) * TOK + cpart * TW + c0, d[q]);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+          for (int q = 0; q < BATCH; q++) {
+            if (q0 + q >= cnt || blk + q0 + q >= p.nblk) continue;  // (a block of pure k padding has no scales)
+            const uint32_t sc = at[((q0 + q + 1) * BS - 1) / 4];  // the block's last step
+            const int r = BS == 2 ? (q0 + q) & 1 : 0;
+            const float sw = i8_ld_shared(sc + C::SX_BYTES + r * 512 + row * 4);
+#pragma unroll
+            for (int i = 0; i < 16; i += 4) {
+              const float4 sx = i8_ld_shared4(sc + (r * TOK + cpart * TW + c0 + i) * 4);
+              acc[c0 + i] += to_float(d[q][i]) * sx.x * sw;
+              acc[c0 + i + 1] += to_float(d[q][i + 1]) * sx.y * sw;
+              acc[c0 + i + 2] += to_float(d[q][i + 2]) * sx.z * sw;
+              acc[c0 + i + 3] += to_float(d[q][i + 3]) * sx.w * sw;
             }
-            uint32_t d[16];
-            tc_ld_x16(tmem + lane_base + (buf + q) * TOK + cpart * TW + c0, d);
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-            for (int i = 0; i < 16; i++) acc[c0 + i] += (float)(int)d[i] * (kPrefetchSx ? sxg[q][c0 + i] : sxc[i]) * sw[q];
           }
         }
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) tc_mbar_arrive(tc_smem_u32(&d_free[grp]));
-      b += cnt;
-      buf = (grp + 1) * C::GROUP % C::NBUF;
+      if (lane == 0) {
+        tc_mbar_arrive(tc_smem_u32(&d_free[grp]));
+#pragma unroll
+        for (int t = 0; t < C::SG; t++)
+          if (t < steps) tc_mbar_arrive(tc_smem_u32(&bar_empty[s_first + t < C::STAGES ? s_first + t : s_first + t - C::STAGES]));
+      }
     }
-    if (csize == 1) {
+    if (csize > 1) {
+      asm volatile("bar.sync 1, %0;" ::"n"(C::THREADS - 64) : "memory");  // nobody still reads scales from the stages
+      const uint32_t sp = smem_base + (uint32_t)((row * TOK + cpart * TW) * 4);
+#pragma unroll
+      for (int c0 = 0; c0 < TW; c0 += 4) tc_st_shared_f4(sp + c0 * 4, make_float4(acc[c0], acc[c0 + 1], acc[c0 + 2], acc[c0 + 3]));
+    } else if (!dead) {
 #pragma unroll
       for (int c0 = 0; c0 < TW; c0 += 16) {
         float v[16], v2[16];
@@ -422,10 +468,6 @@ qlinear_i8_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
         const int tok0 = tm * TOK + cpart * TW + c0;
         if (n < p.t.N && tok0 < p.t.M) tc_finish16<false>(p.t, tok0, n, v, v2);
       }
-    } else {
-      const uint32_t sp = smem_base + (uint32_t)((row * TOK + cpart * TW) * 4);
-#pragma unroll
-      for (int c0 = 0; c0 < TW; c0 += 4) tc_st_shared_f4(sp + c0 * 4, make_float4(acc[c0], acc[c0 + 1], acc[c0 + 2], acc[c0 + 3]));
     }
   }
   tc_fence_before();
@@ -459,7 +501,7 @@ qlinear_i8_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
 struct I8Plan {
   int tokp, ksteps, tiles, cluster, TM;  // tiles = feature tiles x token tiles
   int64_t Kp, Np, Mp;
-  size_t off_xq, off_sx, total;
+  size_t off_xq, xq_bytes, total;
 };
 
 static I8Plan i8_plan(int64_t M, int64_t N, int64_t K, int64_t B) {
@@ -479,20 +521,20 @@ static I8Plan i8_plan(int64_t M, int64_t N, int64_t K, int64_t B) {
   pl.cluster = c < 1 ? 1 : c;
   size_t o = kTcCounterBytes;
   auto bump = [&](size_t bytes) { size_t r = o; o += (bytes + 1023) & ~(size_t)1023; return r; };
-  pl.off_xq = bump((size_t)pl.Mp * pl.Kp);
-  pl.off_sx = bump((size_t)(K / B) * pl.Mp * sizeof(float));
+  pl.xq_bytes = (size_t)pl.TM * pl.ksteps * I8Act(pl.tokp, pl.ksteps, (int)B).bytes;
+  pl.off_xq = bump(pl.xq_bytes);
   pl.total = o;
   return pl;
 }
 
-template <int TOK>
-static int i8_launch(const CUtensorMap& w, const CUtensorMap& x, I8Params p, int tiles, cudaStream_t st) {
-  using C = I8Cfg<TOK>;
+template <int TOK, int BS>
+static int i8_launch(const CUtensorMap& w, I8Params p, int tiles, cudaStream_t st) {
+  using C = I8Cfg<TOK, BS>;
   static bool opted[16] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 16 || !opted[dev]) {
-    TPX_CUDA_OK(cudaFuncSetAttribute(qlinear_i8_kernel<TOK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM));
+    TPX_CUDA_OK(cudaFuncSetAttribute(qlinear_i8_kernel<TOK, BS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM));
     if (dev >= 0 && dev < 16) opted[dev] = true;
   }
   cudaLaunchConfig_t cfg = {};
@@ -516,7 +558,7 @@ static int i8_launch(const CUtensorMap& w, const CUtensorMap& x, I8Params p, int
       cfg.gridDim = dim3((unsigned)(tiles * c));
       cfg.numAttrs = 2;
       int n = 0;
-      cudaError_t e = cudaOccupancyMaxActiveClusters(&n, qlinear_i8_kernel<TOK>, &cfg);
+      cudaError_t e = cudaOccupancyMaxActiveClusters(&n, qlinear_i8_kernel<TOK, BS>, &cfg);
       if (e != cudaSuccess) { n = 0; (void)cudaGetLastError(); }
       f = 1 + n;
     }
@@ -528,8 +570,18 @@ static int i8_launch(const CUtensorMap& w, const CUtensorMap& x, I8Params p, int
   cfg.gridDim = dim3((unsigned)(tiles * c));
   cfg.numAttrs = c > 1 ? 2 : 1;
   count_launch();
-  TPX_CUDA_OK(cudaLaunchKernelEx(&cfg, qlinear_i8_kernel<TOK>, w, x, p));
+  TPX_CUDA_OK(cudaLaunchKernelEx(&cfg, qlinear_i8_kernel<TOK, BS>, w, p));
   return TPX_OK;
+}
+
+template <int BS>
+static int i8_launch_tok(int tokp, const CUtensorMap& w, const I8Params& p, int tiles, cudaStream_t st) {
+  switch (tokp) {
+    case 16: return i8_launch<16, BS>(w, p, tiles, st);
+    case 32: return i8_launch<32, BS>(w, p, tiles, st);
+    case 64: return i8_launch<64, BS>(w, p, tiles, st);
+    default: return i8_launch<128, BS>(w, p, tiles, st);
+  }
 }
 
 static int make_map_u8(CUtensorMap* m, const void* base, uint64_t rows, uint64_t row_bytes, uint32_t box_rows) {
@@ -604,35 +656,35 @@ extern "C" int tpx_qlinear_qint8_tc(const int8_t* wq, const float* swT, const ui
               scratch_bytes);
   cudaStream_t st = (cudaStream_t)stream;
   unsigned char* sc = reinterpret_cast<unsigned char*>(scratch);
-  int8_t* xq = reinterpret_cast<int8_t*>(sc + pl.off_xq);
-  float* sx = reinterpret_cast<float*>(sc + pl.off_sx);
-  if (!reuse_act && pl.Kp != K) TPX_CUDA_OK(cudaMemsetAsync(xq, 0, (size_t)pl.Mp * pl.Kp, st));  // the k padding reads as zero
+  uint8_t* xq = sc + pl.off_xq;
+  const I8Act L(pl.tokp, pl.ksteps, (int)block_size);
+  if (!reuse_act && pl.Kp != K) TPX_CUDA_OK(cudaMemsetAsync(xq, 0, pl.xq_bytes, st));  // the k padding reads as zero
   TPX_REQUIRE(!gamma || (K <= 8192 && block_size <= 256 && ((uintptr_t)gamma & 15) == 0), TPX_ERR_UNSUPPORTED,
               "qlinear_qint8_tc: the fused RMSNorm takes rows of up to 8192 values, blocks of up to 256 and a 16-byte aligned gamma");
-  if (!reuse_act && block_size <= 256) {
-    TPX_CUDA_OK(launch_pdl(quantize_act_i8_row_kernel, dim3((unsigned)pl.Mp), dim3(kQaThreads), 0, st, x, gamma, gamma_is_f32, eps, (int)M,
-                           (int)K, (int)pl.Kp, (int)block_size, (int)pl.Mp, xq, sx));
+  if (!reuse_act && gamma) {
+    TPX_CUDA_OK(launch_pdl(quantize_act_i8_row_kernel<4>, dim3((unsigned)pl.Mp), dim3(kQaThreads), 0, st, x, gamma, gamma_is_f32, eps, (int)M,
+                           (int)K, L, xq));
+  } else if (!reuse_act && block_size <= 256) {
+    TPX_CUDA_OK(launch_pdl(quantize_act_i8_row_kernel<1>, dim3((unsigned)pl.Mp, (unsigned)((K / 8 + kQaThreads - 1) / kQaThreads)), dim3(kQaThreads), 0,
+                           st, x, gamma, gamma_is_f32, eps, (int)M, (int)K, L, xq));
   } else if (!reuse_act) {
     const long long threads = (long long)pl.Mp * (K / block_size);
-    TPX_CUDA_OK(launch_pdl(quantize_act_i8_kernel, dim3((unsigned)((threads + 127) / 128)), dim3(128), 0, st, x, (int)M, (int)K, (int)pl.Kp,
-                           (int)block_size, (int)pl.Mp, xq, sx));
+    TPX_CUDA_OK(launch_pdl(quantize_act_i8_kernel, dim3((unsigned)((threads + 127) / 128)), dim3(128), 0, st, x, (int)M, (int)K, (int)pl.Mp, L, xq));
   }
-  CUtensorMap mw, mx;
+  CUtensorMap mw;
   int rc = make_map_u8(&mw, wq, (uint64_t)pl.Np, (uint64_t)pl.Kp, 128);
-  if (rc) return rc;
-  rc = make_map_u8(&mx, xq, (uint64_t)pl.Mp, (uint64_t)pl.Kp, (uint32_t)pl.tokp);
   if (rc) return rc;
   I8Params p = {};
   p.t.bias = bias; p.t.mul_in = mul_in; p.t.res = res; p.t.res_scale = res_scale; p.t.y = y; p.t.act = act;
   p.t.M = (int)M; p.t.N = (int)N; p.t.K = (int)K; p.t.cluster = pl.cluster;
   p.t.err = reinterpret_cast<unsigned*>(sc + kTcCounterBytes - 4);
-  p.swT = swT; p.sx = sx; p.ksteps = pl.ksteps; p.bsteps = (int)(block_size / 32); p.Np = (int)pl.Np; p.nblk = (int)(K / block_size);
-  p.tilesN = (int)(pl.Np / 128); p.Mp = (int)pl.Mp;
-  switch (pl.tokp) {
-    case 16: return i8_launch<16>(mw, mx, p, pl.tiles, st);
-    case 32: return i8_launch<32>(mw, mx, p, pl.tiles, st);
-    case 64: return i8_launch<64>(mw, mx, p, pl.tiles, st);
-    default: return i8_launch<128>(mw, mx, p, pl.tiles, st);
+  p.swT = swT; p.xq = xq; p.ksteps = pl.ksteps; p.Np = (int)pl.Np; p.nblk = (int)(K / block_size);
+  p.tilesN = (int)(pl.Np / 128);
+  switch (block_size) {
+    case 64: return i8_launch_tok<2>(pl.tokp, mw, p, pl.tiles, st);
+    case 128: return i8_launch_tok<4>(pl.tokp, mw, p, pl.tiles, st);
+    case 256: return i8_launch_tok<8>(pl.tokp, mw, p, pl.tiles, st);
+    default: return i8_launch_tok<16>(pl.tokp, mw, p, pl.tiles, st);
   }
 }
 
