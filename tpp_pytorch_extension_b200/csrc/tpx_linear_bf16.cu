@@ -170,83 +170,100 @@ linear_bf16_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   const uint32_t tmem = tmem_holder;
   pdl_trigger();
 
+  // Loop state of the two issuing warps is the same in all lanes, with a stage counter and its parity instead of divisions of a
+  // running number, and only the issue itself is under an elected lane.
   if (warp == 0) {
     // ------------------------------------------------------------ producer
-    if (tc_elect()) {
-      // at decode sizes W is a model's weight, not the output of a kernel in flight: its copies for the first stages need not
-      // wait for the kernels that make x (many rows may come with a weight unpacked for the call)
-      auto copy_w = [&](int tile, int g, int s) {
-        const uint32_t st = smem_base + (uint32_t)s * C::STAGE_BYTES;
-        const uint32_t bar = tc_smem_u32(&bar_full[s]);
-        tc_mbar_expect_tx(bar, C::STAGE_BYTES);
+    // at decode sizes W is a model's weight, not the output of a kernel in flight: its copies for the first stages need not
+    // wait for the kernels that make x (many rows may come with a weight unpacked for the call)
+    auto copy_w = [&](int row, int g, int s) {
+      const uint32_t st = smem_base + (uint32_t)s * C::STAGE_BYTES;
+      const uint32_t bar = tc_smem_u32(&bar_full[s]);
+      tc_mbar_expect_tx(bar, C::STAGE_BYTES);
 #pragma unroll
-        for (int u = 0; u < C::UK; u++)  // a k step beyond K reads as zeros
-          tc_tma_2d(st + u * C::A_BYTES, &tmW, (g * C::UK + u) * 64, tile / p.TM * 128, bar);
-      };
-      auto copy_x = [&](int tile, int g, int s) {
-        const uint32_t st = smem_base + (uint32_t)s * C::STAGE_BYTES;
-        const uint32_t bar = tc_smem_u32(&bar_full[s]);
+      for (int u = 0; u < C::UK; u++)  // a k step beyond K reads as zeros
+        tc_tma_2d(st + u * C::A_BYTES, &tmW, (g * C::UK + u) * 64, row, bar);
+    };
+    auto copy_x = [&](int row, int g, int s) {
+      const uint32_t st = smem_base + (uint32_t)s * C::STAGE_BYTES;
+      const uint32_t bar = tc_smem_u32(&bar_full[s]);
 #pragma unroll
-        for (int u = 0; u < C::UK; u++)
-          tc_tma_2d(st + C::UK * C::A_BYTES + u * C::B_BYTES, &tmX, (g * C::UK + u) * 64, tile % p.TM * TOK, bar);
-      };
-      BfPieces ahead(p, nstages);
-      int pre = 0;
-      while (TOK <= 64 && pre < C::STAGES && ahead.next())
-        for (int g = ahead.g0; g < ahead.g1 && pre < C::STAGES; g++) copy_w(ahead.tile, g, pre++);
-      pdl_wait();
-      BfPieces pc(p, nstages);
-      long long it = 0;
-      bool dead = false;
-      while (!dead && pc.next()) {
-        for (int g = pc.g0; g < pc.g1; g++, it++) {
-          const int s = (int)(it % C::STAGES);
-          if (it >= C::STAGES && !tc_wait(tc_smem_u32(&bar_empty[s]), (uint32_t)((it / C::STAGES - 1) & 1))) {
-            atomicExch(p.t.err, 2u);
-            dead = true;
-            break;
-          }
-          if (it >= pre) copy_w(pc.tile, g, s);
-          copy_x(pc.tile, g, s);
-        }
+      for (int u = 0; u < C::UK; u++)
+        tc_tma_2d(st + C::UK * C::A_BYTES + u * C::B_BYTES, &tmX, (g * C::UK + u) * 64, row, bar);
+    };
+    BfPieces ahead(p, nstages);
+    int pre = 0;
+    while (TOK <= 64 && pre < C::STAGES && ahead.next()) {
+      const int wrow = ahead.tile / p.TM * 128;
+      for (int g = ahead.g0; g < ahead.g1 && pre < C::STAGES; g++, pre++) {
+        if (tc_elect()) copy_w(wrow, g, pre);
+        __syncwarp();
       }
     }
-    __syncwarp();
+    pdl_wait();
+    BfPieces pc(p, nstages);
+    int s = 0, filled = 0;  // filled: stages whose weights went out ahead and whose turn has come, at most `pre`
+    uint32_t phase = 1;     // parity to wait for on bar_empty: the first round over the ring finds every stage free
+    bool dead = false;
+    while (!dead && pc.next()) {
+      const int wrow = pc.tile / p.TM * 128, xrow = pc.tile % p.TM * TOK;
+      for (int g = pc.g0; g < pc.g1; g++) {
+        if (!tc_wait(tc_smem_u32(&bar_empty[s]), phase)) {
+          if (tc_elect()) atomicExch(p.t.err, 2u);
+          dead = true;
+          break;
+        }
+        const bool have = filled < pre;
+        if (tc_elect()) {
+          if (!have) copy_w(wrow, g, s);
+          copy_x(xrow, g, s);
+        }
+        __syncwarp();
+        if (have) filled++;
+        if (++s == C::STAGES) s = 0, phase ^= 1u;
+      }
+    }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (tc_elect()) {
-      // kind::f16: D = F32 (1), A = B = BF16 (1), both K-major, N = TOK, M = 128
-      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TOK >> 3) << 17) | ((128u >> 4) << 24);
-      long long it = 0;
-      uint32_t empty_phase = 0;  // bit b: parity to wait for on acc_empty[b]
-      bool dead = false;
-      BfPieces pc(p, nstages);
-      for (int i = 0; !dead && pc.next(); i++) {
-        const int buf = i & 1;
-        if (i >= 2) {  // the epilogue must have drained this accumulator
-          if (!tc_wait(tc_smem_u32(&acc_empty[buf]), (empty_phase >> buf) & 1u)) { atomicExch(p.t.err, 3u); break; }
-          empty_phase ^= 1u << buf;
-          tc_fence_after();
+    // kind::f16: D = F32 (1), A = B = BF16 (1), both K-major, N = TOK, M = 128
+    constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TOK >> 3) << 17) | ((128u >> 4) << 24);
+    const uint64_t desc0 = tc_smem_desc(smem_base);
+    int s = 0;
+    uint32_t phase = 0, empty_phase = 0;  // empty_phase: bit b: parity to wait for on acc_empty[b]
+    bool dead = false;
+    BfPieces pc(p, nstages);
+    for (int i = 0; !dead && pc.next(); i++) {
+      const int buf = i & 1;
+      if (i >= 2) {  // the epilogue must have drained this accumulator
+        if (!tc_wait(tc_smem_u32(&acc_empty[buf]), (empty_phase >> buf) & 1u)) {
+          if (tc_elect()) atomicExch(p.t.err, 3u);
+          break;
         }
-        for (int g = pc.g0; g < pc.g1; g++, it++) {
-          const int s = (int)(it % C::STAGES);
-          if (!tc_wait(tc_smem_u32(&bar_full[s]), (uint32_t)((it / C::STAGES) & 1))) { atomicExch(p.t.err, 4u); dead = true; break; }
-          tc_fence_after();
-          const uint32_t st = smem_base + (uint32_t)s * C::STAGE_BYTES;
+        empty_phase ^= 1u << buf;
+        tc_fence_after();
+      }
+      for (int g = pc.g0; g < pc.g1; g++) {
+        if (!tc_wait(tc_smem_u32(&bar_full[s]), phase)) {
+          if (tc_elect()) atomicExch(p.t.err, 4u);
+          dead = true;
+          break;
+        }
+        tc_fence_after();
+        if (tc_elect()) {
+          const uint64_t desc = desc0 + (uint64_t)(s * (C::STAGE_BYTES >> 4));  // descriptors count 16-byte units
 #pragma unroll
-          for (int u = 0; u < C::UK; u++) {
+          for (int u = 0; u < C::UK; u++)
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
-              bf_mma(tmem + buf * TOK, tc_smem_desc(st + u * C::A_BYTES) + (uint64_t)(2 * j),
-                     tc_smem_desc(st + C::UK * C::A_BYTES + u * C::B_BYTES) + (uint64_t)(2 * j), idesc, (g == pc.g0 && u == 0 && j == 0) ? 0u : 1u);
-            }
-          }
+            for (int j = 0; j < 4; j++)
+              bf_mma(tmem + buf * TOK, desc + (uint64_t)(u * (C::A_BYTES >> 4) + 2 * j),
+                     desc + (uint64_t)((C::UK * C::A_BYTES + u * C::B_BYTES) / 16 + 2 * j), idesc, (g > pc.g0 || u || j) ? 1u : 0u);
           tc_commit(tc_smem_u32(&bar_empty[s]));
+          if (g == pc.g1 - 1) tc_commit(tc_smem_u32(&acc_full[buf]));
         }
-        if (!dead) tc_commit(tc_smem_u32(&acc_full[buf]));
+        __syncwarp();
+        if (++s == C::STAGES) s = 0, phase ^= 1u;
       }
     }
-    __syncwarp();
   } else {
     // ------------------------------------------------------------ epilogue (warps 2..5)
     const int sub = warp & 3;  // tensor-memory lanes 32*sub .. 32*sub+31 belong to this warp
