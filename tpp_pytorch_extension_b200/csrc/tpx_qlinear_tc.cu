@@ -1008,6 +1008,8 @@ extern "C" int tpx_repack_mxfp4_tc(const uint8_t* codes, const uint8_t* scales, 
 // below follows a sweep of both kernels over the linear shapes of Llama-3-8B, Llama-2-7B and Llama-2-70B (2 and 8
 // tensor-parallel ranks) at 1 to 64 tokens, launches back to back. TPX_TC_WIDE=1 forces the wide kernel for every
 // M <= 64, TPX_TC_WIDE=0 disables it.
+// A gate/up pair that may hand its output to the next linear as activation terms: the 128-row kernel cannot, families 1 and 2 can.
+static bool tc_hands_over(int64_t M, bool pair) { return pair && M >= knobs().handoff_min && M <= 64; }
 static bool tc_wide(int64_t M, int64_t N, int64_t K, bool pair) {
   if (M > 64) return false;
   if (knobs().tc_wide >= 0) return knobs().tc_wide != 0;
@@ -1016,29 +1018,26 @@ static bool tc_wide(int64_t M, int64_t N, int64_t K, bool pair) {
   auto whole = [&](long long T) { return (T * 10 >= (long long)sms * 7 && T <= sms) || T >= 8LL * sms; };
   const long long T0 = (N + 127) / 128;                        // tiles of the 128-row kernel (a pair: pair tiles)
   const long long T1 = pair ? (N + 127) / 128 : (N + 255) / 256;  // tiles of the wide kernel
+  // Up to 16 tokens the 128-row kernel's MMAs are as short as they get: faster where a CTA or a cluster owns whole tiles (14336 x 4096
+  // pair at 16 tokens: 16.9 against 18.5 us; 4096 x 4096: 8.5 / 9.9; 4096 x 14336: 13.7 / 15.1; 7168 x 8192 pair: 19.0 / 19.3), not
+  // where it has to cut tiles between CTAs (11008 x 4096 pair: 20.7 / 20.4; 12288 x 4096: 13.1 / 12.8).
+  if (M <= 16 && !tc_hands_over(M, pair) && (whole(T0) || T0 * 2 <= sms)) return false;
   if (whole(T1)) return true;  // every CTA owns whole tiles
-  // A pair has the same tiles in both kernels; the wide one measured faster or equal at every token count (Llama-2-7B
+  // A pair has the same tiles in both kernels; beyond 16 tokens the wide one measured faster or equal at every token count (Llama-2-7B
   // gate/up, 86 tiles, 64 tokens: 28.5 against 41.2 us; 28 tiles of K = 8192: 24.8 against 28.8 us).
   if (pair) return true;
   if (whole(T0)) return false;
   // The 128-row kernel would cut tiles between CTAs and add a fix-up pass; the wide kernel has half as many tiles and
   // can usually split K inside clusters (q/k/v of 12288 features, 64 tokens: 20.2 against 27.2 us).
   if (T0 * 2 > sms) return true;
-  // Both split K inside clusters. Up to 16 tokens the wide kernel: launched back to back the 128-row kernel measured
-  // faster at 16 tokens (4096 x 14336: 17.6 against 19.5 us) but a whole Llama-3-8B decode step at batch 16 slower (4.13
-  // against 3.96 ms), so the choice follows the model-level measurement. Beyond 16 tokens the 128-row kernel has the
-  // shorter epilogue (4096 x 4096 at 64 tokens: 16.4 against 19.2 us).
-  return M <= 16;
+  // Both split K inside clusters: the 128-row kernel has the shorter epilogue (4096 x 4096 at 64 tokens: 13.9 against 15.9 us).
+  return false;
 }
 
 // Kernel family for a call: 0 = weights on the 128-row side (all M), 1 = weights on the N side (M <= 64),
-// 2 = packed-fp4 operands (M <= 32). Default where every CTA owns whole tiles (the gate/up pair of a decode step:
-// 20.0 against 24.3 us at M = 8, 23.2 against 26.2 us at M = 32, launches back to back; Llama-3-8B decodes at 2.81
-// against 2.94 ms/token). Not where tiles are cut between CTAs with a fix-up pass: single launches measured faster up
-// to 16 tokens (gate/up pair of 11008 features: 22.2 against 24.3 us at M = 8) but a whole model slower (Llama-2-7B,
-// its q/k/v and gate/up linears on this family: 2.76 against 2.66 ms/token). Not where few tiles cut K inside a
-// cluster either (down projection: 19.4 against 18.7 us at M = 8). TPX_TC_F4=1 selects it for every M <= 32,
-// TPX_TC_F4=0 never.
+// 2 = packed-fp4 operands (M <= 32), only with TPX_TC_F4=1 or for a pair of whole tiles that TPX_HANDOFF_MIN_TOKENS lets hand over: four E2M1 terms per activation paid while a short MMA cost the issuing
+// thread as much as a long one; with issue under an elected lane families 0 and 1 are faster at every shape measured (14336 x 4096
+// pair at 8 tokens: 16.5 against 16.9 us, at 32: 18.6 against 22.1; 11008 x 4096: 12.1 against 14.3 us).
 constexpr int kW4AutoMaxTokens = 0;  // token counts up to which family 3 is chosen without being asked for
 static int tc_kind(int64_t M, int64_t N, int64_t K, bool pair) {
   // 3 = weights on the N side with packed-fp4 operands (tpx_qlinear_tcw4.cu): the default up to 32 tokens wherever its
@@ -1050,11 +1049,8 @@ static int tc_kind(int64_t M, int64_t N, int64_t K, bool pair) {
     if (w4 != 0 && (w4 > 0 || (!other_forced && M <= kW4AutoMaxTokens)) && tcw4_serves(M, N, K, pair)) return 3;
   }
   if (M <= 32) {
-    const int forced = knobs().tc_f4;
-    const long long T = (N + 127) / 128;  // one token tile up to 32 tokens
-    const int sms = sm_count();
-    const bool whole = (T * 10 >= (long long)sms * 7 && T <= sms) || T >= 8LL * sms;
-    if (forced >= 0 ? forced != 0 : whole) return 2;
+    const long long T = (N + 127) / 128, sms = sm_count();
+    if (knobs().tc_f4 > 0 || (knobs().tc_f4 < 0 && tc_hands_over(M, pair) && ((T * 10 >= sms * 7 && T <= sms) || T >= 8 * sms))) return 2;
   }
   if (tcp2_serves(M, N, K, pair)) return 5;  // many tokens on CTA pairs
   if (tcp_serves(M, N, K, pair)) return 4;  // many tokens in whole tiles: the kernel with overlapped epilogue
