@@ -238,12 +238,15 @@ __global__ void rope_kv_v8_kernel(const uint16_t* __restrict__ qkv, const float*
   const int heads = Nq + 2 * Nkv;
   const int half = H / 2, groups = half / 8;
   const int64_t offset = dev_len ? (int64_t)*dev_len : offset_arg;
-  int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= (int64_t)B * S * heads * groups) return;
-  const int h2 = (int)(idx % groups) * 8;
-  const int hd = (int)((idx / groups) % heads);
-  const int s = (int)((idx / ((int64_t)groups * heads)) % S);
-  const int b = (int)(idx / ((int64_t)groups * heads * S));
+  // `chunks` CTAs per token, so that the token is found in 32 bits instead of by four 64-bit divisions per thread (16 x 2048 tokens, 96
+  // heads of 128: 635 -> 607 us; 1.6 GB of copies with pieces of 256 bytes on one side bound it)
+  const unsigned per = (unsigned)(heads * groups), chunks = (per + blockDim.x - 1) / blockDim.x;
+  const unsigned tok = blockIdx.x / chunks, i = blockIdx.x % chunks * blockDim.x + threadIdx.x;
+  if (i >= per) return;
+  const int h2 = (int)(i % groups) * 8;
+  const int hd = (int)(i / groups);
+  const int s = (int)(tok % S);
+  const int b = (int)(tok / S);
   const uint16_t* src = qkv + ((int64_t)(b * S + s) * heads + hd) * H;
   uint4 lo = *reinterpret_cast<const uint4*>(src + h2), hi = *reinterpret_cast<const uint4*>(src + h2 + half);
   if (hd < Nq + Nkv) {
@@ -784,8 +787,9 @@ static int rope_kv_update_impl(const uint16_t* qkv, const float* ep, const int64
   if (S == 0) return TPX_OK;
   const bool aligned = (((uintptr_t)qkv | (uintptr_t)ep | (uintptr_t)q_out | (uintptr_t)kc | (uintptr_t)vc) & 15) == 0;
   if (H % 16 == 0 && aligned) {  // pages are whole [B][Nkv][32][H] slabs of an aligned allocation
-    int64_t total8 = B * S * (Nq + 2 * Nkv) * (H / 16);
-    TPX_CUDA_OK(launch_pdl(rope_kv_v8_kernel, dim3((unsigned)((total8 + 255) / 256)), dim3(256), 0, (cudaStream_t)stream, qkv, ep, pos, (int)B,
+    const int64_t per = (Nq + 2 * Nkv) * (H / 16), block = per < 256 ? (per + 31) / 32 * 32 : 256, ctas = B * S * ((per + block - 1) / block);
+    TPX_REQUIRE(ctas < (1ll << 31), TPX_ERR_UNSUPPORTED, "rope_kv_update: too many tokens in one call");
+    TPX_CUDA_OK(launch_pdl(rope_kv_v8_kernel, dim3((unsigned)ctas), dim3((unsigned)block), 0, (cudaStream_t)stream, qkv, ep, pos, (int)B,
                            (int)S, (int)Nq, (int)Nkv, (int)H, (int)MP, (int)HR, (int)Bpos, offset, dev_len, capacity, q_out, kc, vc, kpages, vpages));
     return TPX_OK;
   }
