@@ -797,13 +797,14 @@ def run_ours(args):
             "config": workload_config(),
             "prefill": {"tflops": world * pre_flops / (pre_ms * 1e-3) / 1e12 if pre_ms > 0 else None, "unit": "TFLOP/s",
                         "frac_of_bf16_peak": pre_flops / (pre_ms * 1e-3) / 1e12 / pk["bf16_tflops"] if pre_ms > 0 else None,
-                        # the prefill kernel issues kind::mxf8f6f4 MMAs, which run at the 8-bit rate (twice the bf16 rate)
+                        # below 2048 (gate/up) or 4096 tokens the kernel issues kind::mxf8f6f4 MMAs at the 8-bit rate (twice the bf16 rate), from
+                        # there on kind::f16 on the unpacked weight
                         "frac_of_issued_kind_peak": pre_flops / (pre_ms * 1e-3) / 1e12 / (2 * pk["bf16_tflops"]) if pre_ms > 0 else None,
-                        "issued_kind_peak": "2 x the bf16 cuBLAS burst figure (no 8-bit GEMM peak is measured on this pool)",
+                        "issued_kind_peak": "2 x the bf16 cuBLAS burst figure (no 8-bit GEMM peak is measured on this pool); calls on the unpacked weight issue bf16 MMAs",
                         "peak_src": pk["src"], "clocks": pre_clocks, "rounds": pre_rounds},
             "roofline": {"bound": "hbm",
-                         "kernel": f"MXFP4 gate/up pair GEMM, M={SWEEP[dom]} (tcgen05: qlinear_tc4_kernel, kind::mxf4, for M <= 32; "
-                                   f"qlinear_tcw_kernel, kind::mxf8f6f4, for M <= 64; qlinear_tcp2_kernel, cta_group::2, beyond)"
+                         "kernel": f"MXFP4 gate/up pair GEMM, M={SWEEP[dom]} (tcgen05: qlinear_tc_kernel for M <= 16, "
+                                   f"qlinear_tcw_kernel for M <= 64, both kind::mxf8f6f4; cta_group::2 kernels beyond)"
                                    if F.mxfp4_path() == "tc" else f"qlinear_stream gate/up pair, M={SWEEP[dom]}",
                          "achieved": dom_gbs, "peak": pk["hbm_gbs"], "unit": "GB/s", "frac": dom_gbs / pk["hbm_gbs"],
                          "peak_src": pk["src"], "traffic": NCU_TRAFFIC.get(SWEEP[dom]),
