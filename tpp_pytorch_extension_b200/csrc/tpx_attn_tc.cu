@@ -265,7 +265,17 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       float t4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
       for (int i = 0; i < 32; i++) t4[i & 3] = fmaxf(t4[i & 3], x[i]);
-      xmax[s][part][rl] = fmaxf(fmaxf(t4[0], t4[1]), fmaxf(t4[2], t4[3])) * unit;
+      const float top = fmaxf(fmaxf(t4[0], t4[1]), fmaxf(t4[2], t4[3]));
+      // The multiply-add takes the rounded maximum off an unrounded score: the weight of the maximum is then 2^r with r up to half an ulp
+      // of the maximum, which is nothing for ordinary scores but infinite from 2^31 on. Large scores are rounded first: r = 0.
+      if (unit != 1.0f && !(fabsf(top) * unit < 4096.0f)) {
+#pragma unroll
+        for (int i = 0; i < 32; i++) x[i] *= unit;
+        xmax[s][part][rl] = top * unit;
+        unit = 1.0f;
+      } else {
+        xmax[s][part][rl] = top * unit;
+      }
       asm volatile("bar.sync %0, 128;" ::"r"(1 + sub) : "memory");  // the four warps of this quarter
       const float tmax = fmaxf(fmaxf(xmax[s][0][rl], xmax[s][1][rl]), fmaxf(xmax[s][2][rl], xmax[s][3][rl]));
       const float m_new = fmaxf(m_run, tmax);
