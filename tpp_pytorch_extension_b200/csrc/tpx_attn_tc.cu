@@ -213,10 +213,14 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
 #pragma unroll
     for (int i = 0; i < HP; i++) o[i] = 0.0f;
     float m_run = -INFINITY, l_run = 0.0f, alpha_prev = 1.0f;
-    bool dead = false;
+    bool dead = false;  // a warp that gave up still meets the others of its quarter at their barriers
 
     auto accumulate = [&](int t, float alpha) {  // o = o * alpha + T_t (this warp's columns)
-      if (!tc_wait(tc_smem_u32(&o_full), (uint32_t)(t & 1))) { atomicExch(&g_attn_tc_err, 7u); dead = true; return; }
+      if (!tc_wait_warp(tc_smem_u32(&o_full), (uint32_t)(t & 1))) {
+        if (lane == 0) atomicExch(&g_attn_tc_err, 7u);
+        dead = true;
+        return;
+      }
       tc_fence_after();
       uint32_t v[HP];
       if (HP == 32) {
@@ -231,7 +235,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       tc_mbar_arrive(tc_smem_u32(&o_free));
     };
 
-    for (int j = 0; j < ntiles && !dead; j++) {
+    for (int j = 0; j < ntiles; j++) {
       const int s = j & 1;
       const int k0 = j * 128 + part * 32;  // this thread's 32 keys
       // The mask of the warp's 32 keys, one per lane. Almost everywhere it is zero (prompts of one length, and all but the padding of
@@ -242,7 +246,14 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       float drop = 0.0f;
       if (am && k0 + lane < p.Spad) drop = fmaxf(bf16_bits_to_f32(am[k0 + lane]) * 1.4426950408889634f, -3.0e38f);
       const bool masked = __any_sync(0xffffffffu, drop != 0.0f);
-      if (!tc_wait(tc_smem_u32(&s_full[s]), (uint32_t)((j >> 1) & 1))) { atomicExch(&g_attn_tc_err, 8u); dead = true; break; }
+      if (!dead && !tc_wait_warp(tc_smem_u32(&s_full[s]), (uint32_t)((j >> 1) & 1))) {
+        if (lane == 0) atomicExch(&g_attn_tc_err, 8u);
+        dead = true;
+      }
+      if (dead) {
+        asm volatile("bar.sync %0, 128;" ::"r"(1 + sub) : "memory");
+        continue;
+      }
       tc_fence_after();
       uint32_t v[32];
       at_ld_x32(tmem + lane_base + C::COL_S + s * 128 + part * 32, v);

@@ -152,16 +152,15 @@ __device__ __forceinline__ void bp_commit_both(uint32_t bar) {  // arrives on th
 __device__ __forceinline__ void bp_arrive_cluster(uint32_t cluster_bar) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
 }
-__device__ __forceinline__ bool bp_wait_cluster(uint32_t bar, uint32_t parity) {  // arrivals come from both CTAs
-  for (unsigned spins = 0; spins < kTcSpinLimit; spins++) {
-    uint32_t ok;
+__device__ __forceinline__ bool bp_wait_cluster(uint32_t bar, uint32_t parity) {  // arrivals come from both CTAs; one verdict per warp
+  uint32_t ok = 0;
+  for (unsigned spins = 0; spins < kTcSpinLimit && !ok; spins++) {
     asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
                  : "=r"(ok)
                  : "r"(bar), "r"(parity)
                  : "memory");
-    if (ok) return true;
   }
-  return false;
+  return __all_sync(0xffffffffu, ok != 0);
 }
 
 // Eight consecutive values; the caller guarantees 16-byte alignment.

@@ -208,7 +208,7 @@ linear_bf16_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     while (!dead && pc.next()) {
       const int wrow = pc.tile / p.TM * 128, xrow = pc.tile % p.TM * TOK;
       for (int g = pc.g0; g < pc.g1; g++) {
-        if (!tc_wait(tc_smem_u32(&bar_empty[s]), phase)) {
+        if (!tc_wait_warp(tc_smem_u32(&bar_empty[s]), phase)) {
           if (tc_elect()) atomicExch(p.t.err, 2u);
           dead = true;
           break;
@@ -235,7 +235,7 @@ linear_bf16_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     for (int i = 0; !dead && pc.next(); i++) {
       const int buf = i & 1;
       if (i >= 2) {  // the epilogue must have drained this accumulator
-        if (!tc_wait(tc_smem_u32(&acc_empty[buf]), (empty_phase >> buf) & 1u)) {
+        if (!tc_wait_warp(tc_smem_u32(&acc_empty[buf]), (empty_phase >> buf) & 1u)) {
           if (tc_elect()) atomicExch(p.t.err, 3u);
           break;
         }
@@ -243,7 +243,7 @@ linear_bf16_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
         tc_fence_after();
       }
       for (int g = pc.g0; g < pc.g1; g++) {
-        if (!tc_wait(tc_smem_u32(&bar_full[s]), phase)) {
+        if (!tc_wait_warp(tc_smem_u32(&bar_full[s]), phase)) {
           if (tc_elect()) atomicExch(p.t.err, 4u);
           dead = true;
           break;
@@ -275,7 +275,7 @@ linear_bf16_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     bool dead = false;  // a warp that gave up still meets the others at their barriers
     for (int i = 0; pc.next(); i++) {
       const int buf = i & 1;
-      if (!dead && !tc_wait(tc_smem_u32(&acc_full[buf]), (full_phase >> buf) & 1u)) {
+      if (!dead && !tc_wait_warp(tc_smem_u32(&acc_full[buf]), (full_phase >> buf) & 1u)) {
         if (lane == 0) atomicExch(p.t.err, 6u);
         dead = true;
       }

@@ -175,7 +175,7 @@ linear_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_co
     for (BpWork k(p); !dead && k.next();) {
       const int row = k.tm * 256 + crank * 128, col = k.tn * 256 + crank * 128;
       for (int g = k.g0; g < k.g1; g++) {
-        if (!tc_wait(tc_smem_u32(&bar_empty[s]), phase)) {
+        if (!tc_wait_warp(tc_smem_u32(&bar_empty[s]), phase)) {
           if (tc_elect()) atomicExch(p.t.err, 2u);
           dead = true;
           break;
@@ -210,7 +210,7 @@ linear_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_co
           tc_fence_after();
         }
         for (int g = k.g0; g < k.g1; g++) {
-          if (!tc_wait(tc_smem_u32(&bar_full[s]), phase)) {
+          if (!tc_wait_warp(tc_smem_u32(&bar_full[s]), phase)) {
             if (tc_elect()) atomicExch(p.t.err, 4u);
             dead = true;
             break;
@@ -240,7 +240,7 @@ linear_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_co
     bool dead = false;  // a warp that gave up still meets the others at their barriers
     for (BpWork k(p); k.next(); i++) {
       const int buf = i & 1;
-      if (!dead && !tc_wait(tc_smem_u32(&acc_full[buf]), (uint32_t)((i / 2) & 1))) {
+      if (!dead && !tc_wait_warp(tc_smem_u32(&acc_full[buf]), (uint32_t)((i / 2) & 1))) {
         if (lane == 0) atomicExch(p.t.err, 6u);
         dead = true;
       }

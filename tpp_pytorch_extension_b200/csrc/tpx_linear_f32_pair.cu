@@ -153,7 +153,7 @@ linear_f32_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_con
     for (BpWork k(p); !dead && k.next();) {
       const int row = k.tm * 256 + crank * 128, col = k.tn * 256 + crank * 128;
       for (int g = k.g0; g < k.g1; g++) {
-        if (!tc_wait(tc_smem_u32(&bar_empty[s]), phase)) {
+        if (!tc_wait_warp(tc_smem_u32(&bar_empty[s]), phase)) {
           if (tc_elect()) atomicExch(p.t.err, 2u);
           dead = true;
           break;
@@ -192,7 +192,7 @@ linear_f32_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_con
               break;
             }
           }
-          if (!tc_wait(tc_smem_u32(&bar_full[s]), phase)) {
+          if (!tc_wait_warp(tc_smem_u32(&bar_full[s]), phase)) {
             if (tc_elect()) atomicExch(p.t.err, 4u);
             dead = true;
             break;
@@ -226,7 +226,7 @@ linear_f32_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_con
       float acc[kBpEpiCols] = {};
       for (int g = k.g0; g < k.g1; g++, i++) {
         const int buf = i & 1;
-        if (!dead && !tc_wait(tc_smem_u32(&acc_full[buf]), (uint32_t)((i / 2) & 1))) {
+        if (!dead && !tc_wait_warp(tc_smem_u32(&acc_full[buf]), (uint32_t)((i / 2) & 1))) {
           if (lane == 0) atomicExch(p.t.err, 6u);
           dead = true;
         }

@@ -327,7 +327,7 @@ qlinear_i8_kernel(const __grid_constant__ CUtensorMap tmW, I8Params p) {
     uint32_t phase = 1;  // parity to wait for on bar_empty: the first round over the ring finds every stage free
     for (int it = 0; it < nsteps; it++) {
       if (it >= C::STAGES) {
-        if (!tc_wait(tc_smem_u32(&bar_empty[s]), phase)) {
+        if (!tc_wait_warp(tc_smem_u32(&bar_empty[s]), phase)) {
           if (tc_elect()) atomicExch(p.t.err, 2u);
           break;
         }
@@ -351,7 +351,7 @@ qlinear_i8_kernel(const __grid_constant__ CUtensorMap tmW, I8Params p) {
     for (int left = nsteps; !dead && left > 0; left -= C::SG, g++) {
       const int grp = g % C::NGRP;
       if (g >= C::NGRP) {  // a recycled group: the epilogue must have read it
-        if (!tc_wait(tc_smem_u32(&d_free[grp]), (uint32_t)((g / C::NGRP - 1) & 1))) {
+        if (!tc_wait_warp(tc_smem_u32(&d_free[grp]), (uint32_t)((g / C::NGRP - 1) & 1))) {
           if (tc_elect()) atomicExch(p.t.err, 3u);
           dead = true;
           break;
@@ -362,7 +362,7 @@ qlinear_i8_kernel(const __grid_constant__ CUtensorMap tmW, I8Params p) {
 #pragma unroll
       for (int t = 0; t < C::SG; t++) {
         if (t >= left || dead) continue;
-        if (!tc_wait(tc_smem_u32(&bar_full[s]), phase)) {
+        if (!tc_wait_warp(tc_smem_u32(&bar_full[s]), phase)) {
           if (tc_elect()) atomicExch(p.t.err, 4u);
           dead = true;
           continue;
@@ -412,7 +412,7 @@ qlinear_i8_kernel(const __grid_constant__ CUtensorMap tmW, I8Params p) {
         ok = ok && tc_wait(tc_smem_u32(&bar_full[s]), phase);
         if (++s == C::STAGES) s = 0, phase ^= 1u;
       }
-      if (!ok || !tc_wait(tc_smem_u32(&d_full[grp]), (uint32_t)((g / C::NGRP) & 1))) {
+      if (!__all_sync(0xffffffffu, ok && tc_wait(tc_smem_u32(&d_full[grp]), (uint32_t)((g / C::NGRP) & 1)))) {
         if (lane == 0) atomicExch(p.t.err, 6u);
         dead = true;
         break;

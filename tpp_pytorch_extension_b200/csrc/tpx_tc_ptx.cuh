@@ -99,6 +99,9 @@ __device__ __forceinline__ bool tc_wait(uint32_t bar, uint32_t parity) {
     if (tc_mbar_try_wait(bar, parity)) return true;
   return false;
 }
+// The same where a whole warp waits and then issues under tc_elect or meets other warps: one verdict for all lanes. With a verdict per
+// lane a barrier that flips just as some lanes run out of polls would leave the warp waiting for itself at the next warp-wide instruction.
+__device__ __forceinline__ bool tc_wait_warp(uint32_t bar, uint32_t parity) { return __all_sync(0xffffffffu, tc_wait(bar, parity)); }
 __device__ __forceinline__ void tc_tma_2d(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
