@@ -120,3 +120,33 @@ def test_f32_values_without_terms(bad, where):
     assert torch.equal(terms.isposinf(), plain.isposinf()) and torch.equal(terms.isneginf(), plain.isneginf())
     fine = plain.isfinite()
     assert torch.allclose(terms[fine], plain[fine], rtol=1e-3, atol=1e-3)
+
+
+@pytest.mark.parametrize("a,b", [(-112, 0), (-118, 10), (-126, 30), (-130, 60), (-140, 100), (0, -120), (-60, -62), (24, 24), (29, -140)])
+def test_f32_operands_of_any_size(a, b):
+    """Rows whose values are all near 2^a against weights near 2^b, down to subnormal ones: no further off than the CUDA cores."""
+    from tpp_pytorch_extension_b200 import _lib
+    M, N, K = 256, 1024, 2048
+    g = torch.Generator(device="cuda").manual_seed(a * 1000 + b + 200000)
+    x, w = (_rnd(g, *s, dtype=torch.float64).clamp(-1.9, 1.9) * 2.0 ** e for s, e in (((M, K), a), ((N, K), b)))
+    x, w = x.float(), w.float()
+    want = x.double() @ w.double().T
+    off = [float((_linear_f32(x, w, n).double() - want).norm() / want.norm()) for n in (_lib.lib().tpx_linear_f32_scratch_bytes(M, N, K), 65536)]
+    assert off[0] <= off[1] < 1e-5
+
+
+@pytest.mark.parametrize("u,v", [(3e38, 1e3), (-3e38, 1e3), (3e38, -1e30), (2.9e35, 1e9), (1.1e30, 3e12), (2.0 ** 30, 3e38)])
+def test_f32_products_beyond_the_range(u, v):
+    """Finite operands whose product overflows by any amount: infinities and NaN as on the CUDA cores, whatever the signs of the terms."""
+    from tpp_pytorch_extension_b200 import _lib
+    M, N, K = 200, 9000, 2048
+    g = _gen(M, N, K)
+    x, w = _rnd(g, M, K), _rnd(g, N, K)
+    x[7, 5], w[3, 5], w[N - 1, 5] = u, v, -v
+    x[8, 6], w[4, 6] = u * 0.9, v * 1.01  # other remainders
+    terms, plain = _linear_f32(x, w, _lib.lib().tpx_linear_f32_scratch_bytes(M, N, K)), _linear_f32(x, w, 65536)
+    assert plain.isinf().any()
+    assert torch.equal(terms.isnan(), plain.isnan())
+    assert torch.equal(terms.isposinf(), plain.isposinf()) and torch.equal(terms.isneginf(), plain.isneginf())
+    fine = plain.isfinite()
+    assert torch.allclose(terms[fine], plain[fine], rtol=1e-3, atol=1e-3)

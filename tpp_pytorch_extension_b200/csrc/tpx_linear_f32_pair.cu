@@ -1,7 +1,10 @@
-// 32-bit linear for many rows on the tensor cores, without loss: every fp32 operand is the sum of three bf16 terms
-// (x = h + m + l, each the rounding of what the terms before it left; 3 x 8 significand bits with signed remainders hold all 24),
-// and a product of two operands is the sum of the six products of terms that reach 2^-24 of it: hh, hm, mh, mm, hl, lh. bf16
-// products are exact in fp32. The three left out (ml, lm, ll) are below 2^-26.
+// 32-bit linear for many rows on the tensor cores: every fp32 operand is the sum of three bf16 terms (x = h + m + l, each the
+// rounding of what the terms before it left; 3 x 8 significand bits with signed remainders hold all 24), and a product of two
+// operands is taken as the sum of six products of terms: hh, hm, mh, mm, hl, lh. bf16 products are exact in fp32. The three left out
+// (ml, lm, ll) are together at most 2^-24 of the product (|m| <= 2^-8 |x|, |l| <= 2^-17 |x|).
+// Operands are multiplied by 2^24 before they are cut, sums by 2^-48 behind: the last bit of any fp32 value, subnormal ones
+// included, is then at least 2^-125, which bf16 terms (multiples of 2^-133) and their products hold. (Without it an operand of 2^-120
+// lost eight bits.) Operands of 2^30 and more are left to the CUDA cores, so that no sum of products of terms can overflow.
 //
 // Sums: the tensor core's own accumulation is kept short. 64 values of k (24 MMAs, the small terms first) accumulate in tensor
 // memory; then sixteen epilogue warps pull the accumulator and add it to fp32 registers with rounding to nearest, while the
@@ -10,8 +13,8 @@
 // Bounds: 6 bf16 products per fp32 product, i.e. a sixth of the bf16 rate; 96 KB per 64 values of k and CTA leave room for two
 // stages, and 3072 cycles of MMAs per stage hide the copies.
 // The terms are made per call in the scratch: all of x (up to kFpRows rows at a time), the weights in slabs small enough to
-// stay in L2 between the kernel that writes them and the one that reads them. An infinity or a NaN cannot be cut into terms:
-// the split kernels raise a flag for it, the tensor-core kernel then leaves that slab alone and linear_f32_kernel computes it.
+// stay in L2 between the kernel that writes them and the one that reads them. For an infinity, a NaN or a value of 2^30 and more the
+// split kernels raise a flag: the tensor-core kernel then leaves that slab alone and linear_f32_kernel computes it.
 #include "tpx_bf16_pair.cuh"
 
 namespace tpx {
@@ -19,6 +22,10 @@ namespace tpx {
 constexpr int64_t kFpRows = 2048;             // rows of x at a time
 constexpr int64_t kFpSlabBytes = 48ll << 20;  // terms of a slab of weight rows
 constexpr int kFpFlags = 128;                 // x, then one per slab
+
+constexpr float kFpScale = 16777216.0f, kFpUnscale = 1.0f / (kFpScale * kFpScale);  // 2^24, 2^-48
+constexpr float kFpLargest = 1073741824.0f;                                        // 2^30: K products stay below K 2^108
+constexpr int64_t kFpMostK = 1 << 19;
 
 constexpr double kFpUsPerStep = 1.7;
 
@@ -46,10 +53,10 @@ __global__ void __launch_bounds__(256) split3_kernel(const float* __restrict__ s
     bool odd = false;
 #pragma unroll
     for (int j = 0; j < 8; j++) {
-      const float h = __bfloat162float(__float2bfloat16_rn(v[j]));
-      const bool bad = (__float_as_uint(h) & 0x7f800000u) == 0x7f800000u;
+      const bool bad = !(fabsf(v[j]) < kFpLargest);
       odd |= bad;
-      const float r1 = bad ? 0.0f : v[j] - h;
+      v[j] *= kFpScale;
+      const float r1 = bad ? 0.0f : v[j] - __bfloat162float(__float2bfloat16_rn(v[j]));
       m[j] = __bfloat162float(__float2bfloat16_rn(r1));
       l[j] = r1 - m[j];
     }
@@ -256,7 +263,7 @@ linear_f32_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_con
       for (int c = 0; c < kBpEpiCols; c += 8) {
         float x[8];
 #pragma unroll
-        for (int j = 0; j < 8; j++) x[j] = acc[c + j];
+        for (int j = 0; j < 8; j++) x[j] = acc[c + j] * kFpUnscale;
         if (!dead && row < p.t.M && n0 + c < p.t.N) fp_finish8(e, row0 + row, n00 + n0 + c, x);
       }
     }
@@ -294,7 +301,7 @@ static FpPlan fp_plan(int64_t M, int64_t N, int64_t K) {
 
 // From 48 rows on and where the CUDA cores would take 40 us or more (they do 15 TFLOP/s); rows in whole 16-byte units of eight values.
 static bool fp_shape(int64_t M, int64_t N, int64_t K) {
-  return M >= 48 && K % 8 == 0 && N % 8 == 0 && 2.0 * M * N * K >= 6e8;
+  return M >= 48 && K % 8 == 0 && K <= kFpMostK && N % 8 == 0 && 2.0 * M * N * K >= 6e8;
 }
 size_t f32_pair_scratch_bytes(int64_t M, int64_t N, int64_t K) { return fp_shape(M, N, K) ? fp_plan(M, N, K).total : 0; }
 
