@@ -113,3 +113,17 @@ def test_argmax_rows_matches_torch(cuda):
     y = F.argmax_rows(x.to(cuda))
     assert y[1].item() == 100 and y[0].item() == int(x[0].float().argmax())
     assert F.argmax_rows(torch.empty(0, 16, dtype=torch.bfloat16, device=cuda)).shape == (0,)
+
+
+@pytest.mark.parametrize("N,K", [(256, 512), (1024, 2048), (49 * 128, 512), (50 * 128, 512)])
+def test_pairs_on_either_side_of_the_choice_of_kernel(cuda, N, K):
+    """Gate/up pairs of up to 16 tokens: few tiles on the wide kernel, from a third as many tiles as SMs (49 and 50) on the 128-row kernel."""
+    from tpp_pytorch_extension_b200._C import _fused_llm_infer as F
+    rng = np.random.default_rng(N + K)
+    qg, wg, _ = make_qweight(rng, N, K, "mxfp4", cuda)
+    qu, wu, _ = make_qweight(rng, N, K, "mxfp4", cuda)
+    for M in (1, 15, 16, 17):
+        x = O.randn_bf16(rng, (M, K))
+        y = to_host_bits(F.fc_gate_up(to_dev_bf16(x, cuda), qg, qu))
+        assert O.rel_err(y, O.gate_up(x, wg, wu)) <= 2e-2
+    assert_no_kernel_error()

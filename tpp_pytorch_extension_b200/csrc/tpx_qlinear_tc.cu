@@ -1020,8 +1020,11 @@ static bool tc_wide(int64_t M, int64_t N, int64_t K, bool pair) {
   const long long T1 = pair ? (N + 127) / 128 : (N + 255) / 256;  // tiles of the wide kernel
   // Up to 16 tokens the 128-row kernel's MMAs are as short as they get: faster where a CTA or a cluster owns whole tiles (14336 x 4096
   // pair at 16 tokens: 16.9 against 18.5 us; 4096 x 4096: 8.5 / 9.9; 4096 x 14336: 13.7 / 15.1; 7168 x 8192 pair: 19.0 / 19.3), not
-  // where it has to cut tiles between CTAs (11008 x 4096 pair: 20.7 / 20.4; 12288 x 4096: 13.1 / 12.8).
-  if (M <= 16 && !tc_hands_over(M, pair) && (whole(T0) || T0 * 2 <= sms)) return false;
+  // where it has to cut tiles between CTAs (11008 x 4096 pair: 20.7 / 20.4; 12288 x 4096: 13.1 / 12.8). A pair's cluster may have two CTAs: with
+  // more, both halves of every tile cross distributed shared memory many times for few k steps each (device times at 4 tokens: 1024 x 2048
+  // 10.9 against 8.3, 1024 x 4096 11.3 / 9.1, 2048 x 2048 10.3 / 8.8, 3584 x 8192 13.0 / 12.8; with two, 7168 x 8192 18.6 / 19.0), one weight's
+  // any size (2048 x 2048 7.5 / 7.6, 1024 x 8192 9.1 / 9.4, at 16 tokens 9.3 / 10.5). 8-bit weights: the same to 1 %.
+  if (M <= 16 && !tc_hands_over(M, pair) && (whole(T0) || (T0 * 2 <= sms && (!pair || T0 * 3 > sms)))) return false;
   if (whole(T1)) return true;  // every CTA owns whole tiles
   // A pair has the same tiles in both kernels; beyond 16 tokens the wide one measured faster or equal at every token count (Llama-2-7B
   // gate/up, 86 tiles, 64 tokens: 28.5 against 41.2 us; 28 tiles of K = 8192: 24.8 against 28.8 us).
