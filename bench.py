@@ -35,7 +35,7 @@ SWEEP = [1, 8, 64, 512, 4096]
 DECODE_MAX_M = 64
 # dram__bytes_read.sum + dram__bytes_write.sum of one gate/up launch of the tensor-core kernels, from the ncu captures
 # summarised under profiles/ (bytes); None where no capture exists
-NCU_TRAFFIC = {1: 63.02e6, 8: 63.02e6, 64: 63.82e6}  # M=1 runs the M=8 kernel instantiation on the same weight bytes
+NCU_TRAFFIC = {64: 63.82e6}
 N_COPIES = 6  # distinct packed weight sets: 6 x 93.6 MB = 561 MB >> 126 MB of L2
 
 
@@ -797,10 +797,7 @@ def run_ours(args):
             "config": workload_config(),
             "prefill": {"tflops": world * pre_flops / (pre_ms * 1e-3) / 1e12 if pre_ms > 0 else None, "unit": "TFLOP/s",
                         "frac_of_bf16_peak": pre_flops / (pre_ms * 1e-3) / 1e12 / pk["bf16_tflops"] if pre_ms > 0 else None,
-                        # below 2048 (gate/up) or 4096 tokens the kernel issues kind::mxf8f6f4 MMAs at the 8-bit rate (twice the bf16 rate), from
-                        # there on kind::f16 on the unpacked weight
-                        "frac_of_issued_kind_peak": pre_flops / (pre_ms * 1e-3) / 1e12 / (2 * pk["bf16_tflops"]) if pre_ms > 0 else None,
-                        "issued_kind_peak": "2 x the bf16 cuBLAS burst figure (no 8-bit GEMM peak is measured on this pool); calls on the unpacked weight issue bf16 MMAs",
+                        # 512 tokens run kind::mxf8f6f4 MMAs on the packed weight (twice the bf16 rate), 4096 kind::f16 on the unpacked one
                         "peak_src": pk["src"], "clocks": pre_clocks, "rounds": pre_rounds},
             "roofline": {"bound": "hbm",
                          "kernel": f"MXFP4 gate/up pair GEMM, M={SWEEP[dom]} (tcgen05: qlinear_tc_kernel for M <= 16, "
