@@ -68,12 +68,89 @@ __global__ void __launch_bounds__(128) diff_gather_kernel(TpxDiffAttn p) {
   for (int e = threadIdx.x; e < p.R; e += 128) dst[e] = src[e];
 }
 
-// ---------------------------------------------------------------- attention, any type and size: a warp per (QT tokens, head)
-// Lanes hold a key each for the scores and NR value columns each for the sums. With QT = 4 a key row, which every lane fetches on its
-// own, and a value row serve four tokens, and fp32 keys come in 16-byte pieces: one token per warp and 4-byte loads 32 rows apart
-// waited for L1 (2 x 513 tokens, 16 heads of 64 + 64 / 128 in fp32: 2380 us, now 544).
+// ---------------------------------------------------------------- attention, any type and size
 constexpr int kDiffWarps = 4;
 
+// A warp per (token, head) for bf16: lanes hold a key each for the scores and NR value columns each for the sums.
+template <typename T, int NR>
+__global__ void __launch_bounds__(kDiffWarps * 32) diff_attn_token_kernel(TpxDiffAttn p) {
+  extern __shared__ __align__(16) float df_q[];  // [warps][2 dim]
+  pdl_trigger();
+  pdl_wait();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t item = (int64_t)blockIdx.x * kDiffWarps + warp;
+  const int64_t row = item / p.heads;
+  const int head = (int)(item % p.heads), dim = (int)p.dim, vdim = (int)p.vdim, dp = (dim + 15) / 16 * 16;
+  if (row >= p.B * p.S) return;
+  const int64_t b = row / p.S, g = head / (p.heads / p.kv_heads);
+  const int64_t past = p.dev_len ? *p.dev_len : p.past, t = past + row % p.S;
+  const int64_t start = p.start ? p.start[b] : 0;
+  const int64_t lo = t < start ? t + 1 : start + (t - start) / p.chunk * p.chunk;  // padding sees nothing
+  float* q = df_q + warp * 2 * dim;
+  const T* pq = reinterpret_cast<const T*>(p.proj) + row * p.ldp + p.q_col + (int64_t)head * 2 * dim;
+  for (int i = lane; i < 2 * dim; i += 32) q[i] = hy_ld(pq + i) * p.scale;
+  __syncwarp();
+  auto key = [&](int64_t j) -> const T* {
+    if (p.live) return reinterpret_cast<const T*>(p.live) + ((b * p.L + j - (past - (p.L - p.S))) * p.kv_heads + g) * p.R;
+    return reinterpret_cast<const T*>(p.pages[(j / 32) % p.npages]) + ((b * p.kv_heads + g) * 32 + j % 32) * p.R;
+  };
+  float o[2][NR] = {}, mx[2] = {-INFINITY, -INFINITY}, sum[2] = {0.0f, 0.0f};
+  for (int64_t j0 = lo; j0 <= t; j0 += 32) {
+    const int n = (int)min((int64_t)32, t - j0 + 1);
+    float s[2] = {-INFINITY, -INFINITY};
+    if (lane < n) {
+      const T* k = key(j0 + lane);
+#pragma unroll
+      for (int m = 0; m < 2; m++) {
+        float a = 0.0f;
+        for (int c = 0; c < dim; c++) a = fmaf(q[m * dim + c], hy_ld(k + m * dp + c), a);
+        s[m] = p.softcap * tanhf(a / p.softcap);
+      }
+    }
+    float e[2];
+#pragma unroll
+    for (int m = 0; m < 2; m++) {
+      float x = s[m];
+#pragma unroll
+      for (int d = 16; d > 0; d >>= 1) x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, d));
+      const float mn = fmaxf(mx[m], x), al = expf(mx[m] - mn);
+      e[m] = lane < n ? expf(s[m] - mn) : 0.0f;
+      sum[m] = sum[m] * al + hy_warp_sum(e[m]);
+      mx[m] = mn;
+#pragma unroll
+      for (int i = 0; i < NR; i++) o[m][i] *= al;
+    }
+    for (int j = 0; j < n; j++) {
+      const T* v = key(j0 + j) + 2 * dp;
+      const float e1 = __shfl_sync(0xffffffffu, e[0], j), e2 = __shfl_sync(0xffffffffu, e[1], j);
+#pragma unroll
+      for (int i = 0; i < NR; i++)
+        if (lane + 32 * i < vdim) {
+          const float x = hy_ld(v + lane + 32 * i);
+          o[0][i] = fmaf(e1, x, o[0][i]);
+          o[1][i] = fmaf(e2, x, o[1][i]);
+        }
+    }
+  }
+  const float i1 = sum[0] > 0.0f ? 1.0f / sum[0] : 0.0f, i2 = sum[1] > 0.0f ? 1.0f / sum[1] : 0.0f;
+  float ss = 0.0f;
+#pragma unroll
+  for (int i = 0; i < NR; i++) {
+    o[0][i] = o[0][i] * i1 - p.lambda * (o[1][i] * i2);
+    ss = fmaf(o[0][i], o[0][i], ss);
+  }
+  const float inv = p.mult / sqrtf(hy_warp_sum(ss) / (float)vdim + p.eps);
+  T* out = reinterpret_cast<T*>(p.out) + row * p.ldo + (int64_t)head * vdim;
+#pragma unroll
+  for (int i = 0; i < NR; i++)
+    if (lane + 32 * i < vdim) hy_st(out + lane + 32 * i, o[0][i] * inv);
+}
+
+// The same for fp32, and for bf16 where it pays: a warp per (QT tokens, head).
+// Lanes hold a key each for the scores and NR value columns each for the sums. With QT = 4 a key row, which every lane fetches on its
+// own, and a value row serve four tokens, and fp32 keys come in 16-byte pieces: one token per warp and 4-byte loads 32 rows apart
+// waited for L1 (2 x 513 tokens, 16 heads of 64 + 64 / 128 in fp32: 2380 us, 850 with the pieces, 560 with four tokens). Scores of both maps come
+// first, then their reductions, whose shuffles fill each other's gaps.
 template <typename T, int NR, int QT>
 __global__ void __launch_bounds__(kDiffWarps * 32) diff_attn_kernel(TpxDiffAttn p) {
   extern __shared__ __align__(16) float df_q[];  // [warps][QT][2 dim]
@@ -111,7 +188,7 @@ __global__ void __launch_bounds__(kDiffWarps * 32) diff_attn_kernel(TpxDiffAttn 
   for (int i = 0; i < QT; i++) mx[i][0] = mx[i][1] = -INFINITY;
   for (int64_t j0 = from; j0 <= to; j0 += 32) {
     const int n = (int)min((int64_t)32, to - j0 + 1);
-    float e[QT][2];
+    float e[QT][2], s[QT][2];
     unsigned any[QT];  // the lanes' keys that a token sees
     const T* k = key(j0 + min(lane, n - 1));
 #pragma unroll
@@ -128,6 +205,7 @@ __global__ void __launch_bounds__(kDiffWarps * 32) diff_attn_kernel(TpxDiffAttn 
           }
         }
       } else {
+#pragma unroll 4
         for (int c = 0; c < dim; c++) {
           const float x = hy_ld(k + m * dp + c);
 #pragma unroll
@@ -135,15 +213,21 @@ __global__ void __launch_bounds__(kDiffWarps * 32) diff_attn_kernel(TpxDiffAttn 
         }
       }
 #pragma unroll
-      for (int i = 0; i < QT; i++) {
-        const bool seen = lane < n && j0 + lane >= lo[i] && j0 + lane <= t[i];
-        any[i] = __ballot_sync(0xffffffffu, seen);
-        const float s = seen ? p.softcap * tanhf(a[i] / p.softcap) : -INFINITY;
-        float x = s;
+      for (int i = 0; i < QT; i++) s[i][m] = a[i];
+    }
+#pragma unroll
+    for (int i = 0; i < QT; i++) {
+      const bool seen = lane < n && (QT == 1 || (j0 + lane >= lo[i] && j0 + lane <= t[i]));
+      if (QT > 1) any[i] = __ballot_sync(0xffffffffu, seen);
+#pragma unroll
+      for (int m = 0; m < 2; m++) s[i][m] = seen ? p.softcap * tanhf(s[i][m] / p.softcap) : -INFINITY;
+#pragma unroll
+      for (int m = 0; m < 2; m++) {
+        float x = s[i][m];
 #pragma unroll
         for (int d = 16; d > 0; d >>= 1) x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, d));
         const float mn = fmaxf(mx[i][m], x), al = mn == -INFINITY ? 1.0f : expf(mx[i][m] - mn);
-        e[i][m] = seen ? expf(s - mn) : 0.0f;
+        e[i][m] = seen ? expf(s[i][m] - mn) : 0.0f;
         sum[i][m] = sum[i][m] * al + hy_warp_sum(e[i][m]);
         mx[i][m] = mn;
 #pragma unroll
@@ -158,7 +242,7 @@ __global__ void __launch_bounds__(kDiffWarps * 32) diff_attn_kernel(TpxDiffAttn 
 #pragma unroll
       for (int i = 0; i < QT; i++) {
         const float e1 = __shfl_sync(0xffffffffu, e[i][0], j), e2 = __shfl_sync(0xffffffffu, e[i][1], j);
-        if (!(any[i] >> j & 1u)) continue;
+        if (QT > 1 && !(any[i] >> j & 1u)) continue;
 #pragma unroll
         for (int r = 0; r < NR; r++) {
           o[i][0][r] = fmaf(e1, x[r], o[i][0][r]);
@@ -190,17 +274,24 @@ static int diff_launch(const TpxDiffAttn& a, cudaStream_t st) {
   const int64_t nr = (a.vdim + 31) / 32;
   void (*k)(TpxDiffAttn) = nullptr;
   if constexpr (QT == 4) k = nr <= 1 ? diff_attn_kernel<T, 1, 4> : nr <= 2 ? diff_attn_kernel<T, 2, 4> : diff_attn_kernel<T, 4, 4>;
-  else k = nr <= 1 ? diff_attn_kernel<T, 1, 1> : nr <= 2 ? diff_attn_kernel<T, 2, 1> : nr <= 4 ? diff_attn_kernel<T, 4, 1>
-           : nr <= 8 ? diff_attn_kernel<T, 8, 1> : diff_attn_kernel<T, 16, 1>;
+  else if constexpr (sizeof(T) == 4)
+    k = nr <= 1 ? diff_attn_kernel<T, 1, 1> : nr <= 2 ? diff_attn_kernel<T, 2, 1> : nr <= 4 ? diff_attn_kernel<T, 4, 1>
+        : nr <= 8 ? diff_attn_kernel<T, 8, 1> : diff_attn_kernel<T, 16, 1>;
+  else k = nr <= 1 ? diff_attn_token_kernel<T, 1> : nr <= 2 ? diff_attn_token_kernel<T, 2> : nr <= 4 ? diff_attn_token_kernel<T, 4>
+           : nr <= 8 ? diff_attn_token_kernel<T, 8> : diff_attn_token_kernel<T, 16>;
   const int64_t items = a.B * ((a.S + QT - 1) / QT) * a.heads;
   TPX_CUDA_OK(launch_pdl(k, dim3((unsigned)((items + kDiffWarps - 1) / kDiffWarps)), dim3(kDiffWarps * 32), (size_t)kDiffWarps * QT * 2 * a.dim * 4, st, a));
   return TPX_OK;
 }
-// Four tokens per warp where their queries (16 KB per CTA at 128 channels) and sums (vdim <= 128) leave the registers and the shared memory
-// for more than one CTA per SM; single tokens and wider heads one by one.
+// Four tokens per warp read keys and values once for four, but a quarter of the warps then do four softmaxes in a row each: it takes heads of
+// at most 128 channels (16 KB of queries per CTA, sums in registers) and enough tokens to fill the GPU with warps all the same. Tokens x heads
+// per SM from which it paid. fp32 (one token per warp against four, us): vdim above 64: 28 (16 heads of 64 + 64 / 128, 400 tokens: 321 / 244, 200:
+// 113 / 131), above 32: 40 (16 heads of 32 + 32 / 64, 400 tokens: 0.88 of the time, 200: 1.5), else 96 (64 heads of 20 + 20 / 24, 2 x 300 tokens: 0.87,
+// 100: 1.12). bf16, sizes off the tensor cores: 64 (8 heads of 20 + 20 / 24, 2 x 513 tokens: 0.9, 300: 1.25; 64 heads, 200 tokens: 0.65).
 template <typename T>
 static int diff_run(const TpxDiffAttn& a, cudaStream_t st) {
-  return a.S > 1 && a.dim <= 128 && a.vdim <= 128 ? diff_launch<T, 4>(a, st) : diff_launch<T, 1>(a, st);
+  const int64_t least = (int64_t)sm_count() * (sizeof(T) == 2 ? 64 : a.vdim > 64 ? 28 : a.vdim > 32 ? 40 : 96);
+  return a.S >= 4 && a.dim <= 128 && a.vdim <= 128 && a.B * a.S * a.heads >= least ? diff_launch<T, 4>(a, st) : diff_launch<T, 1>(a, st);
 }
 
 }  // namespace tpx
