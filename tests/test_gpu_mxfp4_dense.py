@@ -19,17 +19,24 @@ def _rnd(g, *s, std=1.0):
 
 
 def _weight(g, N, K):
-    from tpp_pytorch_extension_b200.llm.llm_common import quantize_weight
     w = _rnd(g, N, K, std=K ** -0.5)
     w[0, :32] = 0  # an empty block
     w[-1] *= 2.0 ** -40
+    q, code, scale = _quantize(w)
+    return q, (code * scale).view(N, K)
+
+
+def _quantize(w):
+    """The packed weight, and its codes and scales in float64 [N, K / 32, 32], [N, K / 32, 1]."""
+    from tpp_pytorch_extension_b200.llm.llm_common import quantize_weight
+    N = w.shape[0]
     q = quantize_weight(w, "mxfp4")
     b = w.double().view(N, -1, 32)
     top = b.abs().amax(-1, keepdim=True)
     scale = torch.where(top > 0, torch.exp2(torch.floor(torch.log2(top.clamp(min=1e-30))) - 2), torch.ones_like(top))
     a = (b / scale).abs()
     step = torch.where(a < 2, 0.5, torch.where(a < 4, 1.0, 2.0))
-    return q, (torch.sign(b) * (torch.round(a / step) * step).clamp(max=6) * scale).view(N, K)
+    return q, torch.sign(b) * (torch.round(a / step) * step).clamp(max=6), scale
 
 
 def _close(got, want):
@@ -64,6 +71,41 @@ def test_gate_up(M, N, K):
         _close(F.fc_gate_up(x, qg, qu), gate * torch.sigmoid(gate) * up)
         _close(F.fc_gate_up(x, qg, qu, "relu"), gate.clamp(min=0) * up)
         assert_no_kernel_error()
+
+
+@pytest.mark.parametrize("byte", [0, 1, 2, 3, 127, 252, 253, 254])
+@pytest.mark.parametrize("pair", [0, 1])
+def test_scales_at_the_ends_of_their_range(byte, pair):
+    """Every scale byte is exact, also where a code times its scale is beyond bf16 (253 and 254) or subnormal (0 to 2)."""
+    from tpp_pytorch_extension_b200._C import _fused_llm_infer as F
+    M, N, K = 300, 256, 512
+    g = torch.Generator(device="cuda").manual_seed(byte)
+    q, code, _ = _quantize(_rnd(g, N, K))
+    q.scales.fill_(byte)
+    x = (_rnd(g, M, K).float() * 2.0 ** -max(min(byte - 127, 100), -100)).to(torch.bfloat16)
+    y = x.double() @ (code.view(N, K) * 2.0 ** (byte - 127)).T
+    with knob_env(TPX_MXFP4_DENSE=1):
+        got = F.fc_gate_up(x, q, q, "relu") if pair else F.fc_plain(x, q)
+        assert_no_kernel_error()
+    assert got.isfinite().all()
+    _close(got, y.clamp(min=0) * y if pair else y)
+
+
+def test_a_block_without_a_value():
+    """Scale byte 255 is the format's NaN: every result that its block enters is NaN, whatever the block's codes, and no other is."""
+    from tpp_pytorch_extension_b200._C import _fused_llm_infer as F
+    M, N, K = 300, 256, 512
+    g = torch.Generator(device="cuda").manual_seed(5)
+    q, code, scale = _quantize(_rnd(g, N, K).abs())
+    x = _rnd(g, M, K).abs()
+    want = x.double() @ (code * scale).view(N, K).T
+    q.scales.view(N // 32, K // 64, 2, 32)[1, 3, 1, 7] = 255  # feature 39, block 7
+    with knob_env(TPX_MXFP4_DENSE=1):
+        got = F.fc_plain(x, q)
+    bad = torch.zeros_like(got, dtype=torch.bool)
+    bad[:, 39] = True
+    assert torch.equal(got.isnan(), bad)
+    _close(got[~bad], want[~bad])
 
 
 @pytest.mark.parametrize("less", [0, 1])

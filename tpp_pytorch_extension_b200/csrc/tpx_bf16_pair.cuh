@@ -25,7 +25,8 @@ struct BfParams {
   TcParams t;   // epilogue fields (bias, act, mul_in, res, res_scale, y, M, N, err)
   int ksteps;   // k steps of 64 (K rounded up)
   int TN, TM;   // feature tiles, token tiles
-  int glu;      // (bf16 pair kernel, plain epilogue) features 2i and 2i+1 are gate and up of unit i: y = act(gate + bias) * up, rows of N / 2
+  int quarter;  // (bf16 pair kernel, plain epilogue) the weight holds a quarter of its values (tpx_mxfp4_dense.cu)
+  int glu;      // (with `quarter`) features 2i and 2i+1 are gate and up of unit i: y = act(gate + bias) * up, rows of N / 2
   int split;    // (pair kernels: see BpWork) 1: the CTAs share all pipeline stages of all tiles evenly; a tile cut between CTAs is put together by the last of them
   BfEx ex;
 };

@@ -1,7 +1,7 @@
 // MXFP4 linear for many tokens: the weight unpacked to bf16 for this call, then the bf16 kernel on CTA pairs.
 //
 // Serves the same calls as tpx_qlinear_tcp2.cu (fc_plain / fc_gate_up / fc_add of src/csrc/llm/fused_llm_infer.cpp on MXFP4
-// weights). An E2M1 code times a power-of-two scale is exact in bf16, and the activations enter as they are, where the block-scaled
+// weights). A quarter of an E2M1 code times its power-of-two scale is exact in bf16, and the activations enter as they are, where the block-scaled
 // kernel multiplies two 8-bit terms per activation: half of its MMA work carries the remainders, so that it ends at 1050 TFLOP/s
 // where the bf16 pair kernel reaches 1300-1450 beside the unpacking.
 // What it costs is one pass over the weight, 2.5 bytes per value (a gate/up pair of 14336 x 4096: 54 us), hence a
@@ -31,7 +31,9 @@ __global__ void __launch_bounds__(256) unpack_mxfp4_bf16_kernel(const uint8_t* _
     const int r = r0 + 16 * i;
     q[i] = __ldg(reinterpret_cast<const uint32_t*>(wq + tile * 8192 + r * 64 + c * 4));
     const uint32_t e = __ldg(sfa + tile * 512 + (r % 32) * 16 + (r / 32) * 4 + c / 4);
-    s[i] = __uint_as_float(e ? e << 23 : 0x00400000u);  // 2^(e - 127)
+    // 2^(e - 129), a quarter of the scale: six times 2^127 is beyond bf16, and the smallest product, 2^-130, is exact as a subnormal. The
+    // multiplying kernel's epilogue takes the sums four times. 255 is the format's NaN.
+    s[i] = __uint_as_float(e == 255 ? 0x7fc00000u : e > 2 ? (e - 2) << 23 : 0x00100000u << e);
   }
   pdl_wait();  // `out` may still be read by an earlier grid
   if (k >= K) return;
@@ -108,6 +110,7 @@ int mxfp4_dense_run(const uint8_t* wq, const uint8_t* sfa, bool pair, const uint
   BfParams p = {};
   p.t = base;
   p.glu = pair;
+  p.quarter = 1;
   p.t.err = reinterpret_cast<unsigned*>(sc + kTcCounterBytes - 4);
   return bf_pair_run(p, w, x, M, nw * N, K, K, K, scratch, d.off_w, st);
 }
