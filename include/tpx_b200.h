@@ -134,7 +134,10 @@ int tpx_qlinear(int kind, const uint8_t* pk_codes, const void* pk_scales, const 
  * Activations are split on the device into two E4M3 terms with a shared power-of-two block scale
  * (exact for bf16 inputs within 2^-10 of their block maximum). The scratch buffer holds those terms and the
  * partial tiles; its first 64 KiB must be zero before first use, as for tpx_qlinear. x and y may also be
- * pinned (page-locked, device-addressable) host memory: the kernels then read x and write y across the bus.   */
+ * pinned (page-locked, device-addressable) host memory: the kernels then read x and write y across the bus.
+ * Many tokens (from 2048 for a pair, 4096 for one weight, of at most 256 MiB in bf16) with device memory for x and all the scratch that
+ * tpx_qlinear_mxfp4_tc_scratch_bytes asks for: the weight is unpacked to bf16 in the scratch, which is exact, and multiplied by the
+ * activations as they are. With less scratch, or x in host memory, the form above runs.                          */
 int tpx_tc_packed_bytes(int64_t N, int64_t K, int pair, size_t* wq_bytes, size_t* sfa_bytes);
 int tpx_repack_mxfp4_tc(const uint8_t* codes, const uint8_t* scales, const uint8_t* codes2, const uint8_t* scales2,
                         int64_t N, int64_t K, uint8_t* wq, uint8_t* sfa, void* stream);
@@ -146,7 +149,8 @@ int tpx_qlinear_mxfp4_tc(const uint8_t* wq, const uint8_t* sfa, int pair, const 
 /* RMSNorm followed by the linear, the pair the reference's decoder block runs before q/k/v and before gate/up
  * (llama_rms_norm then the fused loop nests, src/csrc/llm/fused_llm_infer.cpp:1204-1272): x is normalised
  * (y = bf16(x * rsqrt(mean(x^2) + eps) * gamma), gamma bf16 or fp32) on its way into the activation split, so the
- * normalised tensor never goes to memory. Rows of up to 8192 elements; otherwise as tpx_qlinear_mxfp4_tc.     */
+ * normalised tensor never goes to memory (but to the scratch where the weight is unpacked). Rows of up to 8192 elements; otherwise as
+ * tpx_qlinear_mxfp4_tc.     */
 int tpx_rmsnorm_qlinear_mxfp4_tc(const uint8_t* wq, const uint8_t* sfa, int pair, const uint16_t* x, const void* gamma,
                                  int gamma_is_f32, float eps, int64_t M, int64_t N, int64_t K, const uint16_t* bias, int act,
                                  const uint16_t* mul_in, const uint16_t* res, float res_scale, uint16_t* y, void* scratch,
@@ -175,8 +179,12 @@ int tpx_qlinear_mxfp4_tc_static(const uint8_t* wq, const uint8_t* sfa, int pair,
  * the reference leaves in bf16 unless it is asked to quantize it (examples/llm/run_generation.py:277-282).
  *     y[M][N] = epilogue(x[M][K] . w[N][K]^T + bias[N]),   epilogue as for tpx_qlinear
  * w is the plain row-major weight (nn.Linear.weight), not re-laid out; K a multiple of 8; any M and N. fp32
- * accumulation, one bf16 rounding at the store. The scratch (tpx_linear_bf16_tc_scratch_bytes, 64 KiB, zero before
- * first use, 256-byte aligned) only carries the error word of the bounded waits at byte 65532.                    */
+ * accumulation, one bf16 rounding at the store.
+ * The scratch (256-byte aligned; tpx_linear_bf16_tc_scratch_bytes gives its size for M, N and K) holds arrival counters of tiles
+ * that are cut along k in its first 64 KiB, with the error word of the bounded waits at byte 65532, and behind them the partial sums
+ * of such tiles (up to about 20 MB). The first 64 KiB are zero before the first use and left zero (but for the error word); what lies
+ * behind needs no initial state. With less than the query says, but at least 64 KiB, no tile is cut. Calls that share a scratch must not
+ * overlap: they would count each other's arrivals and add each other's sums. One scratch per stream is safe.                  */
 size_t tpx_linear_bf16_tc_scratch_bytes(int64_t M, int64_t N, int64_t K);
 int tpx_linear_bf16_tc(const uint16_t* w, const uint16_t* x, int64_t M, int64_t N, int64_t K, const uint16_t* bias, int act,
                        const uint16_t* mul_in, const uint16_t* res, float res_scale, uint16_t* y, void* scratch,

@@ -27,7 +27,8 @@ enum { TPX_ACT_TANH = 4, TPX_ACT_XIELU = 5, TPX_ACT_CLAMPED_GLU = 6 };
  * elements. bf16 operands run on the tcgen05 kernel and need K, ldx, ldw multiples of 8 and 16-byte aligned bases; fp32
  * operands run on the 32-bit kernels: with scratch of tpx_linear_f32_scratch_bytes(M, N, K) many rows run on the tensor cores
  * (every operand as three bf16 terms that hold all its bits; rows of x and weights with an infinity, a NaN or a value of 2^30 and more are
- * computed on the CUDA cores), without it on the CUDA cores. scratch otherwise as tpx_linear_bf16_tc.
+ * computed on the CUDA cores), without it on the CUDA cores. scratch as for tpx_linear_bf16_tc, whatever the operands: its first 64 KiB
+ * zero before the first use, one per stream; for many fp32 rows it also holds the terms and the flags of what could not be cut into any.
  *
  * TPX_ACT_CLAMPED_GLU: the columns from act_from (even) on are pairs (g, u) of one gated unit each, which gives
  * z[M][(N - act_from) / 2] = g' s(1.702 g') (u' + 1) with s the logistic function, g' = min(g, limit) and u' clamped to

@@ -27,7 +27,8 @@ struct BfParams {
   int TN, TM;   // feature tiles, token tiles
   int quarter;  // (bf16 pair kernel, plain epilogue) the weight holds a quarter of its values (tpx_mxfp4_dense.cu)
   int glu;      // (with `quarter`) features 2i and 2i+1 are gate and up of unit i: y = act(gate + bias) * up, rows of N / 2
-  int split;    // (pair kernels: see BpWork) 1: the CTAs share all pipeline stages of all tiles evenly; a tile cut between CTAs is put together by the last of them
+  int ctas;     // (one-CTA kernel) 0: whole tiles; else so many CTAs share all pipeline stages of all tiles evenly, a tile cut between CTAs is put together by the last of them
+  int pieces;   // (pair kernels: see BpWork) pieces that each tile of the last round is cut into along k; up to 1: not cut
   BfEx ex;
 };
 
@@ -66,13 +67,13 @@ constexpr int kBpEpiCols = 1024 / kBpEpiWarps;  // features per warp
 constexpr int kBpGroup = 16;  // token tiles walked side by side (bf16, 16384 x 14336 x 4096: 1210 us, with 8: 1231, with 4: 1270)
 
 // What a cluster works on: k steps [g0, g1) of tile (tn, tm). Tiles are dealt out in turn, in blocks of kBpGroup token tiles (inside
-// a block the token tiles of one feature tile are neighbours). p.split = S > 1: the tiles of the last, partly filled round are
+// a block the token tiles of one feature tile are neighbours). p.pieces = S > 1: the tiles of the last, partly filled round are
 // cut along k into S pieces for as many clusters.
 struct BpWork {
   int T, ks, G, cid, TN, TM, S, W;  // W: tiles in front of the cut ones
   int tile, piece, g0, g1, tn, tm;
   __device__ __forceinline__ BpWork(const BfParams& p)
-      : T(p.TN * p.TM), ks(p.ksteps), G((int)gridDim.x / 2), cid((int)blockIdx.x / 2), TN(p.TN), TM(p.TM), S(p.split > 1 ? p.split : 1) {
+      : T(p.TN * p.TM), ks(p.ksteps), G((int)gridDim.x / 2), cid((int)blockIdx.x / 2), TN(p.TN), TM(p.TM), S(p.pieces > 1 ? p.pieces : 1) {
     W = T / G * G;
     tile = cid - G;
     piece = 0;
@@ -118,7 +119,7 @@ __device__ __forceinline__ bool bp_last(const BfParams& p, const BpWork& k, int 
   __threadfence();
   return last;
 }
-// The tile's pieces, added in the order of k; all columns of a piece in flight at once (16 at a time: 14 us for five pieces).
+// The tile's pieces, added in the order of k; all columns of a piece are in flight at once, each load a round trip to L2.
 __device__ __forceinline__ void bp_sum(const BfParams& p, const BpWork& k, int crank, int ew, int lane, float (&v)[kBpEpiCols]) {
 #pragma unroll
   for (int j = 0; j < kBpEpiCols; j++) v[j] = 0.0f;

@@ -45,10 +45,10 @@ extern "C" int tpx_llama_layer_mlp(const TpxLlamaLayer* L, const TpxLlamaLayerIO
   // With 33 to 64 tokens the gate/up kernel's epilogue also writes its output as the activation terms the down
   // projection reads (io->handoff), when both kernels chosen for these shapes can: one kernel fewer in the chain
   // (Llama-3-8B shape, 1024 cached tokens: 4.53 against 4.63 ms per step at batch 33, 5.20 against 5.30 at batch 48,
-  // 5.86 against 5.96 at batch 64). With fewer tokens it loses: the split kernel it
-  // saves is short and ran while the down projection's CTAs fetched their first weights, and the packed-fp4 kernel's
-  // four epilogue warps pay for the conversion on the critical path (batch 16: 4.52 against 4.06 ms; batch 1: 2.9
-  // against 2.76). TPX_HANDOFF_MIN_TOKENS moves the lower bound.
+  // 5.86 against 5.96 at batch 64). With fewer tokens it loses: the split kernel it saves is short and ran while the down
+  // projection's CTAs fetched their first weights, and the 128-row kernel, the fastest up to 16 tokens, cannot hand over: a lower
+  // bound (TPX_HANDOFF_MIN_TOKENS) takes the packed-fp4 kernel for it, whose four epilogue warps pay for the conversion on the
+  // critical path (batch 16: 4.52 against 4.06 ms, batch 1: 2.9 against 2.76, both measured on that kernel).
   tpx::TcEmit E = {};
   if (T >= tpx::knobs().handoff_min && T <= 64 && io->handoff) {
     int rc0 = tpx::tc_handoff_plan(T, D, L->FF, io->handoff, io->handoff_bytes, &E);

@@ -31,7 +31,7 @@ struct BfPieces {
   int tile, g0, g1;
   __device__ __forceinline__ BfPieces(const BfParams& p, int nstages) : ns(nstages) {
     const long long T = (long long)p.TN * p.TM;
-    if (p.split) {
+    if (p.ctas) {
       const long long U = T * ns;
       u = blockIdx.x * U / gridDim.x;
       u1 = (blockIdx.x + 1) * U / gridDim.x;
@@ -388,7 +388,7 @@ static int bf_launch(const CUtensorMap& w, const CUtensorMap& x, const BfParams&
   }
   const long long T = (long long)p.TN * p.TM;
   const int sms = sm_count();
-  const int grid = p.split ? p.split : (int)(T < sms ? T : sms);
+  const int grid = p.ctas ? p.ctas : (int)(T < sms ? T : sms);
   TPX_CUDA_OK(launch_pdl(linear_bf16_kernel<TOK>, dim3((unsigned)grid), dim3(kTcThreads), C::SMEM, st, w, x, p));
   return TPX_OK;
 }
@@ -409,8 +409,8 @@ static size_t bf_split_bytes(int64_t M, int grid) { return (size_t)grid * 2 * (M
 static int bf_run(BfParams& p, const void* w, const void* x, int64_t M, int64_t N, int64_t K, int64_t ldw, int64_t ldx, void* scratch,
                   size_t scratch_bytes, cudaStream_t st) {
   if (bf_pair_serves(p, M, N, K)) return bf_pair_run(p, w, x, M, N, K, ldw, ldx, scratch, scratch_bytes, st);
-  p.split = bf_split_ctas(M, N, K);
-  if (p.split && scratch_bytes < kTcCounterBytes + bf_split_bytes(M, p.split)) p.split = 0;
+  p.ctas = bf_split_ctas(M, N, K);
+  if (p.ctas && scratch_bytes < kTcCounterBytes + bf_split_bytes(M, p.ctas)) p.ctas = 0;
   p.t.counters = reinterpret_cast<unsigned*>(scratch);
   p.t.partial = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(scratch) + kTcCounterBytes);
   const int tok = M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : M <= 128 ? 128 : 256;

@@ -355,8 +355,8 @@ size_t bf_pair_scratch_bytes(int64_t M, int64_t N, int64_t K) {
 int bf_pair_run(BfParams& p, const void* w, const void* x, int64_t M, int64_t N, int64_t K, int64_t ldw, int64_t ldx, void* scratch,
                 size_t scratch_bytes, cudaStream_t st) {
   using C = BpCfg;
-  p.split = bf_pair_split(M, N, K, kBpUsPerStep);
-  if (p.split > 1 && scratch_bytes < kTcCounterBytes + bf_pair_split_bytes()) p.split = 1;
+  p.pieces = bf_pair_split(M, N, K, kBpUsPerStep);
+  if (p.pieces > 1 && scratch_bytes < kTcCounterBytes + bf_pair_split_bytes()) p.pieces = 1;
   p.t.counters = reinterpret_cast<unsigned*>(scratch);
   p.t.partial = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(scratch) + kTcCounterBytes);
   p.t.M = (int)M; p.t.N = (int)N; p.t.K = (int)K;
@@ -376,7 +376,7 @@ int bf_pair_run(BfParams& p, const void* w, const void* x, int64_t M, int64_t N,
     TPX_CUDA_OK(cudaFuncSetAttribute(linear_bf16_pair_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM));
     if (dev >= 0 && dev < 16) opted[dev] = true;
   }
-  const int grid = 2 * bf_pair_clusters(M, N, p.split);
+  const int grid = 2 * bf_pair_clusters(M, N, p.pieces);
   TPX_CUDA_OK(launch_pdl(p.quarter ? linear_bf16_pair_kernel<true> : linear_bf16_pair_kernel<false>, dim3((unsigned)grid), dim3(C::THREADS), C::SMEM, st, mw, mx, p));
   return TPX_OK;
 }

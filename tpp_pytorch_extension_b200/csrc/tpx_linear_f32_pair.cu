@@ -356,8 +356,8 @@ int f32_pair_run(const TpxLinear& a, const F32Epi& e, cudaStream_t st) {
       p.ksteps = (int)((a.K + 63) / 64);
       p.TN = (int)((n + 255) / 256);
       p.TM = (int)((rows + 255) / 256);
-      p.split = bf_pair_split(rows, n, a.K, kFpUsPerStep);
-      const int grid = 2 * bf_pair_clusters(rows, n, p.split);
+      p.pieces = bf_pair_split(rows, n, a.K, kFpUsPerStep);
+      const int grid = 2 * bf_pair_clusters(rows, n, p.pieces);
       TPX_CUDA_OK(launch_pdl(linear_f32_pair_kernel, dim3((unsigned)grid), dim3(C::THREADS), C::SMEM, st, mw, mx, p, e, (long long)m0, (int)n0,
                              flags, flags + 1 + slab));
     }

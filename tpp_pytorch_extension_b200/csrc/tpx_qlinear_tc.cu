@@ -1038,14 +1038,15 @@ static bool tc_wide(int64_t M, int64_t N, int64_t K, bool pair) {
 }
 
 // Kernel family for a call: 0 = weights on the 128-row side (all M), 1 = weights on the N side (M <= 64),
-// 2 = packed-fp4 operands (M <= 32), only with TPX_TC_F4=1 or for a pair of whole tiles that TPX_HANDOFF_MIN_TOKENS lets hand over: four E2M1 terms per activation paid while a short MMA cost the issuing
-// thread as much as a long one; with issue under an elected lane families 0 and 1 are faster at every shape measured (14336 x 4096
-// pair at 8 tokens: 16.5 against 16.9 us, at 32: 18.6 against 22.1; 11008 x 4096: 12.1 against 14.3 us).
-constexpr int kW4AutoMaxTokens = 0;  // token counts up to which family 3 is chosen without being asked for
+// 2 = packed-fp4 operands (M <= 32), only with TPX_TC_F4=1 or for a pair of whole tiles that TPX_HANDOFF_MIN_TOKENS lets hand over: four
+// E2M1 terms per activation paid while a short MMA cost the issuing thread as much as a long one; with issue under an elected lane
+// families 0 and 1 are faster at every shape measured (14336 x 4096 pair at 8 tokens: 16.5 against 16.9 us, at 32: 18.6 against 22.1;
+// 11008 x 4096: 12.1 against 14.3 us), and their two E4M3 terms are closer (normal activations: error against 64 bits 1.656e-3, of which
+// 1.656e-3 are the result's rounding, against 1.661e-3; heavy-tailed ones 1.661e-3 against 1.791e-3).
+constexpr int kW4AutoMaxTokens = 0;  // token counts up to which family 3 is chosen without being asked for: none
 static int tc_kind(int64_t M, int64_t N, int64_t K, bool pair) {
-  // 3 = weights on the N side with packed-fp4 operands (tpx_qlinear_tcw4.cu): the default up to 32 tokens wherever its
-  // work split applies (whole tiles or a cluster per tile), unless a test forces another family; TPX_TC_W4=1 selects it
-  // for every shape it serves (up to 64 tokens), TPX_TC_W4=0 never.
+  // 3 = weights on the N side with packed-fp4 operands (tpx_qlinear_tcw4.cu): TPX_TC_W4=1 selects it for every shape it serves (up to 64
+  // tokens); otherwise never chosen.
   {
     const int w4 = knobs().tc_w4;
     const bool other_forced = knobs().tc_f4 >= 0 || knobs().tc_wide >= 0;
