@@ -8,7 +8,7 @@ pytestmark = pytest.mark.gpu
 # heads, kv_heads, dim, vdim: 16-byte pieces of a key row and not, one to four value columns per lane, wider than four tokens per warp take
 HEADS = [(4, 2, 64, 128), (2, 1, 20, 24), (3, 3, 9, 11), (2, 1, 130, 40), (2, 2, 32, 136)]
 LAM, MULT, EPS, CAP = 0.3, 0.7, 1e-5, 9.0
-# a sum of fp32 products and exponentials, a few 2^-24 each and more where the maps cancel; bf16: the result rounded once, 2^-9 of it
+# a sum of fp32 products and exponentials, a few 2^-24 each and more where the maps cancel; bf16: the result rounded once, at most 2^-8 of it
 TOL = {torch.float32: 2e-5, torch.bfloat16: 2.0 ** -8}
 
 

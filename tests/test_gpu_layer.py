@@ -22,7 +22,7 @@ def test_rmsnorm(cuda):
         assert np.array_equal(y32, y)
 
 
-def _rope_case(cuda, B, S, Nq, Nkv, H, offset, pos):
+def _rope_case(cuda, B, S, Nq, Nkv, H, offset, pos, same=np.array_equal):
     from tpp_pytorch_extension_b200 import _lib
     rng = np.random.default_rng(B * 100 + S)
     MP = 64
@@ -45,11 +45,11 @@ def _rope_case(cuda, B, S, Nq, Nkv, H, offset, pos):
     q_ref = O.rope_llama(qr, ep, pos, Nq, H).reshape(B, S, Nkv, R, H).transpose(0, 2, 1, 3, 4)
     k_ref = O.rope_llama(kr, ep, pos, Nkv, H).reshape(B, S, Nkv, H)
     v_ref = vr.reshape(B, S, Nkv, H)
-    assert np.array_equal(to_host_bits(q), np.ascontiguousarray(q_ref))
+    assert same(to_host_bits(q), np.ascontiguousarray(q_ref))
     kh, vh = to_host_bits(kc), to_host_bits(vc)
     for s in range(S):
         t = offset + s
-        assert np.array_equal(kh[t // 32, :, :, t % 32], k_ref[:, s])
+        assert same(kh[t // 32, :, :, t % 32], k_ref[:, s])
         assert np.array_equal(vh[t // 32, :, :, t % 32], v_ref[:, s])
     assert not kh[(offset + S + 31) // 32:].any()  # nothing beyond the written tokens
 
@@ -59,6 +59,17 @@ def test_rope_kv_update_bit_exact(cuda):
     _rope_case(cuda, 3, 1, 4, 4, 64, 37, np.array([[37], [12], [63]], dtype=np.int64))
     # positions at and beyond the table leave the row untouched
     _rope_case(cuda, 1, 3, 2, 1, 128, 30, np.array([[62, 64, 100]], dtype=np.int64))
+
+
+@pytest.mark.parametrize("Nq,Nkv,H", [(1, 1, 16), (6, 2, 64), (28, 4, 128), (32, 32, 128), (4, 2, 48)])
+def test_rope_units_per_token(cuda, Nq, Nkv, H):
+    """A token's vector units from a fraction of one CTA to several CTAs, full ones and not. A product and a sum may be rounded together: half a
+    bf16 unit of the result (2^-8) and 2^-23 of values of a few units apart."""
+    def same(a, b):
+        a, b = O.bf16_to_f32(a), O.bf16_to_f32(b)
+        return a.shape == b.shape and bool((np.abs(a - b) <= 2.0 ** -7 * np.abs(b) + 1e-6).all())
+    _rope_case(cuda, 2, 9, Nq, Nkv, H, 30, np.arange(9, dtype=np.int64)[None], same)
+    _rope_case(cuda, 5, 1, Nq, Nkv, H, 3, np.arange(5, dtype=np.int64)[:, None], same)
 
 
 def test_rope_rejects_overflow(cuda):

@@ -7,7 +7,7 @@ pytestmark = pytest.mark.gpu
 
 # rows, features, inner size: one tile, tile edges, several tiles with and without a cut along k, an inner size off the k step
 SHAPES = [(129, 256, 1024), (256, 512, 4096), (257, 264, 72), (300, 4096, 1536), (1030, 2056, 2048), (2049, 1288, 520), (4100, 5128, 256)]
-# a result is rounded to bf16 once: at most 2^-9 of it; in fp32 the sum of K products is off by a few 2^-24 of its size
+# a result is rounded to bf16 once: at most 2^-8 of it; in fp32 the sum of K products is off by a few 2^-24 of its size
 BF16, F32 = 2.0 ** -8, 2e-6
 
 

@@ -17,9 +17,9 @@ TOL = 2e-2
 @pytest.fixture(autouse=True, params=[(1, 2, 1), (1, 1, 1), (1, 2, 0), (0, 2, 1), (0, 1, 1)],
                 ids=["pair-uks2", "pair-uks1", "pair-blockscales", "one-uks2", "one-uks1"])
 def forced(request, cuda):
-    """pair: CTA-pair kernel, with one activation scale per token (default) or per 32 values (TPX_TC_P_ROWS=0)."""
+    """pair: CTA-pair kernel, with one activation scale per token (default) or per 32 values (TPX_TC_P_ROWS=0). All on the packed weight, whatever the token count."""
     p2, uks, rows = request.param
-    with knob_env(TPX_MXFP4_PATH="tc", TPX_TC_P=1, TPX_TC_P2=p2, TPX_TC_P_UKS=uks, TPX_TC_P_ROWS=rows):
+    with knob_env(TPX_MXFP4_PATH="tc", TPX_TC_P=1, TPX_TC_P2=p2, TPX_TC_P_UKS=uks, TPX_TC_P_ROWS=rows, TPX_MXFP4_DENSE=0):
         yield
 
 
