@@ -32,7 +32,7 @@ def _case(H, S, grow, padding, dropped):
     real[1, :padding] = False
     real[:, dropped] = False
     keep = real[:, None, :, None, None].expand_as(got)
-    # weights and result are rounded to bf16 once each: at most 2^-8 of what they are, sums of at most max |v|; typical sums are well inside
+    # weights (which sum to one) and the result are rounded to bf16 once each: at most 2^-8 of max |v| each
     assert float((got - want)[keep].abs().max()) <= 2.0 ** -7 * float(v.double().abs().max())
 
 

@@ -67,7 +67,8 @@ static DensePlan dense_plan(int64_t M, int64_t N, int64_t K, bool pair) {
 // Below the least number of tokens the unpacking costs more than the faster MMAs save. Weights of more than 256 MiB in bf16 stay
 // packed, so that the scratch stays bounded. TPX_MXFP4_DENSE=0 never, =1 from 129 tokens on.
 // (14336 x 4096 pair, packed against unpacked: 2048 tokens 433 / 375 us, 4096: 873 / 732, 8192: 1792 / 1355; one weight, 4096 x 14336: 222 / 211,
-// 441 / 405, 901 / 762; 6144 x 4096: 116 / 114, 171 / 174, 370 / 320; 8192 x 2048: 80 / 81, 114 / 109, 255 / 215.)
+// 441 / 405, 901 / 762; 6144 x 4096: 116 / 114, 171 / 174, 370 / 320; 8192 x 2048: 80 / 81, 114 / 109, 255 / 215. The line leaves out N and K: where
+// tiles end just past a round the unpacked form loses up to 10 % above it, 2560 x 2048 at 4096 tokens 56 / 61, and elsewhere it would win below.)
 constexpr int64_t kDenseMinTokens = 4096, kDenseMinTokensPair = 2048;
 constexpr int64_t kDenseMaxBytes = 256ll << 20;
 bool mxfp4_dense_serves(int64_t M, int64_t N, int64_t K, bool pair) {
