@@ -191,7 +191,8 @@ int tpx_linear_bf16_tc(const uint16_t* w, const uint16_t* x, int64_t M, int64_t 
                        size_t scratch_bytes, void* stream);
 
 /* ---------------------------------------------------------------- int8 linear on the tcgen05 tensor cores
- * Any number of tokens (tiles of 16, 32, 64 or 128 tokens x 128 features) with the reference's own int8 arithmetic
+ * Any number of tokens (blocks of 64 and up to 32 tokens: a kernel that streams the weight
+ * through registers; else tiles of 16, 32, 64 or 128 tokens x 128 features) with the reference's own int8 arithmetic
  * (TppBlockedQInt8LinearW, src/csrc/fused_gemm.h:1075-1341):
  * the activations are quantised on the fly to int8 with one scale per (token, K block) (:1249), each K block is an
  * int8 x int8 -> int32 product and y accumulates tmp * s_x * s_w (:1197-1204); the running sum stays in fp32 where
@@ -214,6 +215,11 @@ size_t tpx_qlinear_qint8_tc_scratch_bytes(int64_t M, int64_t N, int64_t K, int64
 int tpx_qlinear_qint8_tc(const int8_t* wq, const float* swT, const uint16_t* x, const void* gamma, int gamma_is_f32,
                          float eps, int64_t M, int64_t N, int64_t K, int64_t block_size, int reuse_act, const uint16_t* bias, int act, const uint16_t* mul_in,
                          const uint16_t* res, float res_scale, uint16_t* y, void* scratch, size_t scratch_bytes, void* stream);
+/* act(x . wq^T) * (x . wq2^T) of two weights of the same shape, scratch and norm as above. Up to 16 tokens and blocks of 64 in one kernel, the
+ * activated gate staying in fp32; else two linears, the second multiplying by the bf16 gate that the first left in y.          */
+int tpx_qlinear_qint8_pair_tc(const int8_t* wq, const float* swT, const int8_t* wq2, const float* swT2, const uint16_t* x, const void* gamma,
+                              int gamma_is_f32, float eps, int64_t M, int64_t N, int64_t K, int64_t block_size, int act, uint16_t* y, void* scratch,
+                              size_t scratch_bytes, void* stream);
 
 /* ---------------------------------------------------------------- decoder-layer pieces
  * RMSNorm: y = x * rsqrt(mean(x^2) + eps) * gamma, fp32 statistics. Replaces llama_rms_norm

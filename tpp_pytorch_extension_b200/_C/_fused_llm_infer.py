@@ -38,9 +38,9 @@ INT8_DENSE_MIN_TOKENS = 128  # above this the int8 weight is unpacked to bf16 pe
 
 
 def _int8_tc(x, y, w, w2, bias, act, mul_in, res, res_scale, norm=None):
-    """int8 weights: up to 128 tokens through tpx_qlinear_qint8_tc (the reference's activation-quantised arithmetic); a
-    gate/up pair runs as two calls, the second multiplying by the activated first. More tokens: weight-only arithmetic
-    on the bf16 tensor-core kernel (TPX_INT8_DENSE=0 keeps the int8 kernel for every token count)."""
+    """int8 weights: up to 128 tokens through tpx_qlinear_qint8_tc and, a gate/up pair, tpx_qlinear_qint8_pair_tc (the
+    reference's activation-quantised arithmetic). More tokens: weight-only arithmetic on the bf16 tensor-core kernel
+    (TPX_INT8_DENSE=0 keeps the int8 kernels for every token count)."""
     L = _lib.lib()
     N, K = w.out_features, w.in_features
     M = x.numel() // K
@@ -63,26 +63,22 @@ def _int8_tc(x, y, w, w2, bias, act, mul_in, res, res_scale, norm=None):
         return _bf16_linear(x, dense(w2), None, None, h, None, 1.0)
 
     gam, eps = (norm[0], float(norm[1])) if norm is not None else (None, 0.0)
-
-    def run(wt, out, b, a, m, r, rs, reuse=0):
-        wq, sw = wt.packed_i8tc()
-        key = ("i8tc", M, N, K, wt.block_size)
-        nb = _SCRATCH_BYTES.get(key)
-        if nb is None:
-            nb = _SCRATCH_BYTES[key] = L.tpx_qlinear_qint8_tc_scratch_bytes(M, N, K, wt.block_size)
-        sc = _lib.scratch(nb, x.device)
-        rc = L.tpx_qlinear_qint8_tc(wq.data_ptr(), sw.data_ptr(), x.data_ptr(), _lib.ptr(gam), int(gam is not None and gam.dtype == torch.float32),
-                                    eps, M, N, K, wt.block_size, reuse, _lib.ptr(b), ACT[a], _lib.ptr(m),
-                                    _lib.ptr(r), float(rs), out.data_ptr(), sc.data_ptr(), sc.numel(), _lib.stream())
-        if rc:
-            _lib.check(rc)
-
+    g32 = int(gam is not None and gam.dtype == torch.float32)
+    key = ("i8tc", M, N, K, w.block_size)
+    nb = _SCRATCH_BYTES.get(key)
+    if nb is None:
+        nb = _SCRATCH_BYTES[key] = L.tpx_qlinear_qint8_tc_scratch_bytes(M, N, K, w.block_size)
+    sc = _lib.scratch(nb, x.device)
+    wq, sw = w.packed_i8tc()
     if w2 is None:
-        run(w, y, bias, act, mul_in, res, res_scale)
-        return y
-    h = torch.empty_like(y)
-    run(w, h, bias, act, None, None, 1.0)
-    run(w2, y, None, None, h, None, 1.0, reuse=1)  # same x: the quantised activations are still in the scratch
+        rc = L.tpx_qlinear_qint8_tc(wq.data_ptr(), sw.data_ptr(), x.data_ptr(), _lib.ptr(gam), g32, eps, M, N, K, w.block_size, 0, _lib.ptr(bias),
+                                    ACT[act], _lib.ptr(mul_in), _lib.ptr(res), float(res_scale), y.data_ptr(), sc.data_ptr(), sc.numel(), _lib.stream())
+    else:
+        wq2, sw2 = w2.packed_i8tc()
+        rc = L.tpx_qlinear_qint8_pair_tc(wq.data_ptr(), sw.data_ptr(), wq2.data_ptr(), sw2.data_ptr(), x.data_ptr(), _lib.ptr(gam), g32, eps, M, N, K,
+                                         w.block_size, ACT[act], y.data_ptr(), sc.data_ptr(), sc.numel(), _lib.stream())
+    if rc:
+        _lib.check(rc)
     return y
 
 

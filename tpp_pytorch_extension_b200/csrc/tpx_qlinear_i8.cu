@@ -15,7 +15,7 @@
 // when tiles are few, a thread-block cluster per tile cuts K between its CTAs, which add their parts over distributed
 // shared memory. (Sharing the k units of all tiles evenly between the CTAs, 86 tiles of 11008 features on 148 SMs, brought nothing
 // up to 64 tokens: a CTA's chain of copy, MMA, drain is short enough, and putting cut tiles together costs what it saves.)
-#include "tpx_tc_ptx.cuh"
+#include "tpx_qlinear_i8_rows.cuh"
 
 namespace tpx {
 
@@ -119,9 +119,9 @@ __global__ void __launch_bounds__(kQbWarps * 32) quantize_act_i8_block512_kernel
 // VECS vectors per thread, without it a row is spread over gridDim.y CTAs: the kernel is latency, and one CTA that goes round
 // over a row of 11008 values took 9 us.
 constexpr int kQaThreads = 256;
-template <int VECS>
+template <int VECS, class LAYOUT>
 __global__ void __launch_bounds__(kQaThreads) quantize_act_i8_row_kernel(const uint16_t* __restrict__ x, const void* __restrict__ gamma,
-                                                                         int gamma_f32, float eps, int M, int K, I8Act L, uint8_t* __restrict__ xq) {
+                                                                         int gamma_f32, float eps, int M, int K, LAYOUT L, uint8_t* __restrict__ xq) {
   __shared__ float red[kQaThreads / 32];
   pdl_trigger();
   pdl_wait();
@@ -576,8 +576,9 @@ static int i8_launch(const CUtensorMap& w, I8Params p, int tiles, cudaStream_t s
 
 template <int BS>
 static int i8_launch_tok(int tokp, const CUtensorMap& w, const I8Params& p, int tiles, cudaStream_t st) {
+  if constexpr (BS > 2)  // up to 16 tokens, blocks of 64 are tpx_qlinear_i8_rows.cu's
+    if (tokp == 16) return i8_launch<16, BS>(w, p, tiles, st);
   switch (tokp) {
-    case 16: return i8_launch<16, BS>(w, p, tiles, st);
     case 32: return i8_launch<32, BS>(w, p, tiles, st);
     case 64: return i8_launch<64, BS>(w, p, tiles, st);
     default: return i8_launch<128, BS>(w, p, tiles, st);
@@ -637,9 +638,26 @@ extern "C" size_t tpx_qlinear_qint8_tc_scratch_bytes(int64_t M, int64_t N, int64
   return i8_plan(M, N, K, block_size).total;
 }
 
-extern "C" int tpx_qlinear_qint8_tc(const int8_t* wq, const float* swT, const uint16_t* x, const void* gamma, int gamma_is_f32, float eps,
-                                    int64_t M, int64_t N, int64_t K, int64_t block_size, int reuse_act, const uint16_t* bias, int act, const uint16_t* mul_in,
-                                    const uint16_t* res, float res_scale, uint16_t* y, void* scratch, size_t scratch_bytes, void* stream) {
+namespace tpx {
+// The activations of a call as its GEMM reads them.
+template <class LAYOUT>
+static int i8_quantize(const uint16_t* x, const void* gamma, int gamma_is_f32, float eps, int M, int Mp, int64_t K, const LAYOUT& L, uint8_t* xq,
+                       cudaStream_t st) {
+  if (gamma) {
+    TPX_CUDA_OK(launch_pdl(quantize_act_i8_row_kernel<4, LAYOUT>, dim3((unsigned)Mp), dim3(kQaThreads), 0, st, x, gamma, gamma_is_f32, eps, M, (int)K, L, xq));
+  } else {
+    TPX_CUDA_OK(launch_pdl(quantize_act_i8_row_kernel<1, LAYOUT>, dim3((unsigned)Mp, (unsigned)((K / 8 + kQaThreads - 1) / kQaThreads)), dim3(kQaThreads), 0,
+                           st, x, gamma, gamma_is_f32, eps, M, (int)K, L, xq));
+  }
+  return TPX_OK;
+}
+}  // namespace tpx
+
+// One linear, or with wq2 the pair act(x wq^T) * (x wq2^T): in one kernel for few tokens, else as two linears, the second multiplying by
+// what the first left in y.
+static int i8_linear(const int8_t* wq, const float* swT, const int8_t* wq2, const float* swT2, const uint16_t* x, const void* gamma, int gamma_is_f32,
+                     float eps, int64_t M, int64_t N, int64_t K, int64_t block_size, int reuse_act, const uint16_t* bias, int act,
+                     const uint16_t* mul_in, const uint16_t* res, float res_scale, uint16_t* y, void* scratch, size_t scratch_bytes, void* stream) {
   TPX_REQUIRE(M >= 0 && N > 0 && K > 0, TPX_ERR_ARG, "qlinear_qint8_tc: bad shape");
   if (M == 0) return TPX_OK;
   TPX_REQUIRE(M <= (1 << 20), TPX_ERR_UNSUPPORTED, "qlinear_qint8_tc: at most 2^20 tokens per call (M=%ld)", (long)M);
@@ -648,25 +666,45 @@ extern "C" int tpx_qlinear_qint8_tc(const int8_t* wq, const float* swT, const ui
               "qlinear_qint8_tc: block size %ld not supported (64, 128, 256, 512)", (long)block_size);
   TPX_REQUIRE(N % 16 == 0 && K % block_size == 0, TPX_ERR_ARG, "qlinear_qint8_tc: needs N %% 16 == 0 and K %% block_size == 0");
   TPX_REQUIRE(act >= TPX_ACT_NONE && act <= TPX_ACT_RELU, TPX_ERR_ARG, "qlinear_qint8_tc: unknown activation %d", act);
-  TPX_REQUIRE((((uintptr_t)wq | (uintptr_t)x | (uintptr_t)swT) & 15) == 0 && ((uintptr_t)scratch & 255) == 0, TPX_ERR_ARG,
-              "qlinear_qint8_tc: misaligned pointer");
+  TPX_REQUIRE((((uintptr_t)wq | (uintptr_t)wq2 | (uintptr_t)x | (uintptr_t)swT | (uintptr_t)swT2) & 15) == 0 && ((uintptr_t)scratch & 255) == 0,
+              TPX_ERR_ARG, "qlinear_qint8_tc: misaligned pointer");
   I8Plan pl = i8_plan(M, N, K, block_size);
   TPX_REQUIRE(pl.Kp % block_size == 0, TPX_ERR_UNSUPPORTED, "qlinear_qint8_tc: K rounded up to 128 must stay a multiple of the block size");
   TPX_REQUIRE(scratch && scratch_bytes >= pl.total, TPX_ERR_SCRATCH, "qlinear_qint8_tc: scratch of %zu bytes needed, %zu given", pl.total,
               scratch_bytes);
+  TPX_REQUIRE(!gamma || (K <= 8192 && block_size <= 256 && ((uintptr_t)gamma & 15) == 0), TPX_ERR_UNSUPPORTED,
+              "qlinear_qint8_tc: the fused RMSNorm takes rows of up to 8192 values, blocks of up to 256 and a 16-byte aligned gamma");
+  if (wq2 && !i8_rows_serves(M, N, block_size, true)) {
+    int rc = i8_linear(wq, swT, nullptr, nullptr, x, gamma, gamma_is_f32, eps, M, N, K, block_size, reuse_act, bias, act, nullptr, nullptr, 1.0f, y,
+                       scratch, scratch_bytes, stream);
+    if (rc) return rc;
+    return i8_linear(wq2, swT2, nullptr, nullptr, x, gamma, gamma_is_f32, eps, M, N, K, block_size, 1, nullptr, TPX_ACT_NONE, y, res, res_scale, y,
+                     scratch, scratch_bytes, stream);
+  }
   cudaStream_t st = (cudaStream_t)stream;
   unsigned char* sc = reinterpret_cast<unsigned char*>(scratch);
   uint8_t* xq = sc + pl.off_xq;
+  TcParams t = {};
+  t.bias = bias; t.mul_in = mul_in; t.res = res; t.res_scale = res_scale; t.y = y; t.act = act;
+  t.M = (int)M; t.N = (int)N; t.K = (int)K; t.cluster = pl.cluster;
+  t.err = reinterpret_cast<unsigned*>(sc + kTcCounterBytes - 4);
+  if (i8_rows_serves(M, N, block_size, wq2 != nullptr)) {
+    const I8Rows L((int)M, K);
+    if (!reuse_act) {
+      int rc = i8_quantize(x, gamma, gamma_is_f32, eps, (int)M, (int)M, K, L, xq, st);
+      if (rc) return rc;
+    }
+    I8RowsParams p = {};
+    p.t = t;
+    p.w[0] = wq; p.w[1] = wq2; p.swT[0] = swT; p.swT[1] = swT2; p.xq = xq;
+    p.nkb = L.nkb; p.Mp = L.Mp; p.Kp = (int)pl.Kp; p.Np = (int)pl.Np; p.tiles = (int)(N / 16);
+    return i8_rows_launch(p, wq2 != nullptr, st);
+  }
   const I8Act L(pl.tokp, pl.ksteps, (int)block_size);
   if (!reuse_act && pl.Kp != K) TPX_CUDA_OK(cudaMemsetAsync(xq, 0, pl.xq_bytes, st));  // the k padding reads as zero
-  TPX_REQUIRE(!gamma || (K <= 8192 && block_size <= 256 && ((uintptr_t)gamma & 15) == 0), TPX_ERR_UNSUPPORTED,
-              "qlinear_qint8_tc: the fused RMSNorm takes rows of up to 8192 values, blocks of up to 256 and a 16-byte aligned gamma");
-  if (!reuse_act && gamma) {
-    TPX_CUDA_OK(launch_pdl(quantize_act_i8_row_kernel<4>, dim3((unsigned)pl.Mp), dim3(kQaThreads), 0, st, x, gamma, gamma_is_f32, eps, (int)M,
-                           (int)K, L, xq));
-  } else if (!reuse_act && block_size <= 256) {
-    TPX_CUDA_OK(launch_pdl(quantize_act_i8_row_kernel<1>, dim3((unsigned)pl.Mp, (unsigned)((K / 8 + kQaThreads - 1) / kQaThreads)), dim3(kQaThreads), 0,
-                           st, x, gamma, gamma_is_f32, eps, (int)M, (int)K, L, xq));
+  if (!reuse_act && block_size <= 256) {
+    int rc = i8_quantize(x, gamma, gamma_is_f32, eps, (int)M, (int)pl.Mp, K, L, xq, st);
+    if (rc) return rc;
   } else if (!reuse_act) {
     const long long warps = (long long)pl.Mp * (K / 512);
     TPX_CUDA_OK(launch_pdl(quantize_act_i8_block512_kernel, dim3((unsigned)((warps + kQbWarps - 1) / kQbWarps)), dim3(kQbWarps * 32), 0, st, x, (int)M, (int)K,
@@ -676,9 +714,7 @@ extern "C" int tpx_qlinear_qint8_tc(const int8_t* wq, const float* swT, const ui
   int rc = make_map_u8(&mw, wq, (uint64_t)pl.Np, (uint64_t)pl.Kp, 128);
   if (rc) return rc;
   I8Params p = {};
-  p.t.bias = bias; p.t.mul_in = mul_in; p.t.res = res; p.t.res_scale = res_scale; p.t.y = y; p.t.act = act;
-  p.t.M = (int)M; p.t.N = (int)N; p.t.K = (int)K; p.t.cluster = pl.cluster;
-  p.t.err = reinterpret_cast<unsigned*>(sc + kTcCounterBytes - 4);
+  p.t = t;
   p.swT = swT; p.xq = xq; p.ksteps = pl.ksteps; p.Np = (int)pl.Np; p.nblk = (int)(K / block_size);
   p.tilesN = (int)(pl.Np / 128);
   switch (block_size) {
@@ -687,6 +723,23 @@ extern "C" int tpx_qlinear_qint8_tc(const int8_t* wq, const float* swT, const ui
     case 256: return i8_launch_tok<8>(pl.tokp, mw, p, pl.tiles, st);
     default: return i8_launch_tok<16>(pl.tokp, mw, p, pl.tiles, st);
   }
+}
+
+extern "C" int tpx_qlinear_qint8_tc(const int8_t* wq, const float* swT, const uint16_t* x, const void* gamma, int gamma_is_f32, float eps,
+                                    int64_t M, int64_t N, int64_t K, int64_t block_size, int reuse_act, const uint16_t* bias, int act, const uint16_t* mul_in,
+                                    const uint16_t* res, float res_scale, uint16_t* y, void* scratch, size_t scratch_bytes, void* stream) {
+  // between 17 and 32 tokens the order of the quantised activations depends on N, which the previous call may have had another of
+  if (block_size == 64 && M > 16 && M <= 32) reuse_act = 0;
+  return i8_linear(wq, swT, nullptr, nullptr, x, gamma, gamma_is_f32, eps, M, N, K, block_size, reuse_act, bias, act, mul_in, res, res_scale, y,
+                   scratch, scratch_bytes, stream);
+}
+
+extern "C" int tpx_qlinear_qint8_pair_tc(const int8_t* wq, const float* swT, const int8_t* wq2, const float* swT2, const uint16_t* x, const void* gamma,
+                                         int gamma_is_f32, float eps, int64_t M, int64_t N, int64_t K, int64_t block_size, int act, uint16_t* y,
+                                         void* scratch, size_t scratch_bytes, void* stream) {
+  TPX_REQUIRE(M == 0 || (wq2 && swT2), TPX_ERR_ARG, "qlinear_qint8_pair_tc: null pointer");
+  return i8_linear(wq, swT, wq2, swT2, x, gamma, gamma_is_f32, eps, M, N, K, block_size, 0, nullptr, act, nullptr, nullptr, 1.0f, y, scratch,
+                   scratch_bytes, stream);
 }
 
 
