@@ -31,6 +31,7 @@
 // arriver per tile) cost a store -> atomic -> load chain at loaded-memory latency (~2 us per hop).
 #include "tpx_mxfp4_dense.cuh"
 #include "tpx_tc_ptx.cuh"
+#include "tpx_qlinear_mx_rows.cuh"
 #include <algorithm>
 #include <cuda_fp8.h>
 
@@ -817,12 +818,18 @@ int tc_padded_ks(int64_t K, bool pair) {
   return (ks + m - 1) / m * m;
 }
 
+static int tc_check_norm(const uint16_t* x, int64_t K, int KS, const TcNorm& norm) {
+  TPX_REQUIRE(KS * 16 <= kNsThreads * kNsVecs, TPX_ERR_UNSUPPORTED, "fused RMSNorm: rows of more than %d elements are not supported (K=%ld)",
+              kNsThreads * kNsVecs * 8, (long)K);
+  TPX_REQUIRE((((uintptr_t)x | (uintptr_t)norm.gamma) & 15) == 0, TPX_ERR_ARG, "fused RMSNorm: x and gamma must be 16-byte aligned");
+  return TPX_OK;
+}
+
 int tc_launch_split(const uint16_t* x, int M, int K, int Mpad, int KS, int TOK, int UKS, int rowmap, uint8_t* terms, uint8_t* sfb,
                     cudaStream_t st, const TcNorm* norm) {
   if (norm && norm->gamma) {
-    TPX_REQUIRE(KS * 16 <= kNsThreads * kNsVecs, TPX_ERR_UNSUPPORTED, "fused RMSNorm: rows of more than %d elements are not supported (K=%d)",
-                kNsThreads * kNsVecs * 8, K);
-    TPX_REQUIRE((((uintptr_t)x | (uintptr_t)norm->gamma) & 15) == 0, TPX_ERR_ARG, "fused RMSNorm: x and gamma must be 16-byte aligned");
+    int rc = tc_check_norm(x, K, KS, *norm);
+    if (rc) return rc;
     TPX_CUDA_OK(launch_pdl(rmsnorm_split_kernel, dim3((unsigned)Mpad), dim3(kNsThreads), 0, st, x, norm->gamma, norm->gamma_f32, norm->eps, M, K,
                            KS, TOK, UKS, rowmap, terms, sfb));
     return TPX_OK;
@@ -1106,6 +1113,20 @@ static int tc_run(const uint8_t* wq, const uint8_t* sfa, int pair, const uint16_
     TPX_REQUIRE((kind == 0 || kind == 1) && !(norm && norm->gamma) && !dual, TPX_ERR_ARG, "qlinear_mxfp4_tc: this launch cannot take handed-over terms");
     with_pre.pre = &pre;
     norm = &with_pre;
+  }
+  // few tokens, unless a switch asks for one of the families or for terms handed from linear to linear
+  const Knobs& kn = knobs();
+  if (!wfmt && kind <= 1 && kn.tc_wide < 0 && kn.tc_f4 < 0 && kn.tc_w4 <= 0 && kn.tc_whole < 0 && kn.tc_cluster != 0 && M < kn.handoff_min &&
+      scratch_bytes >= kTcCounterBytes + mx_rows_scratch_bytes(M, K) && mx_rows_serves(M, N, K, dual)) {
+    const size_t need = tc_scratch_need(M, N, K, dual, kind);
+    TPX_REQUIRE(scratch && scratch_bytes >= need, TPX_ERR_SCRATCH, "qlinear_mxfp4_tc: scratch of %zu bytes needed, %zu given", need, scratch_bytes);
+    if (norm && norm->gamma) {
+      int rc = tc_check_norm(x, K, tc_padded_ks(K, dual), *norm);
+      if (rc) return rc;
+    }
+    TcParams b = {};
+    b.bias = bias; b.mul_in = mul_in; b.res = res; b.res_scale = res_scale; b.y = y; b.act = act;
+    return mx_rows_run(wq, sfa, dual, x, M, N, K, tc_padded_ks(K, dual), b, reinterpret_cast<unsigned char*>(scratch) + kTcCounterBytes, (cudaStream_t)stream, norm);
   }
   if (kind == 5) {
     TcParams b = {};
