@@ -5,16 +5,17 @@
 //
 // A column of S (one value channel) evolves without the others, so the work can be cut along value channels; only the output
 // norm needs a whole head. Kernels:
-//   gla_fast_kernel   bf16, several tokens. Tokens go through the state four at a time: with c_t the decays' product from
+//   gla_fast_kernel   several tokens. Tokens go through the state four at a time: with c_t the decays' product from
 //                     the block's first token to t, and s_t that from t + 1 to its last,
 //                       o_t = (q_t c_t)^T S + sum_(u <= t) (q_t . k_u prod_(u < x <= t) w_x) v_u,
 //                       S <- diag(c_3) S + sum_t (k_t s_t) v_t^T
 //                     i.e. 9 operations per state element for four tokens instead of 12, no division by a decay (all factors are
 //                     products of decays, at most 1), and no dependency between lanes. The state stays in registers, in pairs of key channels
-//                     (packed fp32). DP / LPC key channels x CPT columns per thread.
+//                     (packed fp32). DP / LPC key channels x CPT columns per thread. In fp32 models the decays and gates take the
+//                     library's functions: 2 x 513 tokens, 16 heads of 64 / 128: 427 us token by token, 60 so.
 //   gla_token_kernel  one token: a CTA per (sequence, head) streams the state through once; the low-rank map of the decay is
 //                     computed here as well.
-//   gla_kernel        any type and size, token by token; a column's key channels on neighbouring lanes.
+//   gla_kernel        any size, token by token; a column's key channels on neighbouring lanes.
 // The last and the column-cut form of the first leave o in `raw`; gla_out_kernel finishes it.
 #include "tpx_hybrid.cuh"
 
@@ -32,7 +33,7 @@ __device__ __forceinline__ int gla_first(const TpxGla& p, int b) {  // tokens of
   return n < 0 ? 0 : n > p.S ? (int)p.S : (int)n;
 }
 
-// ---------------------------------------------------------------- any type and size
+// ---------------------------------------------------------------- any size
 constexpr int kGlaTok = 8;
 
 template <int DP>
@@ -206,8 +207,8 @@ __global__ void __launch_bounds__(kGlaTokThreads) gla_token_kernel(TpxGla p) {
   }
 }
 
-// ---------------------------------------------------------------- bf16, several tokens
-// the same on the special-function unit; what counts of the logarithm is its absolute error, below 4e-7
+// ---------------------------------------------------------------- several tokens
+// the decay on the special-function unit, for bf16 mode; what counts of the logarithm is its absolute error, below 4e-7
 __device__ __forceinline__ float gl_ex2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -237,9 +238,10 @@ __device__ __forceinline__ void gl_cp16(void* dst, const void* src, bool ok) {  
 }
 __device__ __forceinline__ float gl_lo(uint32_t v) { return __uint_as_float(v << 16); }
 __device__ __forceinline__ float gl_hi(uint32_t v) { return __uint_as_float(v & 0xffff0000u); }
-// N consecutive bf16 values from shared memory as floats
+// N consecutive values from shared memory as floats
 template <int N>
-__device__ __forceinline__ void gl_ld_bf16(const uint16_t* p, float (&v)[N]) {
+__device__ __forceinline__ void gl_ld(const __nv_bfloat16* q, float (&v)[N]) {
+  const uint16_t* p = reinterpret_cast<const uint16_t*>(q);
   if constexpr (N % 8 == 0) {
 #pragma unroll
     for (int i = 0; i < N; i += 8) {
@@ -276,6 +278,8 @@ __device__ __forceinline__ void gl_ld_f32(const float* p, float (&v)[N]) {
   }
 }
 template <int N>
+__device__ __forceinline__ void gl_ld(const float* p, float (&v)[N]) { gl_ld_f32<N>(p, v); }
+template <int N>
 __device__ __forceinline__ void gl_st_f32(float* p, const float (&v)[N]) {
   if constexpr (N % 4 == 0) {
 #pragma unroll
@@ -290,17 +294,18 @@ __device__ __forceinline__ void gl_st_f32(float* p, const float (&v)[N]) {
 
 // DP: key channels (padded), EC: columns of a CTA, LPC lanes per column, CPT columns per thread, TC tokens staged at once;
 // WHOLE: the CTA has all columns of the head and finishes the output
-template <int DP, int EC, int LPC, int CPT, int TC, bool WHOLE>
+template <typename T, int DP, int EC, int LPC, int CPT, int TC, bool WHOLE>
 struct GfCfg {
+  static constexpr int EB = sizeof(T), EU = 16 / EB;  // bytes of an element, elements of a 16-byte unit
   static constexpr int KPT = DP / LPC, THREADS = EC / CPT * LPC, NW = THREADS / 32, NB = TC / 4;
   static constexpr int STAGED = 2 * TC * DP + NB * (DP + 16) + (WHOLE ? TC * EC : 0);  // floats
-  static constexpr int RQ = 0, RK = TC * DP * 2, RZ = 2 * RK, RV = RZ + TC * DP * 4, RG = RV + TC * EC * 2, RAW = RG + (WHOLE ? TC * EC * 2 : 0);
+  static constexpr int RQ = 0, RK = TC * DP * EB, RZ = 2 * RK, RV = RZ + TC * DP * 4, RG = RV + TC * EC * EB, RAW = RG + (WHOLE ? TC * EC * EB : 0);
   static constexpr size_t SMEM = STAGED * 4 + 2 * RAW;
   static constexpr int M = 4 * CPT / LPC;  // read-outs a lane ends with per block of four tokens
   static_assert(KPT % 4 == 0 && THREADS % 32 == 0 && LPC <= 32 && 4 * CPT >= LPC && (STAGED * 4) % 16 == 0, "whole vectors and warps");
   static_assert(M <= CPT, "a lane's read-outs belong to one token");
-  // 16-byte units that a thread copies: rows of DP bf16, DP fp32, EC bf16; a thread keeps its place in the row
-  static constexpr int UD = DP / 8, UZ = DP / 4, UE = EC / 8;
+  // 16-byte units that a thread copies: rows of DP elements, DP fp32, EC elements; a thread keeps its place in the row
+  static constexpr int UD = DP / EU, UZ = DP / 4, UE = EC / EU;
   static_assert(THREADS % UD == 0 && THREADS % UZ == 0 && THREADS % UE == 0, "copies");
   static constexpr int OW = EC / 32;  // columns per lane in the output norm
 };
@@ -311,9 +316,10 @@ __device__ __forceinline__ void gl_sync() {
   else __syncthreads();
 }
 
-template <int DP, int EC, int LPC, int CPT, int TC, bool WHOLE>
-__global__ void __launch_bounds__(GfCfg<DP, EC, LPC, CPT, TC, WHOLE>::THREADS) gla_fast_kernel(TpxGla p) {
-  using C = GfCfg<DP, EC, LPC, CPT, TC, WHOLE>;
+template <typename T, int DP, int EC, int LPC, int CPT, int TC, bool WHOLE>
+__global__ void __launch_bounds__(GfCfg<T, DP, EC, LPC, CPT, TC, WHOLE>::THREADS) gla_fast_kernel(TpxGla p) {
+  using C = GfCfg<T, DP, EC, LPC, CPT, TC, WHOLE>;
+  constexpr bool F32 = sizeof(T) == 4;
   constexpr int KV = C::KPT / 4, KP = C::KPT / 2, M = C::M;
   extern __shared__ __align__(16) float gf_smem[];
   float *s_q = gf_smem, *s_k = s_q + TC * DP, *s_a = s_k + TC * DP, *s_d = s_a + C::NB * DP, *s_o = s_d + C::NB * 16;
@@ -329,13 +335,13 @@ __global__ void __launch_bounds__(GfCfg<DP, EC, LPC, CPT, TC, WHOLE>::THREADS) g
   pdl_wait();
   const int first = gla_first(p, b);
   const int64_t row0 = (int64_t)b * S;
-  const uint16_t* proj = reinterpret_cast<const uint16_t*>(p.proj) + (row0 + first) * ldp;
+  const T* proj = reinterpret_cast<const T*>(p.proj) + (row0 + first) * ldp;
   // this thread's places in the rows it copies
-  const uint16_t* fq = proj + (int64_t)(tid / C::UD) * ldp + p.q_col + head * dim + tid % C::UD * 8;
-  const uint16_t* fv = proj + (int64_t)(tid / C::UE) * ldp + p.v_col + head * vdim + e0 + tid % C::UE * 8;
+  const T* fq = proj + (int64_t)(tid / C::UD) * ldp + p.q_col + head * dim + tid % C::UD * C::EU;
+  const T* fv = proj + (int64_t)(tid / C::UE) * ldp + p.v_col + head * vdim + e0 + tid % C::UE * C::EU;
   const float* fz = p.zraw + (row0 + first + tid / C::UZ) * zd + head * dim + tid % C::UZ * 4;
   const int64_t kq = p.k_col - p.q_col, gv = p.g_col - p.v_col;
-  const bool inq = tid % C::UD * 8 < dim, inz = tid % C::UZ * 4 < dim, inv = tid % C::UE * 8 < cols;
+  const bool inq = tid % C::UD * C::EU < dim, inz = tid % C::UZ * 4 < dim, inv = tid % C::UE * C::EU < cols;
 
   auto fetch = [&](int t0, int stage) {  // tokens beyond the call and channels beyond the head read as zero
     unsigned char* dst = raw + stage * C::RAW + tid * 16;
@@ -343,10 +349,10 @@ __global__ void __launch_bounds__(GfCfg<DP, EC, LPC, CPT, TC, WHOLE>::THREADS) g
 #pragma unroll
     for (int i = 0; i < TC; i += C::THREADS / C::UD) {
       const bool ok = inq && tid / C::UD + i < n && (C::THREADS / C::UD <= TC || tid / C::UD < TC);
-      const uint16_t* src = ok ? fq + (int64_t)i * ldp : proj;
+      const T* src = ok ? fq + (int64_t)i * ldp : proj;
       if (C::THREADS / C::UD <= TC || tid / C::UD < TC) {
-        gl_cp16(dst + C::RQ + i * DP * 2, src, ok);
-        gl_cp16(dst + C::RK + i * DP * 2, ok ? src + kq : proj, ok);
+        gl_cp16(dst + C::RQ + i * DP * C::EB, src, ok);
+        gl_cp16(dst + C::RK + i * DP * C::EB, ok ? src + kq : proj, ok);
       }
     }
 #pragma unroll
@@ -357,10 +363,10 @@ __global__ void __launch_bounds__(GfCfg<DP, EC, LPC, CPT, TC, WHOLE>::THREADS) g
 #pragma unroll
     for (int i = 0; i < TC; i += C::THREADS / C::UE) {
       const bool ok = inv && tid / C::UE + i < n;
-      const uint16_t* src = ok ? fv + (int64_t)i * ldp : proj;
+      const T* src = ok ? fv + (int64_t)i * ldp : proj;
       if (C::THREADS / C::UE <= TC || tid / C::UE < TC) {
-        gl_cp16(dst + C::RV + i * EC * 2, src, ok);
-        if (WHOLE) gl_cp16(dst + C::RG + i * EC * 2, ok ? src + gv : proj, ok);
+        gl_cp16(dst + C::RV + i * EC * C::EB, src, ok);
+        if (WHOLE) gl_cp16(dst + C::RG + i * EC * C::EB, ok ? src + gv : proj, ok);
       }
     }
     fq += (int64_t)TC * ldp;
@@ -370,8 +376,8 @@ __global__ void __launch_bounds__(GfCfg<DP, EC, LPC, CPT, TC, WHOLE>::THREADS) g
   };
   if (first < S) fetch(first, 0);
   if (WHOLE) {  // padding
-    uint16_t* out = reinterpret_cast<uint16_t*>(p.out) + row0 * p.ldo + head * vdim;
-    for (int i = tid; i < first * vdim; i += C::THREADS) out[(int64_t)(i / vdim) * p.ldo + i % vdim] = 0;
+    T* out = reinterpret_cast<T*>(p.out) + row0 * p.ldo + head * vdim;
+    for (int i = tid; i < first * vdim; i += C::THREADS) hy_st(out + (int64_t)(i / vdim) * p.ldo + i % vdim, 0.0f);
   }
 
   float nw[WHOLE ? C::OW : 1];
@@ -404,23 +410,23 @@ __global__ void __launch_bounds__(GfCfg<DP, EC, LPC, CPT, TC, WHOLE>::THREADS) g
     gl_sync<C::THREADS>();
     if (t0 + TC < S) fetch(t0 + TC, stage ^ 1);
     const unsigned char* rw = raw + stage * C::RAW;
-    const uint16_t* rv = reinterpret_cast<const uint16_t*>(rw + C::RV);
+    const T* rv = reinterpret_cast<const T*>(rw + C::RV);
     // the vectors of a block of four tokens: a warp per block, neighbouring channels per lane
     for (int blk = warp; blk < C::NB; blk += C::NW) {
       const int c = lane * CW;
-      const uint16_t* rq = reinterpret_cast<const uint16_t*>(rw + C::RQ) + blk * 4 * DP + c;
-      const uint16_t* rk = reinterpret_cast<const uint16_t*>(rw + C::RK) + blk * 4 * DP + c;
+      const T* rq = reinterpret_cast<const T*>(rw + C::RQ) + blk * 4 * DP + c;
+      const T* rk = reinterpret_cast<const T*>(rw + C::RK) + blk * 4 * DP + c;
       const float* rz = reinterpret_cast<const float*>(rw + C::RZ) + blk * 4 * DP + c;
       float q[4][CW], k[4][CW], a[4][CW], d[16];
 #pragma unroll
       for (int t = 0; t < 4; t++) {
-        gl_ld_bf16<CW>(rq + t * DP, q[t]);
-        gl_ld_bf16<CW>(rk + t * DP, k[t]);
+        gl_ld<CW>(rq + t * DP, q[t]);
+        gl_ld<CW>(rk + t * DP, k[t]);
         gl_ld_f32<CW>(rz + t * DP, a[t]);
 #pragma unroll
         for (int i = 0; i < CW; i++) {
           q[t][i] *= scale;
-          a[t][i] = blk * 4 + t < n ? gl_decay(a[t][i], inv_tau) : 1.0f;
+          a[t][i] = blk * 4 + t < n ? (F32 ? gla_decay(a[t][i], inv_tau) : gl_decay(a[t][i], inv_tau)) : 1.0f;
         }
       }
 #pragma unroll
@@ -505,7 +511,7 @@ __global__ void __launch_bounds__(GfCfg<DP, EC, LPC, CPT, TC, WHOLE>::THREADS) g
       for (int t = 0; t < 4; t++) {
         const float4* pk = reinterpret_cast<const float4*>(s_k + (blk * 4 + t) * DP) + l;
         float v[CPT];
-        gl_ld_bf16<CPT>(rv + (blk * 4 + t) * EC + c0, v);
+        gl_ld<CPT>(rv + (blk * 4 + t) * EC + c0, v);
         float4 k[KV];
 #pragma unroll
         for (int i = 0; i < KV; i++) k[i] = pk[i * LPC];
@@ -539,7 +545,7 @@ __global__ void __launch_bounds__(GfCfg<DP, EC, LPC, CPT, TC, WHOLE>::THREADS) g
 #pragma unroll
       for (int u = 0; u < 4; u++) {
         float w[M];
-        gl_ld_bf16<M>(rv + (blk * 4 + u) * EC + c0 + c, w);
+        gl_ld<M>(rv + (blk * 4 + u) * EC + c0 + c, w);
 #pragma unroll
         for (int i = 0; i < M; i++) r[i] = fmaf(dd[u], w[i], r[i]);
       }
@@ -549,23 +555,25 @@ __global__ void __launch_bounds__(GfCfg<DP, EC, LPC, CPT, TC, WHOLE>::THREADS) g
     if (WHOLE) {
       gl_sync<C::THREADS>();
       // output norm and gate: a warp per token
-      const uint16_t* rg = reinterpret_cast<const uint16_t*>(rw + C::RG);
+      const T* rg = reinterpret_cast<const T*>(rw + C::RG);
       const int c = lane * C::OW;
-      uint16_t* out = reinterpret_cast<uint16_t*>(p.out) + (row0 + t0) * p.ldo + head * vdim + c;
+      T* out = reinterpret_cast<T*>(p.out) + (row0 + t0) * p.ldo + head * vdim + c;
       for (int t = warp; t < n; t += C::NW) {
         float x[C::OW], g[C::OW], ss = 0.0f;
         gl_ld_f32<C::OW>(s_o + t * EC + c, x);
-        gl_ld_bf16<C::OW>(rg + t * EC + c, g);
+        gl_ld<C::OW>(rg + t * EC + c, g);
 #pragma unroll
         for (int i = 0; i < C::OW; i++) ss = fmaf(x[i], x[i], ss);
         if (c >= cols) ss = 0.0f;
-        const float rms = rsqrtf(hy_warp_sum(ss) / (float)vdim + p.eps);
+        const float ms = hy_warp_sum(ss) / (float)vdim + p.eps, rms = F32 ? 1.0f / sqrtf(ms) : rsqrtf(ms);
 #pragma unroll
-        for (int i = 0; i < C::OW; i++) x[i] = x[i] * rms * nw[i] * gl_silu(g[i]);
+        for (int i = 0; i < C::OW; i++) x[i] = x[i] * rms * nw[i] * (F32 ? gla_silu(g[i]) : gl_silu(g[i]));
         if (c < cols) {
-          uint16_t* dst = out + (int64_t)t * p.ldo;
-          if constexpr (C::OW == 1) {
-            dst[0] = f32_to_bf16_bits(x[0]);
+          T* dst = out + (int64_t)t * p.ldo;
+          if constexpr (F32) {
+            gl_st_f32<C::OW>(dst, x);
+          } else if constexpr (C::OW == 1) {
+            hy_st(dst, x[0]);
           } else {
 #pragma unroll
             for (int i = 0; i < C::OW; i += 2) {
@@ -606,11 +614,11 @@ static int gla_out(const TpxGla& p, cudaStream_t st) {
   return TPX_OK;
 }
 
-template <int DP, int EC, int LPC, int CPT, int TC, bool WHOLE>
+template <typename T, int DP, int EC, int LPC, int CPT, int TC, bool WHOLE>
 static int gla_fast_launch(const TpxGla& p, cudaStream_t st) {
-  using C = GfCfg<DP, EC, LPC, CPT, TC, WHOLE>;
+  using C = GfCfg<T, DP, EC, LPC, CPT, TC, WHOLE>;
   static bool opted[16] = {};
-  void (*k)(TpxGla) = gla_fast_kernel<DP, EC, LPC, CPT, TC, WHOLE>;
+  void (*k)(TpxGla) = gla_fast_kernel<T, DP, EC, LPC, CPT, TC, WHOLE>;
   const int rc = gla_opt_in((const void*)k, C::SMEM, opted);
   if (rc) return rc;
   TPX_CUDA_OK(launch_pdl(k, dim3((unsigned)p.heads, (unsigned)(WHOLE ? 1 : (p.vdim + EC - 1) / EC), (unsigned)p.B), dim3(C::THREADS), C::SMEM, st, p));
@@ -618,27 +626,28 @@ static int gla_fast_launch(const TpxGla& p, cudaStream_t st) {
 }
 
 static bool gla_fast_serves(const TpxGla& a) {
-  return !a.f32 && a.dim % 8 == 0 && a.vdim % 8 == 0 && a.dim <= 128 && a.ldp % 8 == 0 && a.q_col % 8 == 0 && a.k_col % 8 == 0 && a.v_col % 8 == 0 &&
+  return a.dim % 8 == 0 && a.vdim % 8 == 0 && a.dim <= 128 && a.ldp % 8 == 0 && a.q_col % 8 == 0 && a.k_col % 8 == 0 && a.v_col % 8 == 0 &&
          a.g_col % 8 == 0 && a.ldp < (1ll << 30) && a.heads * a.dim < (1ll << 30) &&
          a.ldo % 8 == 0 && (((uintptr_t)a.proj | (uintptr_t)a.zraw | (uintptr_t)a.state | (uintptr_t)a.raw | (uintptr_t)a.out) & 15) == 0;
 }
 
+template <typename T>
 static int gla_fast(const TpxGla& a, cudaStream_t st) {
   // whole heads per CTA when there are many, columns cut over CTAs when a token's latency counts
   const bool many = a.vdim <= 256 && a.B * a.heads >= 2 * sm_count();
   if (a.dim <= 32) {
-    if (!many) return gla_fast_launch<32, 32, 8, 4, 16, false>(a, st);
-    return a.vdim <= 64 ? gla_fast_launch<32, 64, 4, 8, 8, true>(a, st) : a.vdim <= 128 ? gla_fast_launch<32, 128, 4, 8, 8, true>(a, st)
-                                                                                       : gla_fast_launch<32, 256, 4, 8, 8, true>(a, st);
+    if (!many) return gla_fast_launch<T, 32, 32, 8, 4, 16, false>(a, st);
+    return a.vdim <= 64 ? gla_fast_launch<T, 32, 64, 4, 8, 8, true>(a, st) : a.vdim <= 128 ? gla_fast_launch<T, 32, 128, 4, 8, 8, true>(a, st)
+                                                                                       : gla_fast_launch<T, 32, 256, 4, 8, 8, true>(a, st);
   }
   if (a.dim <= 64) {
-    if (!many) return gla_fast_launch<64, 32, 16, 4, 16, false>(a, st);
-    return a.vdim <= 64 ? gla_fast_launch<64, 64, 4, 8, 16, true>(a, st) : a.vdim <= 128 ? gla_fast_launch<64, 128, 4, 8, 16, true>(a, st)
-                                                                                       : gla_fast_launch<64, 256, 4, 8, 16, true>(a, st);
+    if (!many) return gla_fast_launch<T, 64, 32, 16, 4, 16, false>(a, st);
+    return a.vdim <= 64 ? gla_fast_launch<T, 64, 64, 4, 8, 16, true>(a, st) : a.vdim <= 128 ? gla_fast_launch<T, 64, 128, 4, 8, 16, true>(a, st)
+                                                                                       : gla_fast_launch<T, 64, 256, 4, 8, 16, true>(a, st);
   }
-  if (!many) return gla_fast_launch<128, 32, 16, 4, 16, false>(a, st);
-  return a.vdim <= 64 ? gla_fast_launch<128, 64, 8, 8, 8, true>(a, st) : a.vdim <= 128 ? gla_fast_launch<128, 128, 8, 8, 8, true>(a, st)
-                                                                                      : gla_fast_launch<128, 256, 8, 8, 8, true>(a, st);
+  if (!many) return gla_fast_launch<T, 128, 32, 16, 4, 16, false>(a, st);
+  return a.vdim <= 64 ? gla_fast_launch<T, 128, 64, 8, 8, 8, true>(a, st) : a.vdim <= 128 ? gla_fast_launch<T, 128, 128, 8, 8, 8, true>(a, st)
+                                                                                      : gla_fast_launch<T, 128, 256, 8, 8, 8, true>(a, st);
 }
 
 template <typename T, int DP>
@@ -692,6 +701,6 @@ extern "C" int tpx_gla(const TpxGla* a, void* stream) {
   cudaStream_t st = (cudaStream_t)stream;
   if (token) return gla_token(*a, st);
   TPX_REQUIRE(a->raw, TPX_ERR_ARG, "gla: null pointer");
-  if (gla_fast_serves(*a)) return gla_fast(*a, st);
+  if (gla_fast_serves(*a)) return a->f32 ? gla_fast<float>(*a, st) : gla_fast<__nv_bfloat16>(*a, st);
   return a->f32 ? gla_run<float>(*a, st) : gla_run<__nv_bfloat16>(*a, st);
 }
