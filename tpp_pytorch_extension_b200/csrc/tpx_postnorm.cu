@@ -6,6 +6,7 @@
 // computes the inverse root mean squares, then every thread walks its channels through the tokens with the convolution's
 // history in registers. One token per sequence: a CTA per sequence, the history in the layer's state.
 #include "tpx_hybrid.cuh"
+#include "tpx_argmax.cuh"
 
 namespace tpx {
 
@@ -325,38 +326,6 @@ __global__ void __launch_bounds__(256) pnc_final_kernel(const float* __restrict_
   for (int d = D + threadIdx.x; d < ldo; d += 256) hy_st(out + d, 0.0f);
 }
 
-__global__ void __launch_bounds__(256) argmax_f32_kernel(const float* __restrict__ x, long long n, long long* __restrict__ out) {
-  __shared__ float sv[8];
-  __shared__ long long si[8];
-  pdl_trigger();
-  pdl_wait();
-  x += (long long)blockIdx.x * n;
-  float bv = -INFINITY;
-  long long bi = 0;
-  auto take = [&](float v, long long i) {
-    const bool vn = v != v, bn = bv != bv;  // a NaN counts as the largest, as in torch.argmax
-    if (vn != bn ? vn : (!vn && v != bv) ? v > bv : i < bi) { bv = v; bi = i; }
-  };
-  bool any = false;
-  for (long long i = threadIdx.x; i < n; i += 256) {
-    if (!any) { bv = x[i]; bi = i; any = true; }
-    else take(x[i], i);
-  }
-  if (!any) bi = 0x7fffffffffffffffLL;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const float v = __shfl_xor_sync(0xffffffffu, bv, o);
-    const long long i = __shfl_xor_sync(0xffffffffu, bi, o);
-    take(v, i);
-  }
-  if ((threadIdx.x & 31) == 0) { sv[threadIdx.x >> 5] = bv; si[threadIdx.x >> 5] = bi; }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int i = 1; i < 8; i++) take(sv[i], si[i]);
-    out[blockIdx.x] = bi;
-  }
-}
-
 template <typename T>
 static int pnc_run(const TpxPostnormConv& a, cudaStream_t st) {
   PncParams<T> p = {a.ids, (const T*)a.embed, a.x, a.y, a.w, a.conv, a.state, a.start, a.dev_len, a.x_out, (T*)a.h,
@@ -418,7 +387,7 @@ extern "C" int tpx_argmax_f32(const float* x, int64_t rows, int64_t n, int64_t* 
   TPX_REQUIRE(rows >= 0 && n > 0, TPX_ERR_ARG, "argmax_f32: bad shape");
   if (rows == 0) return TPX_OK;
   TPX_REQUIRE(x && out, TPX_ERR_ARG, "argmax_f32: null pointer");
-  TPX_CUDA_OK(launch_pdl(argmax_f32_kernel, dim3((unsigned)rows), dim3(256), 0, (cudaStream_t)stream, x, (long long)n,
+  TPX_CUDA_OK(launch_pdl(argmax_kernel<float>, dim3((unsigned)rows), dim3(kArgmaxThreads), 0, (cudaStream_t)stream, x, (long long)n,
                          reinterpret_cast<long long*>(out)));
   return TPX_OK;
 }
