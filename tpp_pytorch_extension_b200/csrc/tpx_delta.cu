@@ -17,7 +17,7 @@
 // so that a token costs four multiply-adds per state element instead of five and reads the state once; at the chunk's end
 // s is multiplied by G. A decay is at least exp(-0.61), G at least 6e-5 after 16 tokens: nothing under- or overflows, and a
 // scale per channel does not change relative rounding.
-#include "tpx_hybrid.cuh"
+#include "tpx_delta.cuh"
 
 namespace tpx {
 
@@ -167,22 +167,6 @@ __device__ __forceinline__ float2 dl_mul2(float2 a, float2 b) {
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(*reinterpret_cast<unsigned long long*>(&a)), "l"(*reinterpret_cast<unsigned long long*>(&b)));
   return *reinterpret_cast<float2*>(&r);
 }
-__device__ __forceinline__ void dl_cp16(void* dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ float dl_sigmoid(float v) { return __fdividef(1.0f, 1.0f + __expf(-v)); }
-
-struct DeltaFastParams {
-  const uint16_t* proj;
-  const float *wraw, *a_bias, *norm_w;
-  const int *start, *dev_len;
-  float* state;
-  uint16_t* out;
-  long long ldp, ldo;
-  int S, past, H, dim;
-  float eps;
-};
-
 template <int DP, int LPC, int CPT, int TC>
 struct DfCfg {
   static constexpr int KPT = DP / LPC, THREADS = DP * LPC / CPT, NW = THREADS / 32;
@@ -491,6 +475,9 @@ static bool delta_fast_serves(const TpxDeltaRule& a) {
 static int delta_fast(const TpxDeltaRule& a, cudaStream_t st) {
   DeltaFastParams p = {(const uint16_t*)a.proj, a.wraw, a.a_bias, a.norm_w, a.start, a.dev_len, a.state, (uint16_t*)a.out, (long long)a.ldp,
                        (long long)a.ldo, (int)a.S, (int)a.past, (int)a.heads, (int)a.dim, a.eps};
+  // Heads of 64 that one round of CTAs holds: sixteen tokens at a time as matrix products, from 32 tokens on (1 x 4096, 64 heads: 1380 us token by token, 900 so;
+  // 2 x 512, 16 heads 177 / 120; 1 x 33, 2 heads 20 / 16). With more heads the token loop has enough warps (16 x 256, 64 heads: 381 / 410).
+  if (a.dim == 64 && a.S >= 32 && a.B * a.heads <= sm_count()) return delta_chunk(p, a.B, st);
   // eight columns per thread and few warps per head when there are many heads, more warps per head when a token's latency counts
   const bool many = a.B * a.heads >= (a.dim <= 64 ? 4 : 2) * sm_count();
   if (a.dim <= 32) return a.S == 1 ? delta_fast_launch<32, 4, 4, 1>(p, a.B, st) : delta_fast_launch<32, 4, 4, 8>(p, a.B, st);
