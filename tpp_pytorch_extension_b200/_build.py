@@ -23,8 +23,8 @@ NVCC_FLAGS = [
 
 
 # sources of models that do not need the whole library (names without the tpx_ prefix)
-COMPONENTS = {"Dofivik": ("api", "linear_bf16", "linear_bf16_pair", "linear_f32", "linear_f32_pair", "postnorm", "latent", "latent_tc", "latent_dec", "delta", "delta_chunk"),
-              "Vedizen": ("api", "linear_bf16", "linear_bf16_pair", "linear_f32", "linear_f32_pair", "postnorm", "dyt", "gla", "diff", "diff_tc", "diff_dec")}
+COMPONENTS = {"Dofivik": ("api", "linear_bf16", "linear_bf16_pair", "linear_bf16_rows", "linear_f32", "linear_f32_pair", "postnorm", "latent", "latent_tc", "latent_dec", "delta", "delta_chunk"),
+              "Vedizen": ("api", "linear_bf16", "linear_bf16_pair", "linear_bf16_rows", "linear_f32", "linear_f32_pair", "postnorm", "dyt", "gla", "diff", "diff_tc", "diff_dec")}
 
 
 def sources():

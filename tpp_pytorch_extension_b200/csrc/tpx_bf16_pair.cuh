@@ -51,6 +51,9 @@ bool f32_pair_serves(const TpxLinear& a);
 int f32_pair_run(const TpxLinear& a, const F32Epi& e, cudaStream_t st);
 int f32_fma_run(const TpxLinear& a, const F32Epi& e, int64_t m0, int64_t rows, const unsigned* flags, int64_t slab, cudaStream_t st);
 
+// few tokens (tpx_linear_bf16_rows.cu)
+bool bf_rows_serves(int64_t M, int64_t N, int64_t K, int64_t ldw);
+int bf_rows_run(const BfParams& b, const void* w, const void* x, int64_t M, int64_t N, int64_t K, int64_t ldw, int64_t ldx, cudaStream_t st);
 int bf_make_map(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows);
 // many tokens on CTA pairs (tpx_linear_bf16_pair.cu): whether it takes this call, its scratch, the call
 bool bf_pair_serves(const BfParams& p, int64_t M, int64_t N, int64_t K);

@@ -19,7 +19,8 @@
 // stages instead (BfParams::split): every CTA streams the same number of weight bytes, and the pieces of a tile that was
 // cut are added in the order of k by the CTA that finishes last (fp32 partials and an arrival counter in the scratch; no
 // CTA waits for another). Two accumulators in tensor memory: the
-// epilogue of a tile runs under the MMAs of the next. At decode sizes the kernel is a plain stream of W at HBM rate.
+// epilogue of a tile runs under the MMAs of the next. Up to 32 tokens it has only the largest weights: the others stream
+// through the warps' own rings (tpx_linear_bf16_rows.cu), where a call of 4096 x 4096 takes 7.2 us instead of 13.6.
 #include "tpx_bf16_pair.cuh"
 
 namespace tpx {
@@ -409,6 +410,7 @@ static size_t bf_split_bytes(int64_t M, int grid) { return (size_t)grid * 2 * (M
 static int bf_run(BfParams& p, const void* w, const void* x, int64_t M, int64_t N, int64_t K, int64_t ldw, int64_t ldx, void* scratch,
                   size_t scratch_bytes, cudaStream_t st) {
   if (bf_pair_serves(p, M, N, K)) return bf_pair_run(p, w, x, M, N, K, ldw, ldx, scratch, scratch_bytes, st);
+  if (bf_rows_serves(M, N, K, ldw)) return bf_rows_run(p, w, x, M, N, K, ldw, ldx, st);
   p.ctas = bf_split_ctas(M, N, K);
   if (p.ctas && scratch_bytes < kTcCounterBytes + bf_split_bytes(M, p.ctas)) p.ctas = 0;
   p.t.counters = reinterpret_cast<unsigned*>(scratch);
