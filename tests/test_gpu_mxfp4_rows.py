@@ -148,3 +148,17 @@ def test_recorded_chain(M):
         graph.replay()
         torch.cuda.synchronize()
         assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("M", [1, 8])
+def test_result_over_activations(M):
+    from tpp_pytorch_extension_b200._C import _fused_llm_infer as F
+    from tpp_pytorch_extension_b200.llm.llm_common import quantize_weight
+    g = torch.Generator(device="cuda").manual_seed(M)
+    w = quantize_weight((torch.randn(2048, 2048, generator=g, device="cuda") * 0.02).to(torch.bfloat16), "mxfp4")
+    x = torch.randn(M, 2048, generator=g, device="cuda").to(torch.bfloat16)
+    want = F.fc_plain(x.clone(), w)
+    for _ in range(4):
+        y = x.clone()
+        F.fc_plain(y, w, out=y)
+        assert float((y - want).float().norm() / want.float().norm()) < 1e-3  # another group adds the same products

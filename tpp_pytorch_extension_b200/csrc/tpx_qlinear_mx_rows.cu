@@ -398,12 +398,6 @@ __global__ void __launch_bounds__(kMpThreads) mx_rows_prep_kernel(MxRowsParams p
   }
 }
 
-static bool mr_on_device(const void* x) {
-  cudaPointerAttributes a;
-  if (cudaPointerGetAttributes(&a, x) == cudaSuccess) return a.type == cudaMemoryTypeDevice;
-  (void)cudaGetLastError();
-  return false;
-}
 static size_t mr_stage_bytes(const MxRowsParams& p) { return (size_t)p.steps * p.t.M * (256 + 4); }
 
 template <int T, int MG, bool DUAL, int MODE>
@@ -426,9 +420,10 @@ static int mr_launch(MxRowsParams p, uint8_t* scratch, cudaStream_t st) {
   // By every CTA while that costs about what the launch in front would, which a caller of single linears pays for as well: one weight up to 20480 values (4096 x
   // 4096 at 1, 4 and 8 tokens 4.7, 5.3 and 6.2 us, by a kernel in front 5.0, 5.0, 5.1; 4096 x 14336 at 4 tokens 12.4 / 9.8), a pair of more than eight tiles 8 tokens
   // of 4096 (14336 x 4096 at 1 and 8 tokens 14.7 and 16.8, 15.9 and 16.0), behind a norm 2 tokens of 4096 (the same pair 15.9 and 20.8, 15.8 and 16.3). Activations in the
-  // host's memory are read once.
+  // host's memory are read once, and those that the result replaces before it is written.
   const long long values = (long long)p.steps * 128 * p.t.M;
-  if (p.t.M <= (p.gamma ? 2 : 8) && values <= (p.gamma ? 8192 : T > 8 ? 32768 : 20480) && mr_on_device(p.x))
+  if (p.t.M <= (p.gamma ? 2 : 8) && values <= (p.gamma ? 8192 : T > 8 ? 32768 : 20480) &&
+      rows_shared_x(p.x, (size_t)p.t.M * p.t.K * 2, p.t.y, (size_t)p.t.M * p.t.N * 2))
     return p.gamma ? mr_launch_mode<T, 1, DUAL, kMrNorm>(p, st) : mr_launch_mode<T, 1, DUAL, kMrStage>(p, st);
   const int Mp = p.t.M > 8 ? 16 : 8;
   p.xr = scratch;

@@ -37,6 +37,16 @@ __device__ __forceinline__ float rows_ld_member(uint32_t a, int c) {
   return v;
 }
 
+// Whether every CTA may read x for itself: x is in the memory of a device, and no CTA's y lands in it while another still reads.
+inline bool rows_shared_x(const void* x, size_t x_bytes, const void* y, size_t y_bytes) {
+  const uintptr_t a = (uintptr_t)x, b = (uintptr_t)y;
+  if (a < b + y_bytes && b < a + x_bytes) return false;
+  cudaPointerAttributes at;
+  if (cudaPointerGetAttributes(&at, x) == cudaSuccess) return at.type == cudaMemoryTypeDevice;
+  (void)cudaGetLastError();
+  return false;
+}
+
 // Feature tiles per CTA: one round of CTAs where that takes at most seven each, else the fewest rounds.
 inline int rows_tiles(int64_t tiles) {
   const int sms = sm_count();
