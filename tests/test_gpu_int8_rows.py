@@ -87,3 +87,44 @@ def test_recorded_chain(M, monkeypatch):
         graph.replay()
         torch.cuda.synchronize()
         assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("M", [1, 2])
+@pytest.mark.parametrize("K,f32", [(64, False), (4096, True), (4160, False), (8192, True), (8192, False)])
+def test_norm_and_reuse(M, K, f32):
+    from tpp_pytorch_extension_b200 import _lib
+    L, N = _lib.lib(), 272
+    g = torch.Generator(device="cuda").manual_seed(M + K)
+    q, s, wq, sw = _weight(N, K, g)
+    x = torch.randn(M, K, generator=g, device="cuda").to(torch.bfloat16)
+    gamma = torch.randn(K, generator=g, device="cuda").to(torch.float32 if f32 else torch.bfloat16)
+    need = L.tpx_qlinear_qint8_tc_scratch_bytes(M, N, K, 64)
+    sc = torch.zeros(need, device="cuda", dtype=torch.uint8)
+    y, again = (torch.empty(M, N, device="cuda", dtype=torch.bfloat16) for _ in "ya")
+
+    def call(x, gamma, reuse, y):
+        _lib.check(L.tpx_qlinear_qint8_tc(wq.data_ptr(), sw.data_ptr(), x.data_ptr(), _lib.ptr(gamma), int(f32), 1e-5, M, N, K, 64, reuse, None, 0, None, None, 0.0,
+                                          y.data_ptr(), sc.data_ptr(), need, _lib.stream()))
+
+    call(x, gamma, 0, y)
+    call(torch.zeros_like(x), None, 1, again)  # what the call before left in the scratch
+    assert torch.equal(y, again)
+    normed = (x.double() * (x.double().square().mean(-1, keepdim=True) + 1e-5).rsqrt() * gamma.double()).to(torch.bfloat16)
+    a, _ = _reference(normed, q, s, 64)
+    # a normed value may round to the neighbouring bf16 and its int8 to the neighbouring step: one step in a few of K values, random signs
+    assert float((y.double() - a).norm() / a.norm()) < 2.0 ** -8
+
+
+@pytest.mark.parametrize("M", [1, 2])
+def test_result_over_activations(M, monkeypatch):
+    from tpp_pytorch_extension_b200._C import _fused_llm_infer as F
+    from tpp_pytorch_extension_b200.llm.llm_common import quantize_weight
+    monkeypatch.setenv("QINT8_BLOCK_SIZE", "64")
+    g = torch.Generator(device="cuda").manual_seed(M)
+    w = quantize_weight((torch.randn(2048, 2048, generator=g, device="cuda") * 0.02).to(torch.bfloat16), "qint8")
+    x = torch.randn(M, 2048, generator=g, device="cuda").to(torch.bfloat16)
+    want = F.fc_plain(x.clone(), w)
+    for _ in range(4):
+        y = x.clone()
+        F.fc_plain(y, w, out=y)
+        assert torch.equal(y, want)

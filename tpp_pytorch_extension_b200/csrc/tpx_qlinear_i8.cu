@@ -135,14 +135,9 @@ __global__ void __launch_bounds__(kQaThreads) quantize_act_i8_row_kernel(const u
 #pragma unroll
   for (int q = 0; q < VECS; q++) {
     const int i = threadIdx.x + (blockIdx.y * VECS + q) * kQaThreads;
-    const uint4 v = live && i < nv ? xr[i] : make_uint4(0, 0, 0, 0);
-    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+    i8_unpack_bf16(live && i < nv ? xr[i] : make_uint4(0, 0, 0, 0), f[q]);
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-      f[q][2 * j] = bf16_bits_to_f32((uint16_t)(w[j] & 0xffff));
-      f[q][2 * j + 1] = bf16_bits_to_f32((uint16_t)(w[j] >> 16));
-      ss += f[q][2 * j] * f[q][2 * j] + f[q][2 * j + 1] * f[q][2 * j + 1];
-    }
+    for (int j = 0; j < 8; j += 2) ss += f[q][j] * f[q][j] + f[q][j + 1] * f[q][j + 1];
   }
   if (gamma) {
 #pragma unroll
@@ -158,18 +153,7 @@ __global__ void __launch_bounds__(kQaThreads) quantize_act_i8_row_kernel(const u
       const int i = threadIdx.x + q * kQaThreads;
       if (i >= nv) continue;
       float g[8];
-      if (gamma_f32) {
-        const float4 g0 = reinterpret_cast<const float4*>(gamma)[2 * i], g1 = reinterpret_cast<const float4*>(gamma)[2 * i + 1];
-        g[0] = g0.x; g[1] = g0.y; g[2] = g0.z; g[3] = g0.w; g[4] = g1.x; g[5] = g1.y; g[6] = g1.z; g[7] = g1.w;
-      } else {
-        const uint4 gv = reinterpret_cast<const uint4*>(gamma)[i];
-        const uint32_t gw[4] = {gv.x, gv.y, gv.z, gv.w};
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-          g[2 * j] = bf16_bits_to_f32((uint16_t)(gw[j] & 0xffff));
-          g[2 * j + 1] = bf16_bits_to_f32((uint16_t)(gw[j] >> 16));
-        }
-      }
+      i8_gamma(gamma, gamma_f32, i, g);
 #pragma unroll
       for (int j = 0; j < 8; j++) f[q][j] = bf16_bits_to_f32(f32_to_bf16_bits(f[q][j] * inv * g[j]));
     }
@@ -177,26 +161,10 @@ __global__ void __launch_bounds__(kQaThreads) quantize_act_i8_row_kernel(const u
 #pragma unroll
   for (int q = 0; q < VECS; q++) {
     const int i = threadIdx.x + (blockIdx.y * VECS + q) * kQaThreads;
-    float amax = 0.0f;
-#pragma unroll
-    for (int j = 0; j < 8; j++) amax = fmaxf(amax, fabsf(f[q][j]));
-    for (int o = 1; o < lanes; o <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-    const float scale = (float)((double)amax / 127.0);
-    const float iscale = scale != 0.0f ? 1.0f / scale : 0.0f;
-    uint32_t o2[2];
-#pragma unroll
-    for (int h = 0; h < 2; h++) {
-      uint32_t word = 0;
-#pragma unroll
-      for (int e = 0; e < 4; e++) {
-        float r = nearbyintf(f[q][4 * h + e] * iscale);
-        r = fminf(fmaxf(r, -127.0f), 127.0f);
-        word |= ((uint32_t)(uint8_t)(int8_t)(int)r) << (8 * e);
-      }
-      o2[h] = word;
-    }
+    uint2 o2;
+    const float scale = i8_quantize8(f[q], lanes, o2);
     if (i < nv) {
-      *reinterpret_cast<uint2*>(L.value(xq, tok, i * 8)) = make_uint2(o2[0], o2[1]);
+      *reinterpret_cast<uint2*>(L.value(xq, tok, i * 8)) = o2;
       if ((i % lanes) == 0) *L.scale(xq, tok, i / lanes) = live ? scale : 0.0f;
     }
   }
@@ -690,11 +658,13 @@ static int i8_linear(const int8_t* wq, const float* swT, const int8_t* wq2, cons
   t.err = reinterpret_cast<unsigned*>(sc + kTcCounterBytes - 4);
   if (i8_rows_serves(M, N, block_size, wq2 != nullptr)) {
     const I8Rows L((int)M, K);
-    if (!reuse_act) {
+    I8RowsParams p = {};
+    if (!reuse_act && i8_rows_quantizes(x, y, M, N, K)) {
+      p.x = x; p.gamma = gamma; p.gamma_f32 = gamma_is_f32; p.eps = eps;
+    } else if (!reuse_act) {
       int rc = i8_quantize(x, gamma, gamma_is_f32, eps, (int)M, (int)M, K, L, xq, st);
       if (rc) return rc;
     }
-    I8RowsParams p = {};
     p.t = t;
     p.w[0] = wq; p.w[1] = wq2; p.swT[0] = swT; p.swT[1] = swT2; p.xq = xq;
     p.nkb = L.nkb; p.Mp = L.Mp; p.Kp = (int)pl.Kp; p.Np = (int)pl.Np; p.tiles = (int)(N / 16);

@@ -6,8 +6,8 @@
 // and all of K; its groups of warps take the 64-wide k blocks in turn, two neighbours (128 bytes of a row) at a time. A warp's weights come by
 // cp.async into a ring of its own, each lane copying exactly the 16-byte pieces that it feeds to its MMAs: no barrier of the CTA in the loop,
 // 100 to 200 KB per SM on the way, the first of them before the wait for the previous kernel. k is permuted inside a block (a lane's MMA slots
-// are 16 consecutive values), which both operands share, so the plain row-major weight needs no repacking. Activations come straight
-// from L2 to registers, a block ahead. The tcgen05 form has a chain per 256 k values (copies, MMAs, drain of int32 accumulators from tensor memory)
+// are 16 consecutive values), which both operands share, so the plain row-major weight needs no repacking. Quantised activations come straight
+// from L2 to registers, a block ahead; one or two tokens every CTA quantises for itself. The tcgen05 form has a chain per 256 k values (copies, MMAs, drain of int32 accumulators from tensor memory)
 // on whole tiles of 128 features; here the drain is three packed fp32 operations per two sums in the registers where the MMA left them.
 // With the quantisation of x, a chain of calls on one B200, tcgen05 form / here: 11008 x 4096 (7.4 us of HBM) 1 token 16.4 / 11.8 us, 16: 16.4 / 13.6,
 // 32: 18.8 / 17.4; 4096 x 4096 10.2 / 5.7 at 1, 12.6 / 8.9 at 32; the pair 2 x 11008 x 4096 at 1 token 31.8 / 19.4 (one kernel instead of two).
@@ -33,8 +33,84 @@ __device__ __forceinline__ void ir_mma(int (&d)[4], uint32_t a0, uint32_t a1, ui
       : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(c0), "r"(c1), "r"(c2), "r"(c3));
 }
-// T: tiles of 16 features per CTA (of a pair: gate and up tiles in turn), MG: groups of 8 tokens
-template <int T, int MG, bool DUAL>
+constexpr int kIrStaged = 65536;  // quantised values, at most, of one or two tokens in shared memory behind the ring
+
+// Quantises the rows of x as quantize_act_i8_row_kernel does, behind the same norm, into shared memory: values [k block][token][64] at xs, scales [k block][token] at fs.
+// Every CTA does all of them for itself; the first leaves them in p.xq too, for a call that reuses them.
+template <int THREADS>
+__device__ __forceinline__ void ir_quantize(const I8RowsParams& p, uint32_t xs, uint32_t fs) {
+  __shared__ float part[2][THREADS / 32];
+  const int M = p.t.M, nv = p.nkb * 8, tid = threadIdx.x;  // nv: pieces of 8 values per token
+  float gm[2][8];
+  if (p.gamma) {
+#pragma unroll
+    for (int r = 0; r < 2; r++)
+      if (r * THREADS + tid < nv) i8_gamma(p.gamma, p.gamma_f32, r * THREADS + tid, gm[r]);
+  }
+  pdl_wait();
+  for (int q0 = 0; q0 < nv; q0 += 2 * THREADS) {  // with the norm (at most 8192 values) once
+    uint4 v[2][2];
+#pragma unroll
+    for (int r = 0; r < 2; r++)
+#pragma unroll
+      for (int m = 0; m < 2; m++) {
+        const int q = q0 + r * THREADS + tid;
+        v[r][m] = q < nv && m < M ? rows_ldg16(p.x + (size_t)m * nv * 8 + q * 8) : make_uint4(0, 0, 0, 0);
+      }
+    float inv[2] = {};
+    if (p.gamma) {
+#pragma unroll
+      for (int m = 0; m < 2; m++) {
+        float ss = 0.0f;
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+          float f[8];
+          i8_unpack_bf16(v[r][m], f);
+#pragma unroll
+          for (int j = 0; j < 8; j += 2) ss += f[j] * f[j] + f[j + 1] * f[j + 1];
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        if ((tid & 31) == 0) part[m][tid >> 5] = ss;
+      }
+      __syncthreads();
+#pragma unroll
+      for (int m = 0; m < 2; m++) {
+        float tot = 0.0f;
+#pragma unroll
+        for (int w = 0; w < THREADS / 32; w++) tot += part[m][w];
+        inv[m] = rsqrtf(tot / (float)(nv * 8) + p.eps);
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < 2; r++)
+#pragma unroll
+      for (int m = 0; m < 2; m++) {
+        const int q = q0 + r * THREADS + tid;
+        if (m >= M || q0 + r * THREADS >= nv) continue;
+        float f[8];
+        i8_unpack_bf16(v[r][m], f);
+        if (p.gamma && q < nv) {
+#pragma unroll
+          for (int j = 0; j < 8; j++) f[j] = bf16_bits_to_f32(f32_to_bf16_bits(f[j] * inv[m] * gm[r][j]));
+        }
+        uint2 o;
+        const float scale = i8_quantize8(f, 8, o);
+        if (q >= nv) continue;
+        const int blk = q >> 3;
+        asm volatile("st.shared.v2.u32 [%0], {%1,%2};" ::"r"(xs + (uint32_t)((blk * M + m) * 64 + (q & 7) * 8)), "r"(o.x), "r"(o.y) : "memory");
+        if ((q & 7) == 0) asm volatile("st.shared.f32 [%0], %1;" ::"r"(fs + (uint32_t)(blk * M + m) * 4), "f"(scale) : "memory");
+        if (blockIdx.x == 0) {
+          *reinterpret_cast<uint2*>(p.xq + ((size_t)blk * p.Mp + m) * 64 + (q & 7) * 8) = o;
+          if ((q & 7) == 0) reinterpret_cast<float*>(p.xq + (size_t)p.nkb * p.Mp * 64)[(size_t)blk * p.Mp + m] = scale;
+        }
+      }
+  }
+  __syncthreads();
+}
+
+// T: tiles of 16 features per CTA (of a pair: gate and up tiles in turn), MG: groups of 8 tokens, QUANT: the kernel quantises the activations itself
+template <int T, int MG, bool DUAL, bool QUANT>
 __global__ void __launch_bounds__(IrCfg<T, MG>::W * 32, 1) qlinear_i8_rows_kernel(I8RowsParams p) {
   using C = IrCfg<T, MG>;
   constexpr int KG = C::KG, N = C::N, D = C::D, S = C::S, TF = DUAL ? T / 2 : T;  // TF: feature tiles
@@ -56,10 +132,12 @@ __global__ void __launch_bounds__(IrCfg<T, MG>::W * 32, 1) qlinear_i8_rows_kerne
   const char* const sb0 = reinterpret_cast<const char*>(p.swT[0] + tile0 * 16);
   const char* const sb1 = DUAL ? reinterpret_cast<const char*>(p.swT[1] + tile0 * 16) : nullptr;
   uint32_t w0 = f0 * row16 + g * p.Kp + t * 16 + turn * 128, s0 = turn * 8 * p.Np + f0 * 64 + lane * 16;
-  const uint32_t xrow = p.Mp * 64, xstep = groups * 2 * xrow;
+  const uint32_t xrow = (QUANT ? p.t.M : p.Mp) * 64, xstep = groups * 2 * xrow;
   const uint8_t* const sxb = p.xq + (size_t)p.nkb * xrow;  // a scale is 4 bytes where its 64 values are 64
   uint32_t x0 = turn * 2 * xrow;
-  const uint32_t xl = g * 64 + t * 16;
+  const int last = p.t.M - 1;  // QUANT: columns behind the last token repeat it and are not stored
+  const uint32_t xl = (QUANT ? min(g, last) : g) * 64 + t * 16;
+  const uint32_t xs = tc_smem_u32(ir_smem_raw) + (uint32_t)C::SMEM, fs = xs + p.nkb * xrow;
   pdl_trigger();
 
   // slot q of the ring, k block `ord` of this warp's, `td` blocks behind the one that w0 and s0 point at
@@ -79,16 +157,22 @@ __global__ void __launch_bounds__(IrCfg<T, MG>::W * 32, 1) qlinear_i8_rows_kerne
   };
 #pragma unroll
   for (int q = 0; q < S - 1; q++) issue(q, q / N, q / N);
-  pdl_wait();
+  if constexpr (QUANT) ir_quantize<C::W * 32>(p, xs, fs);
+  else pdl_wait();
 
   uint4 xv[2][MG];
   float2 sv[2][MG];
   auto fetch = [&](int z, int td) {
     const uint32_t x = x0 + (td >> 1) * xstep + (td & 1) * xrow;
+    if constexpr (QUANT) {
+      xv[z][0] = rows_lds16(xs + x + xl);
+      sv[z][0] = make_float2(rows_lds4(fs + x / 16 + min(2 * t, last) * 4), rows_lds4(fs + x / 16 + min(2 * t + 1, last) * 4));
+    } else {
 #pragma unroll
-    for (int m = 0; m < MG; m++) {
-      xv[z][m] = rows_ldg16(p.xq + (x + xl + m * 512));
-      sv[z][m] = rows_ldg8(sxb + (x / 16 + t * 8 + m * 32));
+      for (int m = 0; m < MG; m++) {
+        xv[z][m] = rows_ldg16(p.xq + (x + xl + m * 512));
+        sv[z][m] = rows_ldg8(sxb + (x / 16 + t * 8 + m * 32));
+      }
     }
   };
   if (cnt > 0) fetch(0, 0);
@@ -136,18 +220,27 @@ __global__ void __launch_bounds__(IrCfg<T, MG>::W * 32, 1) qlinear_i8_rows_kerne
   rows_finish<C, DUAL>(acc, ir_smem_raw, p.t, tile0, tile_own, csize, crank);
 }
 
-template <int T, int MG, bool DUAL>
-static int ir_launch(const I8RowsParams& p, cudaStream_t st) {
-  constexpr size_t smem = IrCfg<T, MG>::SMEM;
+template <int T, int MG, bool DUAL, bool QUANT>
+static int ir_launch_as(const I8RowsParams& p, cudaStream_t st) {
+  constexpr size_t base = IrCfg<T, MG>::SMEM, most = base + (QUANT ? kIrStaged / 64 * 68 : 0);
+  static_assert(most <= 225 * 1024, "shared memory");
   static bool opted[16] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 16 || !opted[dev]) {
-    TPX_CUDA_OK(cudaFuncSetAttribute(qlinear_i8_rows_kernel<T, MG, DUAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    TPX_CUDA_OK(cudaFuncSetAttribute(qlinear_i8_rows_kernel<T, MG, DUAL, QUANT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
     if (dev >= 0 && dev < 16) opted[dev] = true;
   }
   constexpr int TF = DUAL ? T / 2 : T;
-  return rows_launch(qlinear_i8_rows_kernel<T, MG, DUAL>, (p.tiles + TF - 1) / TF, p.t.cluster, IrCfg<T, MG>::W * 32, smem, st, p);
+  return rows_launch(qlinear_i8_rows_kernel<T, MG, DUAL, QUANT>, (p.tiles + TF - 1) / TF, p.t.cluster, IrCfg<T, MG>::W * 32,
+                     base + (QUANT ? (size_t)p.nkb * p.t.M * 68 : 0), st, p);
+}
+template <int T, int MG, bool DUAL>
+static int ir_launch(const I8RowsParams& p, cudaStream_t st) {
+  if constexpr (MG == 1) {
+    if (p.x) return ir_launch_as<T, 1, DUAL, true>(p, st);
+  }
+  return ir_launch_as<T, MG, DUAL, false>(p, st);
 }
 
 template <int MG>
@@ -180,6 +273,13 @@ static int ir_launch_t(const I8RowsParams& p, bool pair, int tf, cudaStream_t st
 // tokens: 14336 x 4096 at 32 tokens 21.0 us here, 19.7 on the tcgen05 kernel; six tiles (12288 x 4096) 18.7 / 19.3, one (2048 x 8192) 10.1 / 14.0.
 bool i8_rows_serves(int64_t M, int64_t N, int64_t block, bool pair) {
   return block == 64 && (M <= 16 || (M <= 32 && !pair && rows_tiles(N / 16) < 7));
+}
+
+// One and two tokens: in every CTA, which costs less than the launch in front. Generation of 40 tokens behind 64, 8 layers of 4096 x 11008: 1 token 24.0 ms, from
+// 26.6 with a kernel in front; 2 tokens 26.5 (26.7 with only the norms in here, 28.1 with none). Calls in a chain at 1 token, without a norm: 11008 x 4096 11.9 -> 10.6 us, 4096 x
+// 11008 11.9 -> 11.5, 4096 x 4096 5.7 -> 5.9; at 2 tokens 11.8 -> 11.2, 12.1 -> 12.8, 5.7 -> 6.3. A norm in front is a kernel of 5 us, in here of about one.
+bool i8_rows_quantizes(const void* x, const void* y, int64_t M, int64_t N, int64_t K) {
+  return M <= 2 && M * K <= kIrStaged && rows_shared_x(x, (size_t)M * K * 2, y, (size_t)M * N * 2);
 }
 
 int i8_rows_launch(I8RowsParams p, bool pair, cudaStream_t st) {

@@ -16,15 +16,61 @@ struct I8Rows {
   }
 };
 
+// Eight values of a quantisation block that as many neighbouring lanes have as `lanes` says -> eight int8; returns the block's scale.
+__device__ __forceinline__ float i8_quantize8(const float (&f)[8], int lanes, uint2& out) {
+  float amax = 0.0f;
+#pragma unroll
+  for (int j = 0; j < 8; j++) amax = fmaxf(amax, fabsf(f[j]));
+  for (int o = 1; o < lanes; o <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+  const float scale = (float)((double)amax / 127.0);
+  const float iscale = scale != 0.0f ? 1.0f / scale : 0.0f;
+  uint32_t o2[2];
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    uint32_t word = 0;
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+      float r = nearbyintf(f[4 * h + e] * iscale);
+      r = fminf(fmaxf(r, -127.0f), 127.0f);
+      word |= ((uint32_t)(uint8_t)(int8_t)(int)r) << (8 * e);
+    }
+    o2[h] = word;
+  }
+  out = make_uint2(o2[0], o2[1]);
+  return scale;
+}
+__device__ __forceinline__ void i8_unpack_bf16(uint4 v, float (&f)[8]) {
+  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+  for (int j = 0; j < 4; j++) {
+    f[2 * j] = bf16_bits_to_f32((uint16_t)(w[j] & 0xffff));
+    f[2 * j + 1] = bf16_bits_to_f32((uint16_t)(w[j] >> 16));
+  }
+}
+// piece i of the norm's weight
+__device__ __forceinline__ void i8_gamma(const void* gamma, int gamma_f32, int i, float (&g)[8]) {
+  if (gamma_f32) {
+    const float4 g0 = reinterpret_cast<const float4*>(gamma)[2 * i], g1 = reinterpret_cast<const float4*>(gamma)[2 * i + 1];
+    g[0] = g0.x; g[1] = g0.y; g[2] = g0.z; g[3] = g0.w; g[4] = g1.x; g[5] = g1.y; g[6] = g1.z; g[7] = g1.w;
+  } else {
+    i8_unpack_bf16(reinterpret_cast<const uint4*>(gamma)[i], g);
+  }
+}
+
 struct I8RowsParams {
   TcParams t;                // epilogue fields (bias, act, mul_in, res, res_scale, y, M, N)
   const int8_t* w[2];        // plain int8 weight [Np][Kp]; of a pair: gate, up
   const float* swT[2];       // [K/64][Np]
-  const uint8_t* xq;         // I8Rows
+  uint8_t* xq;               // I8Rows
+  const uint16_t* x;         // or, if not null: bf16 activations, to be quantised (behind an RMSNorm if gamma is set) and left in xq as well
+  const void* gamma;
+  int gamma_f32;
+  float eps;
   int nkb, Mp, Kp, Np, tiles;  // tiles: N / 16
 };
 
 bool i8_rows_serves(int64_t M, int64_t N, int64_t block, bool pair);
+bool i8_rows_quantizes(const void* x, const void* y, int64_t M, int64_t N, int64_t K);  // whether the launch takes x instead of xq
 int i8_rows_launch(I8RowsParams p, bool pair, cudaStream_t st);  // sets t.cluster
 
 }  // namespace tpx
