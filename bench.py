@@ -800,7 +800,7 @@ def run_ours(args):
                         # 512 tokens run kind::mxf8f6f4 MMAs on the packed weight (twice the bf16 rate), 4096 kind::f16 on the unpacked one
                         "peak_src": pk["src"], "clocks": pre_clocks, "rounds": pre_rounds},
             "roofline": {"bound": "hbm",
-                         "kernel": f"MXFP4 gate/up pair GEMM, M={SWEEP[dom]} (tcgen05: qlinear_tc_kernel for M <= 16, "
+                         "kernel": f"MXFP4 gate/up pair GEMM, M={SWEEP[dom]} (qlinear_mx_rows_kernel, fp16 mma.sync, for M <= 8; tcgen05: qlinear_tc_kernel for M <= 16, "
                                    f"qlinear_tcw_kernel for M <= 64, both kind::mxf8f6f4; cta_group::2 kernels beyond)"
                                    if F.mxfp4_path() == "tc" else f"qlinear_stream gate/up pair, M={SWEEP[dom]}",
                          "achieved": dom_gbs, "peak": pk["hbm_gbs"], "unit": "GB/s", "frac": dom_gbs / pk["hbm_gbs"],

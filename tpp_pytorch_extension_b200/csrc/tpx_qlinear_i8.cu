@@ -9,7 +9,7 @@
 //                            one int32 accumulator per K block in tensor memory (a ring of them); the four epilogue
 //                            warps pull each finished block, scale it and add it to fp32 registers
 // Difference to the reference, inside the parity tolerance: the running output is kept in fp32, where the reference
-// rounds it to bf16 after every K block.
+// rounds it to bf16 after every K block. Blocks of 64 and few tokens: tpx_qlinear_i8_rows.cu, the same arithmetic.
 //
 // Work split: one output tile (128 features x TOK tokens, TOK = 16, 32, 64 or, for more than 64 tokens, 128) per CTA;
 // when tiles are few, a thread-block cluster per tile cuts K between its CTAs, which add their parts over distributed

@@ -276,7 +276,7 @@ bool i8_rows_serves(int64_t M, int64_t N, int64_t block, bool pair) {
 }
 
 // One and two tokens: in every CTA, which costs less than the launch in front. Generation of 40 tokens behind 64, 8 layers of 4096 x 11008: 1 token 24.0 ms, from
-// 26.6 with a kernel in front; 2 tokens 26.5 (26.7 with only the norms in here, 28.1 with none). Calls in a chain at 1 token, without a norm: 11008 x 4096 11.9 -> 10.6 us, 4096 x
+// 26.2 with a kernel in front; 2 tokens 26.5 (26.7 with only the norms in here, 27.9 with none). Calls in a chain at 1 token, without a norm: 11008 x 4096 11.9 -> 10.6 us, 4096 x
 // 11008 11.9 -> 11.5, 4096 x 4096 5.7 -> 5.9; at 2 tokens 11.8 -> 11.2, 12.1 -> 12.8, 5.7 -> 6.3. A norm in front is a kernel of 5 us, in here of about one.
 bool i8_rows_quantizes(const void* x, const void* y, int64_t M, int64_t N, int64_t K) {
   return M <= 2 && M * K <= kIrStaged && rows_shared_x(x, (size_t)M * K * 2, y, (size_t)M * N * 2);

@@ -1010,7 +1010,8 @@ extern "C" int tpx_repack_mxfp4_tc(const uint8_t* codes, const uint8_t* scales, 
   return TPX_OK;
 }
 
-// Kernel choice for up to 64 tokens. The kernel with the weights on the wide (N) side of the MMA spends fewer
+// Kernel choice for up to 64 tokens, of what mx_rows_serves does not take (no switch set, MXFP4: all up to 8 tokens and small calls up to 16; figures of
+// fewer tokens below hold between these two kernels). The kernel with the weights on the wide (N) side of the MMA spends fewer
 // tensor-pipe cycles per weight byte (one 128x256x32 MMA per 4 KiB instead of two 128x32x32 per 2 KiB each); the rule
 // below follows a sweep of both kernels over the linear shapes of Llama-3-8B, Llama-2-7B and Llama-2-70B (2 and 8
 // tensor-parallel ranks) at 1 to 64 tokens, launches back to back. TPX_TC_WIDE=1 forces the wide kernel for every
