@@ -8,10 +8,15 @@
 //   s <- s0 + K^T v - A^T q
 // and with W and Y solving (I + N) [W, Y] = [c u, M]:
 //   q = W s0 + Y v,   o = (R - G2 W) s0 + (G1 - G2 Y) v.
-// Only s0 ties a chunk to the one before: eight warps prepare the next chunk's W, R - G2 W, Y, G1 - G2 Y, K, A while four apply the present one's, each to 16
-// value channels, whose state they hold as mma accumulators (transposed, so that an accumulator is the next product's left operand as it lies).
+// Only s0 ties a chunk to the one before: two groups of eight warps, a chunk each, prepare the next chunks' W, R - G2 W, Y, G1 - G2 Y, K, A while four warps apply
+// the present one's, each to 16 value channels, whose state they hold as mma accumulators (transposed, so that an accumulator is the next product's left operand
+// as it lies).
 //
-// 32-bit throughout: mma.sync in TF32 with both operands as a rounded value and the rounded remainder, three products each (two where the operand is v, whose
+// The matrix products hold that form only for numbers: a token's infinity or NaN would reach the tokens before it through the zeros of the triangles, and the split
+// below loses both. A chunk with one, or with a value so large that a product of two overflows, goes token by token (dc_token_loop), and so does one that finds
+// such a state, for the value channels of that warp.
+//
+// State and sums are 32-bit: mma.sync in TF32 with both operands as a rounded value and the rounded remainder, three products each (two where the operand is v, whose
 // bf16 values are TF32 values). Decays and rates take the library's exponential and division: with the fast ones the state was 1.25e-7 off 64 bits, so 1.02e-7 (the
 // token loop 1.03e-7 to 1.08e-7); o's rounding to bf16 hides either.
 // Bound by the instructions of the preparation (11000 of a chunk's 14700; splits, fragment loads, the triangular solve): issue slots 56 % busy, tensor pipe 31 %, the
@@ -25,13 +30,15 @@ constexpr int kDcTok = 16, kDcMain = 4, kDcPrep = 8, kDcThreads = 32 * (kDcMain 
 constexpr int kDcMeet = 32 * (kDcMain + kDcPrep);  // threads that hand a buffer over
 // floats: row strides are chosen so that the fragment loads meet no bank twice
 constexpr int kDcY = 72, kDcH = 24, kDcK = 68, kDcN = 20;
-struct DcBuf {  // what the four warps need of a chunk; h: rounded to TF32, l: the remainder
+struct __align__(16) DcBuf {  // what the four warps need of a chunk; h: rounded to TF32, l: the remainder
   float yh[32 * kDcY], yl[32 * kDcY];  // rows 0-15 W, 16-31 R - G2 W
   float hh[32 * kDcH], hl[32 * kDcH];  // rows 0-15 Y, 16-31 G1 - G2 Y
   float kh[kDcTok * kDcK], kl[kDcTok * kDcK], ah[kDcTok * kDcK], al[kDcTok * kDcK];
   float v[kDcTok * kDcK], gate[kDcTok * 64], g[64];
+  float u[kDcTok * 64], r[kDcTok * 64], c[kDcTok];  // for the token loop, with K = kh + kl and A = ah + al
+  int loop;  // the chunk is not for matrix products; yh to hl are not set
 };
-struct DcPrep {  // of the eight warps that prepare every other chunk
+struct __align__(16) DcPrep {  // of the eight warps that prepare every other chunk
   float w[kDcTok * kDcY], u[kDcTok * kDcY], k[kDcTok * kDcY], a[kDcTok * kDcY], r[kDcTok * kDcY];
   float n[kDcTok * kDcN], m[kDcTok * kDcN], g1[kDcTok * kDcN], g2[kDcTok * kDcN];
   float v[kDcTok * 64], gate[kDcTok * 64], g[64], c[kDcTok];
@@ -43,6 +50,9 @@ struct DcSmem {
   DcPrep prep[2];
   float o[2][kDcTok * kDcK];
 };
+static_assert(offsetof(DcSmem, buf[1]) % 16 == 0 && offsetof(DcSmem, prep) % 16 == 0 && offsetof(DcSmem, prep[1]) % 16 == 0 && offsetof(DcBuf, u) % 16 == 0 &&
+                  offsetof(DcPrep, raw) % 16 == 0 && sizeof(DcSmem) <= 227 * 1024,
+              "vectors of 16 bytes");
 
 __device__ __forceinline__ float dc_hi(float x) { return __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xffffe000u); }
 __device__ __forceinline__ void dc_split(float x, float& h, float& l) {
@@ -55,9 +65,68 @@ __device__ __forceinline__ void dc_mma(float (&d)[4], const float (&a)[4], float
       : "r"(__float_as_uint(a[0])), "r"(__float_as_uint(a[1])), "r"(__float_as_uint(a[2])), "r"(__float_as_uint(a[3])), "r"(__float_as_uint(b0)),
         "r"(__float_as_uint(b1)));
 }
+// The larger magnitude, a NaN before all; the sign is of no use. Below the bounds a chunk's products are all finite, and so is the split.
+constexpr float kDcBig = 1125899906842624.0f, kDcBigState = 1.2676506002282294e30f;  // 2^50, 2^100
+__device__ __forceinline__ void dc_larger(float& m, float x) { asm("max.NaN.xorsign.abs.f32 %0, %0, %1;" : "+f"(m) : "f"(x)); }
 __device__ __forceinline__ void dc_bar_sync(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
 __device__ __forceinline__ void dc_bar_arrive(int id, int n) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(n) : "memory"); }
+__device__ __forceinline__ bool dc_bar_any(int id, int n, bool mine) {
+  int any;
+  asm volatile("{ .reg .pred p, q; setp.ne.s32 p, %3, 0; bar.red.or.pred q, %1, %2, p; selp.s32 %0, 1, 0, q; }"
+               : "=r"(any)
+               : "r"(id), "r"(n), "r"((int)mine)
+               : "memory");
+  return any != 0;
+}
 // barriers: 1 and 7 the preparing warps, 2 the applying ones, 3 and 4 a buffer is ready, 5 and 6 it is free
+
+// A chunk token by token, in the order and with the formulas of delta_fast_kernel: value channels e0 ... + 15, the warp's state as it lies in s; o to sh.o.
+__device__ __forceinline__ void dc_token_loop(float (&s)[8][4], const DcBuf& B, float* o, int e0) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+#pragma unroll 1
+  for (int tok = 0; tok < kDcTok; tok++) {
+    float2 k[8], a[8];
+    float x[6] = {0, 0, 0, 0, 0, 0};  // u . s of both value channels, R . s, then r . k and r . a k
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+      const int at = 8 * j + 2 * t;
+      const float2 u = *reinterpret_cast<const float2*>(B.u + tok * 64 + at), r = *reinterpret_cast<const float2*>(B.r + tok * 64 + at);
+      const float2 kh = *reinterpret_cast<const float2*>(B.kh + tok * kDcK + at), kl = *reinterpret_cast<const float2*>(B.kl + tok * kDcK + at);
+      const float2 ah = *reinterpret_cast<const float2*>(B.ah + tok * kDcK + at), al = *reinterpret_cast<const float2*>(B.al + tok * kDcK + at);
+      k[j] = make_float2(kh.x + kl.x, kh.y + kl.y);
+      a[j] = make_float2(ah.x + al.x, ah.y + al.y);
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        x[e] = fmaf(u.y, s[j][2 * e + 1], fmaf(u.x, s[j][2 * e], x[e]));
+        x[2 + e] = fmaf(r.y, s[j][2 * e + 1], fmaf(r.x, s[j][2 * e], x[2 + e]));
+      }
+      x[4] = fmaf(r.y, k[j].y, fmaf(r.x, k[j].x, x[4]));
+      x[5] = fmaf(r.y, a[j].y, fmaf(r.x, a[j].x, x[5]));
+    }
+#pragma unroll
+    for (int i = 0; i < 6; i++) {
+      x[i] += __shfl_xor_sync(0xffffffffu, x[i], 1);
+      x[i] += __shfl_xor_sync(0xffffffffu, x[i], 2);
+    }
+#pragma unroll
+    for (int e = 0; e < 2; e++) {
+      const float q = -B.c[tok] * x[e], v = B.v[tok * kDcK + e0 + g + 8 * e];
+      // times zero: as there, where all but one of a column's lanes add the last two terms so
+      if (t == 0) o[tok * kDcK + e0 + g + 8 * e] = fmaf(x[4], v, fmaf(x[5], q, x[2 + e])) + fmaf(0.0f, v, 0.0f * q);
+#pragma unroll
+      for (int j = 0; j < 8; j++) {
+        s[j][2 * e] = fmaf(a[j].x, q, fmaf(k[j].x, v, s[j][2 * e]));
+        s[j][2 * e + 1] = fmaf(a[j].y, q, fmaf(k[j].y, v, s[j][2 * e + 1]));
+      }
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 8; j++) {
+    const float2 g2 = *reinterpret_cast<const float2*>(B.g + 8 * j + 2 * t);
+#pragma unroll
+    for (int i = 0; i < 4; i++) s[j][i] *= (i & 1) ? g2.y : g2.x;
+  }
+}
 
 __global__ void __launch_bounds__(kDcThreads, 1) delta_chunk_kernel(DeltaFastParams p) {
   extern __shared__ __align__(16) unsigned char dc_smem[];
@@ -82,102 +151,111 @@ __global__ void __launch_bounds__(kDcThreads, 1) delta_chunk_kernel(DeltaFastPar
     for (int c = 0; c < chunks; c++) {
       DcBuf& B = sh.buf[c & 1];
       dc_bar_sync(3 + (c & 1), kDcMeet);
-      // [q of tokens 0-7, 8-15, o of tokens 0-7, 8-15], transposed; small: the products with remainders, summed for themselves, and the others in
-      // two sums: an MMA's addition is cut off, not rounded. Products that go to the same sum are four apart: an MMA waits for its accumulator.
-      float x[4][4], y[4][4], small[4][4];
-#pragma unroll
-      for (int n = 0; n < 4; n++)
-#pragma unroll
-        for (int i = 0; i < 4; i++) x[n][i] = y[n][i] = small[n][i] = 0.0f;
-#pragma unroll
-      for (int j = 0; j < 8; j++) {
-        float h[4], l[4];  // as the left operand: slots t and t + 4 of k are channels 2 t and 2 t + 1
-        dc_split(s[j][0], h[0], l[0]);
-        dc_split(s[j][2], h[1], l[1]);
-        dc_split(s[j][1], h[2], l[2]);
-        dc_split(s[j][3], h[3], l[3]);
-        float2 yh[4], yl[4];
-#pragma unroll
-        for (int n = 0; n < 4; n++) {
-          yh[n] = *reinterpret_cast<const float2*>(B.yh + (8 * n + g) * kDcY + 8 * j + 2 * t);
-          yl[n] = *reinterpret_cast<const float2*>(B.yl + (8 * n + g) * kDcY + 8 * j + 2 * t);
-        }
-#pragma unroll
-        for (int n = 0; n < 4; n++) dc_mma(small[n], l, yh[n].x, yh[n].y);
-#pragma unroll
-        for (int n = 0; n < 4; n++) dc_mma((j & 1) ? y[n] : x[n], h, yh[n].x, yh[n].y);
-#pragma unroll
-        for (int n = 0; n < 4; n++) dc_mma(small[n], h, yl[n].x, yl[n].y);
-      }
-      float v[2][4];
-#pragma unroll
-      for (int i = 0; i < 2; i++)
-#pragma unroll
-        for (int e = 0; e < 4; e++) v[i][e] = B.v[(8 * i + 2 * t + (e >> 1)) * kDcK + e0 + g + (e & 1) * 8];
-#pragma unroll
-      for (int i = 0; i < 2; i++) {
-        float2 hh[4], hl[4];
-#pragma unroll
-        for (int n = 0; n < 4; n++) {
-          hh[n] = *reinterpret_cast<const float2*>(B.hh + (8 * n + g) * kDcH + 8 * i + 2 * t);
-          hl[n] = *reinterpret_cast<const float2*>(B.hl + (8 * n + g) * kDcH + 8 * i + 2 * t);
-        }
-#pragma unroll
-        for (int n = 0; n < 4; n++) dc_mma(small[n], v[i], hl[n].x, hl[n].y);
-#pragma unroll
-        for (int n = 0; n < 4; n++) dc_mma(x[n], v[i], hh[n].x, hh[n].y);
-      }
-#pragma unroll
-      for (int n = 0; n < 4; n++)
-#pragma unroll
-        for (int i = 0; i < 4; i++) x[n][i] += y[n][i] + small[n][i];
       float* o = sh.o[c & 1];
+      float most = 0.0f;
 #pragma unroll
-      for (int n = 0; n < 2; n++)
+      for (int j = 0; j < 8; j++)
 #pragma unroll
-        for (int i = 0; i < 4; i++) o[(8 * n + 2 * t + (i & 1)) * kDcK + e0 + g + (i >> 1) * 8] = x[2 + n][i];
-      float zh[2][4], zl[2][4];
+        for (int i = 0; i < 4; i++) dc_larger(most, s[j][i]);
+      if (B.loop || __any_sync(0xffffffffu, !(fabsf(most) < kDcBigState))) {
+        dc_token_loop(s, B, o, e0);
+      } else {
+        // [q of tokens 0-7, 8-15, o of tokens 0-7, 8-15], transposed; small: the products with remainders, summed for themselves, and the others in
+        // two sums: an MMA's addition is cut off, not rounded. Products that go to the same sum are four apart: an MMA waits for its accumulator.
+        float x[4][4], y[4][4], small[4][4];
 #pragma unroll
-      for (int i = 0; i < 2; i++) {
-        dc_split(-x[i][0], zh[i][0], zl[i][0]);
-        dc_split(-x[i][2], zh[i][1], zl[i][1]);
-        dc_split(-x[i][1], zh[i][2], zl[i][2]);
-        dc_split(-x[i][3], zh[i][3], zl[i][3]);
-      }
+        for (int n = 0; n < 4; n++)
 #pragma unroll
-      for (int j0 = 0; j0 < 8; j0 += 4) {  // what the chunk adds, four groups of channels at a time; the state is added outside
-        float d[4][4], dv[4][4], dz[4][4];
+          for (int i = 0; i < 4; i++) x[n][i] = y[n][i] = small[n][i] = 0.0f;
 #pragma unroll
-        for (int j = 0; j < 4; j++)
+        for (int j = 0; j < 8; j++) {
+          float h[4], l[4];  // as the left operand: slots t and t + 4 of k are channels 2 t and 2 t + 1
+          dc_split(s[j][0], h[0], l[0]);
+          dc_split(s[j][2], h[1], l[1]);
+          dc_split(s[j][1], h[2], l[2]);
+          dc_split(s[j][3], h[3], l[3]);
+          float2 yh[4], yl[4];
 #pragma unroll
-          for (int e = 0; e < 4; e++) d[j][e] = dv[j][e] = dz[j][e] = 0.0f;
+          for (int n = 0; n < 4; n++) {
+            yh[n] = *reinterpret_cast<const float2*>(B.yh + (8 * n + g) * kDcY + 8 * j + 2 * t);
+            yl[n] = *reinterpret_cast<const float2*>(B.yl + (8 * n + g) * kDcY + 8 * j + 2 * t);
+          }
+#pragma unroll
+          for (int n = 0; n < 4; n++) dc_mma(small[n], l, yh[n].x, yh[n].y);
+#pragma unroll
+          for (int n = 0; n < 4; n++) dc_mma((j & 1) ? y[n] : x[n], h, yh[n].x, yh[n].y);
+#pragma unroll
+          for (int n = 0; n < 4; n++) dc_mma(small[n], h, yl[n].x, yl[n].y);
+        }
+        float v[2][4];
+#pragma unroll
+        for (int i = 0; i < 2; i++)
+#pragma unroll
+          for (int e = 0; e < 4; e++) v[i][e] = B.v[(8 * i + 2 * t + (e >> 1)) * kDcK + e0 + g + (e & 1) * 8];
 #pragma unroll
         for (int i = 0; i < 2; i++) {
-          float kh[4][2], kl[4][2], ah[4][2], al[4][2];
+          float2 hh[4], hl[4];
+#pragma unroll
+          for (int n = 0; n < 4; n++) {
+            hh[n] = *reinterpret_cast<const float2*>(B.hh + (8 * n + g) * kDcH + 8 * i + 2 * t);
+            hl[n] = *reinterpret_cast<const float2*>(B.hl + (8 * n + g) * kDcH + 8 * i + 2 * t);
+          }
+#pragma unroll
+          for (int n = 0; n < 4; n++) dc_mma(small[n], v[i], hl[n].x, hl[n].y);
+#pragma unroll
+          for (int n = 0; n < 4; n++) dc_mma(x[n], v[i], hh[n].x, hh[n].y);
+        }
+#pragma unroll
+        for (int n = 0; n < 4; n++)
+#pragma unroll
+          for (int i = 0; i < 4; i++) x[n][i] += y[n][i] + small[n][i];
+#pragma unroll
+        for (int n = 0; n < 2; n++)
+#pragma unroll
+          for (int i = 0; i < 4; i++) o[(8 * n + 2 * t + (i & 1)) * kDcK + e0 + g + (i >> 1) * 8] = x[2 + n][i];
+        float zh[2][4], zl[2][4];
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+          dc_split(-x[i][0], zh[i][0], zl[i][0]);
+          dc_split(-x[i][2], zh[i][1], zl[i][1]);
+          dc_split(-x[i][1], zh[i][2], zl[i][2]);
+          dc_split(-x[i][3], zh[i][3], zl[i][3]);
+        }
+#pragma unroll
+        for (int j0 = 0; j0 < 8; j0 += 4) {  // what the chunk adds, four groups of channels at a time; the state is added outside
+          float d[4][4], dv[4][4], dz[4][4];
 #pragma unroll
           for (int j = 0; j < 4; j++)
 #pragma unroll
-            for (int e = 0; e < 2; e++) {
-              const int at = (8 * i + 2 * t + e) * kDcK + 8 * (j0 + j) + g;
-              kh[j][e] = B.kh[at]; kl[j][e] = B.kl[at]; ah[j][e] = B.ah[at]; al[j][e] = B.al[at];
-            }
+            for (int e = 0; e < 4; e++) d[j][e] = dv[j][e] = dz[j][e] = 0.0f;
 #pragma unroll
-          for (int j = 0; j < 4; j++) dc_mma(d[j], v[i], kl[j][0], kl[j][1]);
+          for (int i = 0; i < 2; i++) {
+            float kh[4][2], kl[4][2], ah[4][2], al[4][2];
 #pragma unroll
-          for (int j = 0; j < 4; j++) dc_mma(d[j], zl[i], ah[j][0], ah[j][1]);
+            for (int j = 0; j < 4; j++)
 #pragma unroll
-          for (int j = 0; j < 4; j++) dc_mma(d[j], zh[i], al[j][0], al[j][1]);
+              for (int e = 0; e < 2; e++) {
+                const int at = (8 * i + 2 * t + e) * kDcK + 8 * (j0 + j) + g;
+                kh[j][e] = B.kh[at]; kl[j][e] = B.kl[at]; ah[j][e] = B.ah[at]; al[j][e] = B.al[at];
+              }
 #pragma unroll
-          for (int j = 0; j < 4; j++) dc_mma(dv[j], v[i], kh[j][0], kh[j][1]);
+            for (int j = 0; j < 4; j++) dc_mma(d[j], v[i], kl[j][0], kl[j][1]);
 #pragma unroll
-          for (int j = 0; j < 4; j++) dc_mma(dz[j], zh[i], ah[j][0], ah[j][1]);
-        }
+            for (int j = 0; j < 4; j++) dc_mma(d[j], zl[i], ah[j][0], ah[j][1]);
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-          const float2 gg = *reinterpret_cast<const float2*>(B.g + 8 * (j0 + j) + 2 * t);
-          float(&z)[4] = s[j0 + j];
-          #pragma unroll
-          for (int e = 0; e < 4; e++) z[e] = (z[e] + (dv[j][e] + (dz[j][e] + d[j][e]))) * ((e & 1) ? gg.y : gg.x);
+            for (int j = 0; j < 4; j++) dc_mma(d[j], zh[i], al[j][0], al[j][1]);
+#pragma unroll
+            for (int j = 0; j < 4; j++) dc_mma(dv[j], v[i], kh[j][0], kh[j][1]);
+#pragma unroll
+            for (int j = 0; j < 4; j++) dc_mma(dz[j], zh[i], ah[j][0], ah[j][1]);
+          }
+#pragma unroll
+          for (int j = 0; j < 4; j++) {
+            const float2 gg = *reinterpret_cast<const float2*>(B.g + 8 * (j0 + j) + 2 * t);
+            float(&z)[4] = s[j0 + j];
+#pragma unroll
+            for (int e = 0; e < 4; e++) z[e] = (z[e] + (dv[j][e] + (dz[j][e] + d[j][e]))) * ((e & 1) ? gg.y : gg.x);
+          }
         }
       }
       dc_bar_sync(2, 32 * kDcMain);  // o is whole; the buffer of the chunk after next is written behind the next one's barrier
@@ -225,6 +303,7 @@ __global__ void __launch_bounds__(kDcThreads, 1) delta_chunk_kernel(DeltaFastPar
     dc_bar_sync(bar, 32 * kDcPrep);
     // decays, rates, c, values and gates: a warp per token, two channels per lane; tokens behind the last leave the state as it is
     const uint16_t* raw = sm.raw;
+    float most = 0.0f;  // of this thread's values of the chunk
 #pragma unroll
     for (int q = 0; q < kDcTok / kDcPrep; q++) {
       const int tok = pw + q * kDcPrep;
@@ -237,6 +316,8 @@ __global__ void __launch_bounds__(kDcThreads, 1) delta_chunk_kernel(DeltaFastPar
         w = make_float2(expf(-0.60653065971263342f * hy_sigmoid(ws.x)), expf(-0.60653065971263342f * hy_sigmoid(ws.y)));
         gt = make_float2(nw.x * dl_sigmoid(gs.x), nw.y * dl_sigmoid(gs.y));
       }
+      dc_larger(most, v.x);
+      dc_larger(most, v.y);
       const float k2 = hy_warp_sum(k.x * k.x + k.y * k.y);
       if (lane == 0) sm.c[tok] = 1.0f / (k2 + 1e-6f);
       *reinterpret_cast<float2*>(sm.w + tok * kDcY + 2 * lane) = w;
@@ -263,16 +344,19 @@ __global__ void __launch_bounds__(kDcThreads, 1) delta_chunk_kernel(DeltaFastPar
         const float k = sm.k[at], a = sm.a[at];
         sm.u[at] = G * k;
         G *= sm.w[at];
-        const float gi = 1.0f / G;
-        sm.k[at] = k * gi;
-        sm.a[at] = a * gi;
-        sm.r[at] *= G;
+        const float gi = 1.0f / G, ki = k * gi, ai = a * gi, r = sm.r[at] * G;
+        sm.k[at] = ki;
+        sm.a[at] = ai;
+        sm.r[at] = r;
+        dc_larger(most, ki);  // G k is no larger
+        dc_larger(most, ai);
+        dc_larger(most, r);
       }
       if (q0 == 12) sm.g[ch] = G;
     }
-    dc_bar_sync(bar, 32 * kDcPrep);
-    // [u; R] [K; A]^T: a tile of 16 x 8 per warp
-    {
+    const bool loop = dc_bar_any(bar, 32 * kDcPrep, !(fabsf(most) < kDcBig));
+    // [u; R] [K; A]^T: a tile of 16 x 8 per warp.
+    if (!loop) {
       const float* left = (pw & 1) ? sm.r : sm.u;
       const float* right = ((pw >> 1) & 2) ? sm.a : sm.k;
       const int col0 = ((pw >> 1) & 1) * 8;
@@ -300,9 +384,9 @@ __global__ void __launch_bounds__(kDcThreads, 1) delta_chunk_kernel(DeltaFastPar
         to[row * kDcN + col] = in ? (x[i] + (x1[i] + x2[i])) * ((pw & 1) ? 1.0f : sm.c[row]) : 0.0f;
       }
     }
-    dc_bar_sync(bar, 32 * kDcPrep);
+    if (!loop) dc_bar_sync(bar, 32 * kDcPrep);
     // W (in place of w) and Y (of M): a column per thread
-    if (pt < 80) {
+    if (!loop && pt < 80) {
       const bool isy = pt >= 64;
       const int col = isy ? pt - 64 : pt;
       float y[kDcTok];
@@ -332,18 +416,28 @@ __global__ void __launch_bounds__(kDcThreads, 1) delta_chunk_kernel(DeltaFastPar
 #pragma unroll
     for (int q = 0; q < 4; q++) {
       const int tok = q * 4 + (pt >> 6), ch = pt & 63;
-      dc_split(sm.k[tok * kDcY + ch], B.kh[tok * kDcK + ch], B.kl[tok * kDcK + ch]);
-      dc_split(sm.a[tok * kDcY + ch], B.ah[tok * kDcK + ch], B.al[tok * kDcK + ch]);
+      const float k = sm.k[tok * kDcY + ch], a = sm.a[tok * kDcY + ch];
+      float kh, kl, ah, al;
+      dc_split(k, kh, kl);
+      dc_split(a, ah, al);
+      B.kh[tok * kDcK + ch] = loop ? k : kh;
+      B.kl[tok * kDcK + ch] = loop ? 0.0f : kl;
+      B.ah[tok * kDcK + ch] = loop ? a : ah;
+      B.al[tok * kDcK + ch] = loop ? 0.0f : al;
+      B.u[tok * 64 + ch] = sm.u[tok * kDcY + ch];
+      B.r[tok * 64 + ch] = sm.r[tok * kDcY + ch];
       dc_split(sm.w[tok * kDcY + ch], B.yh[tok * kDcY + ch], B.yl[tok * kDcY + ch]);
       B.v[tok * kDcK + ch] = sm.v[tok * 64 + ch];
       B.gate[tok * 64 + ch] = sm.gate[tok * 64 + ch];
     }
     dc_split(sm.m[(pt >> 4) * kDcN + (pt & 15)], B.hh[(pt >> 4) * kDcH + (pt & 15)], B.hl[(pt >> 4) * kDcH + (pt & 15)]);
     if (pt < 64) B.g[pt] = sm.g[pt];
+    if (pt < kDcTok) B.c[pt] = sm.c[pt];
+    if (pt == 0) B.loop = loop;
     // what o takes: [R, G1] - G2 [W, Y], eight columns per warp (warps 0 and 1: and eight of the second)
 #pragma unroll
     for (int part = 0; part < 2; part++) {
-      if (part == 1 && pw >= 2) break;
+      if (loop || (part == 1 && pw >= 2)) break;
       const float *left = sm.g2, *right = part ? sm.m : sm.w, *base = part ? sm.g1 : sm.r;
       const int ld = part ? kDcN : kDcY, col0 = 8 * pw;
       float x[4] = {0, 0, 0, 0}, x1[4] = {0, 0, 0, 0}, x2[4] = {0, 0, 0, 0};
