@@ -81,6 +81,21 @@ def _inputs(B, S, H, seed, decay=0.0, rank=D):
     return proj.to(torch.bfloat16), rnd(B, S, H * D) * 2 + decay, rnd(H * D), 1 + 0.1 * rnd(H * D), rnd(B, H, D, D)
 
 
+# The loop's sums are rounded, those of the matrix products cut off, whose errors have one sign where the terms have: with keys of all directions the state is no
+# further off than the loop's (with slow decays nearer), with keys of a few directions and fast decays up to `times` as far.
+@pytest.mark.parametrize("S,H,decay,rank,times", [(130, 4, 0.0, D, 1.0), (513, 16, 0.0, D, 1.0), (513, 16, -3.0, D, 0.75), (130, 4, -12.0, D, 0.75), (130, 4, 12.0, D, 1.05),
+                                                  (513, 16, -3.0, 4, 1.0), (513, 16, 0.0, 4, 1.2), (1030, 16, 0.0, 1, 1.5), (130, 4, 12.0, 1, 1.5), (130, 4, -12.0, 1, 0.75)])
+def test_error_of_the_token_loop(S, H, decay, rank, times):
+    proj, wraw, bias, norm, state = _inputs(1, S, H, S + H, decay, rank)
+    start = torch.zeros(1, dtype=torch.int32, device="cuda")
+    want, end = _reference(proj, wraw, bias, norm, state, start)
+    error = lambda a, b: float((a.double() - b).norm() / b.norm())
+    chunked, looped = state.clone(), state.clone()
+    out, out2 = _call(proj, wraw, bias, norm, chunked, start), _portions(proj, wraw, bias, norm, looped, start, 31)
+    assert error(chunked, end) <= times * error(looped, end)
+    assert error(out, want) <= 1.002 * error(out2, want)  # both are the result's rounding to bf16
+
+
 @pytest.mark.parametrize("more", [0, 1])
 def test_heads_of_one_round(more):
     H = torch.cuda.get_device_properties(0).multi_processor_count + more  # with one more the token loop

@@ -475,8 +475,8 @@ static bool delta_fast_serves(const TpxDeltaRule& a) {
 static int delta_fast(const TpxDeltaRule& a, cudaStream_t st) {
   DeltaFastParams p = {(const uint16_t*)a.proj, a.wraw, a.a_bias, a.norm_w, a.start, a.dev_len, a.state, (uint16_t*)a.out, (long long)a.ldp,
                        (long long)a.ldo, (int)a.S, (int)a.past, (int)a.heads, (int)a.dim, a.eps};
-  // Heads of 64 that one round of CTAs holds: sixteen tokens at a time as matrix products, from 32 tokens on (1 x 4096, 64 heads: 1380 us token by token, 900 so;
-  // 2 x 512, 16 heads 177 / 120; 1 x 33, 2 heads 20 / 16). With more heads the token loop has enough warps (16 x 256, 64 heads: 381 / 410).
+  // Heads of 64 that one round of CTAs holds: sixteen tokens at a time as matrix products, from 32 tokens on (1 x 4096, 64 heads: 1380 us token by token, 926 so;
+  // 2 x 512, 16 heads 177 / 126; 1 x 33, 2 heads 20 / 16). With more heads the token loop has enough warps (16 x 256, 64 heads: 381 / 410).
   if (a.dim == 64 && a.S >= 32 && a.B * a.heads <= sm_count()) return delta_chunk(p, a.B, st);
   // eight columns per thread and few warps per head when there are many heads, more warps per head when a token's latency counts
   const bool many = a.B * a.heads >= (a.dim <= 64 ? 4 : 2) * sm_count();

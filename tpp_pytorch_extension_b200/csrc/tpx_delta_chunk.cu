@@ -16,11 +16,13 @@
 // below loses both. A chunk with one, or with a value so large that a product of two overflows, goes token by token (dc_token_loop), and so does one that finds
 // such a state, for the value channels of that warp.
 //
-// State and sums are 32-bit: mma.sync in TF32 with both operands as a rounded value and the rounded remainder, three products each (two where the operand is v, whose
-// bf16 values are TF32 values). Decays and rates take the library's exponential and division: with the fast ones the state was 1.25e-7 off 64 bits, so 1.02e-7 (the
-// token loop 1.03e-7 to 1.08e-7); o's rounding to bf16 hides either.
+// State and sums are 32-bit. mma.sync in TF32 with both operands as a rounded value and the rounded remainder, which hold 23 of 24 bits, three products each (two
+// where the operand is v, whose bf16 values are TF32 values; that of the two remainders, below 2^-22, is left out); an MMA's own sums are cut off, not rounded.
+// Decays and rates take the library's exponential and division, without which the state was 1.25e-7 off 64 bits. As it is, here / token loop: keys of all
+// directions 1.0e-7 / 1.05e-7, with slow decays 1.4e-7 / 2.35e-7 and less beside it the slower, with the fastest 1.04e-7 / 0.87e-7 (512 tokens); keys of four
+// directions 1.2e-7 / 1.1e-7, of one 1.4e-7 / 1.1e-7 to 2.9e-7 / 1.6e-7. o's rounding to bf16, 1.66e-3, hides any of it.
 // Bound by the instructions of the preparation (11000 of a chunk's 14700; splits, fragment loads, the triangular solve): issue slots 56 % busy, tensor pipe 31 %, the
-// applying warps alone would take half the time. One sequence of 4096 tokens, 64 heads: 906 us, the token loop 1380; 2 of 512, 16 heads 119 / 177. One CTA per SM: with more
+// applying warps alone would take half the time. One sequence of 4096 tokens, 64 heads: 926 us, the token loop 1380; 2 of 512, 16 heads 126 / 177. One CTA per SM: with more
 // heads than SMs the token loop is as fast (16 of 256, 64 heads 381 us, here 410).
 #include "tpx_delta.cuh"
 
@@ -68,6 +70,16 @@ __device__ __forceinline__ void dc_mma(float (&d)[4], const float (&a)[4], float
 // The larger magnitude, a NaN before all; the sign is of no use. Below the bounds a chunk's products are all finite, and so is the split.
 constexpr float kDcBig = 1125899906842624.0f, kDcBigState = 1.2676506002282294e30f;  // 2^50, 2^100
 __device__ __forceinline__ void dc_larger(float& m, float x) { asm("max.NaN.xorsign.abs.f32 %0, %0, %1;" : "+f"(m) : "f"(x)); }
+__device__ __forceinline__ void dc_mma0(float (&d)[4], const float (&a)[4], float b0, float b1) {  // the product alone
+  asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+      : "r"(__float_as_uint(a[0])), "r"(__float_as_uint(a[1])), "r"(__float_as_uint(a[2])), "r"(__float_as_uint(a[3])), "r"(__float_as_uint(b0)),
+        "r"(__float_as_uint(b1)), "f"(0.0f));
+}
+__device__ __forceinline__ void dc_add(float (&d)[4], const float (&x)[4]) {
+#pragma unroll
+  for (int i = 0; i < 4; i++) d[i] += x[i];
+}
 __device__ __forceinline__ void dc_bar_sync(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
 __device__ __forceinline__ void dc_bar_arrive(int id, int n) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(n) : "memory"); }
 __device__ __forceinline__ bool dc_bar_any(int id, int n, bool mine) {
@@ -161,7 +173,8 @@ __global__ void __launch_bounds__(kDcThreads, 1) delta_chunk_kernel(DeltaFastPar
         dc_token_loop(s, B, o, e0);
       } else {
         // [q of tokens 0-7, 8-15, o of tokens 0-7, 8-15], transposed; small: the products with remainders, summed for themselves, and the others in
-        // two sums: an MMA's addition is cut off, not rounded. Products that go to the same sum are four apart: an MMA waits for its accumulator.
+        // two sums: an MMA's addition is cut off, not rounded. Products that go to the same sum are four apart: an MMA waits for its accumulator. (Every product
+        // added outside: 6 % slower, no nearer to 64 bits but for keys of one direction.)
         float x[4][4], y[4][4], small[4][4];
 #pragma unroll
         for (int n = 0; n < 4; n++)
@@ -355,7 +368,8 @@ __global__ void __launch_bounds__(kDcThreads, 1) delta_chunk_kernel(DeltaFastPar
       if (q0 == 12) sm.g[ch] = G;
     }
     const bool loop = dc_bar_any(bar, 32 * kDcPrep, !(fabsf(most) < kDcBig));
-    // [u; R] [K; A]^T: a tile of 16 x 8 per warp.
+    // [u; R] [K; A]^T: a tile of 16 x 8 per warp. The main products are added outside, rounded: keys of one direction have sums of terms of one sign, and cut
+    // off they put the state 2.2e-7 off 64 bits, so 1.45e-7 (1030 tokens; the token loop 1.1e-7). 1 x 4096 tokens, 64 heads take 926 us instead of 916.
     if (!loop) {
       const float* left = (pw & 1) ? sm.r : sm.u;
       const float* right = ((pw >> 1) & 2) ? sm.a : sm.k;
@@ -374,7 +388,9 @@ __global__ void __launch_bounds__(kDcThreads, 1) delta_chunk_kernel(DeltaFastPar
         dc_split(rr.y, bh[1], bl[1]);
         dc_mma(x1, l, bh[0], bh[1]);
         dc_mma(x2, h, bl[0], bl[1]);
-        dc_mma(x, h, bh[0], bh[1]);
+        float one[4];
+        dc_mma0(one, h, bh[0], bh[1]);
+        dc_add(x, one);
       }
       float* to = (pw & 1) ? (((pw >> 1) & 2) ? sm.g2 : sm.g1) : (((pw >> 1) & 2) ? sm.n : sm.m);
 #pragma unroll
