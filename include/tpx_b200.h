@@ -200,7 +200,7 @@ int tpx_linear_bf16_tc(const uint16_t* w, const uint16_t* x, int64_t M, int64_t 
  * (zero padding) and swT its scales [K/block][ceil(N/128)*128], both built by tpx_repack_qint8_tc from the
  * interchange tensors of tpx_remap_and_quantize_qint8. Block sizes 64, 128, 256, 512. Post-ops as tpx_qlinear. The
  * scratch holds the quantised activations; its first 64 KiB as for tpx_qlinear. reuse_act != 0 skips the quantisation
- * and reads what the previous call on the same scratch left there (same x, same K and block size: the second linear
+ * and reads what the previous call on the same scratch left there (same x, M, K and block size, any N: the second linear
  * of a gate/up pair). gamma != NULL applies an RMSNorm (gamma bf16 or fp32, eps) to x before the quantisation, in the
  * same kernel (rows of up to 8192 values, blocks of up to 256).                                                    */
 int tpx_tc_packed_bytes_qint8(int64_t N, int64_t K, int64_t block_size, size_t* wq_bytes, size_t* sw_bytes);

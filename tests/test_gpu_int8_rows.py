@@ -128,3 +128,28 @@ def test_result_over_activations(M, monkeypatch):
         y = x.clone()
         F.fc_plain(y, w, out=y)
         assert torch.equal(y, want)
+
+
+# 272 and 14224 features: 17 and 889 tiles of 16, which different kernels take at 17 to 32 tokens; 320: half a step of 128 k values left over
+@pytest.mark.parametrize("M", [1, 2, 8, 16, 17, 24, 32, 33])
+@pytest.mark.parametrize("first,second", [(272, 14224), (14224, 272), (272, 272)])
+@pytest.mark.parametrize("K", [320, 4096])
+def test_reuse_across_sizes(M, first, second, K):
+    from tpp_pytorch_extension_b200 import _lib
+    L = _lib.lib()
+    g = torch.Generator(device="cuda").manual_seed(M + first)
+    x = torch.randn(M, K, generator=g, device="cuda").to(torch.bfloat16)
+    gamma = torch.randn(K, generator=g, device="cuda")
+    need = max(L.tpx_qlinear_qint8_tc_scratch_bytes(M, N, K, 64) for N in (first, second))
+    sc = torch.zeros(need, device="cuda", dtype=torch.uint8)
+
+    def call(w, x, gamma, reuse):
+        y = torch.empty(M, w[0].shape[0], device="cuda", dtype=torch.bfloat16)
+        _lib.check(L.tpx_qlinear_qint8_tc(w[2].data_ptr(), w[3].data_ptr(), x.data_ptr(), _lib.ptr(gamma), 1, 1e-5, M, y.shape[1], K, 64, reuse, None, 0, None, None, 0.0,
+                                          y.data_ptr(), sc.data_ptr(), need, _lib.stream()))
+        return y
+
+    a, b = _weight(first, K, g), _weight(second, K, g)
+    want = call(b, x, gamma, 0)
+    call(a, x, gamma, 0)
+    assert torch.equal(call(b, torch.zeros_like(x), None, 1), want)  # what the call before left in the scratch

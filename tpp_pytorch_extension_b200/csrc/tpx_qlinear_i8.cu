@@ -31,24 +31,6 @@ struct I8Params {
   int tilesN;          // feature tiles; CTA (or cluster) t works on feature tile t % tilesN, token tile t / tilesN
 };
 
-// The quantised activations of a token tile and k step (128 values) are one run of memory, fetched by one untiled copy: TOK rows of 128
-// bytes, their 16-byte units in the order of the 128-byte swizzle, then the scales of the step's blocks, [1 or 2][TOK] (a block that
-// spans several steps: with its last one). As plain rows of K bytes the 16 pieces of a step lay a power of two apart, and all CTAs
-// asking for them at once was what bounded the kernel (11008 x 4096, 16 tokens: 20 us, 19.4 without any weight traffic).
-struct I8Act {
-  int TOK, ksteps, B, bytes;  // bytes per (token tile, step)
-  __host__ __device__ I8Act(int tok, int ks, int block) : TOK(tok), ksteps(ks), B(block), bytes(tok * 128 + (block == 64 ? 2 : 1) * tok * 4) {}
-  __device__ __forceinline__ uint8_t* step(uint8_t* xq, int tok, int k) const { return xq + ((size_t)(tok / TOK) * ksteps + k / 128) * bytes; }
-  __device__ __forceinline__ uint8_t* value(uint8_t* xq, int tok, int k) const {  // up to the next 16 values
-    const int r = tok % TOK;
-    return step(xq, tok, k) + r * 128 + (((k % 128) / 16) ^ (r & 7)) * 16 + k % 16;
-  }
-  __device__ __forceinline__ float* scale(uint8_t* xq, int tok, int blk) const {
-    const int k = blk * B + B - 1;
-    return reinterpret_cast<float*>(step(xq, tok, k) + TOK * 128) + (B == 64 ? blk & 1 : 0) * TOK + tok % TOK;
-  }
-};
-
 __device__ __forceinline__ void i8_mma(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{ .reg .pred p; setp.ne.b32 p, %4, 0;\n"
@@ -312,7 +294,8 @@ qlinear_i8_kernel(const __grid_constant__ CUtensorMap tmW, I8Params p) {
     // ------------------------------------------------------------ MMA issuer
     // kind::i8: D = S32 (2), A = B = S8 (1), both K-major, N = TOK, M = 128
     constexpr uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TOK >> 3) << 17) | ((128u >> 4) << 24);
-    const uint64_t desc0 = tc_smem_desc(smem_base);
+    constexpr bool HALF = I8Act32::serves(TOK, BS * 32);  // the B operand has a block's rows of 64 bytes
+    const uint64_t desc0 = tc_smem_desc(smem_base), bdesc0 = HALF ? tc_smem_desc64(smem_base + C::A_BYTES) : tc_smem_desc(smem_base + C::A_BYTES);
     int s = 0, g = 0;  // g: groups handed out
     uint32_t phase = 0;
     bool dead = false;
@@ -337,10 +320,11 @@ qlinear_i8_kernel(const __grid_constant__ CUtensorMap tmW, I8Params p) {
         }
         tc_fence_after();
         if (tc_elect()) {
-          const uint64_t desc = desc0 + (uint64_t)(s * (C::STAGE_BYTES >> 4));  // descriptors count 16-byte units
+          const uint64_t at = (uint64_t)(s * (C::STAGE_BYTES >> 4));  // descriptors count 16-byte units
 #pragma unroll
           for (int j = 0; j < 4; j++)
-            i8_mma(d + (4 * t + j) / BS * TOK, desc + (uint64_t)(2 * j), desc + (uint64_t)((C::A_BYTES >> 4) + 2 * j), idesc, (4 * t + j) % BS ? 1u : 0u);
+            i8_mma(d + (4 * t + j) / BS * TOK, desc0 + at + (uint64_t)(2 * j), bdesc0 + at + (uint64_t)(HALF ? (j >> 1) * TOK * 4 + 2 * (j & 1) : 2 * j), idesc,
+                   (4 * t + j) % BS ? 1u : 0u);
         }
         __syncwarp();
         if (++s == C::STAGES) s = 0, phase ^= 1u;
@@ -656,29 +640,30 @@ static int i8_linear(const int8_t* wq, const float* swT, const int8_t* wq2, cons
   t.bias = bias; t.mul_in = mul_in; t.res = res; t.res_scale = res_scale; t.y = y; t.act = act;
   t.M = (int)M; t.N = (int)N; t.K = (int)K; t.cluster = pl.cluster;
   t.err = reinterpret_cast<unsigned*>(sc + kTcCounterBytes - 4);
-  if (i8_rows_serves(M, N, block_size, wq2 != nullptr)) {
-    const I8Rows L((int)M, K);
-    I8RowsParams p = {};
-    if (!reuse_act && i8_rows_quantizes(x, y, M, N, K)) {
-      p.x = x; p.gamma = gamma; p.gamma_f32 = gamma_is_f32; p.eps = eps;
-    } else if (!reuse_act) {
-      int rc = i8_quantize(x, gamma, gamma_is_f32, eps, (int)M, (int)M, K, L, xq, st);
-      if (rc) return rc;
-    }
-    p.t = t;
-    p.w[0] = wq; p.w[1] = wq2; p.swT[0] = swT; p.swT[1] = swT2; p.xq = xq;
-    p.nkb = L.nkb; p.Mp = L.Mp; p.Kp = (int)pl.Kp; p.Np = (int)pl.Np; p.tiles = (int)(N / 16);
-    return i8_rows_launch(p, wq2 != nullptr, st);
-  }
+  const bool rows = i8_rows_serves(M, N, block_size, wq2 != nullptr);
+  I8RowsParams r = {};
+  // The order of the quantised activations depends on M, K and block_size alone, so that a call that reuses them may be of another N, and another kernel's.
   const I8Act L(pl.tokp, pl.ksteps, (int)block_size);
-  if (!reuse_act && pl.Kp != K) TPX_CUDA_OK(cudaMemsetAsync(xq, 0, pl.xq_bytes, st));  // the k padding reads as zero
-  if (!reuse_act && block_size <= 256) {
-    int rc = i8_quantize(x, gamma, gamma_is_f32, eps, (int)M, (int)pl.Mp, K, L, xq, st);
+  if (!reuse_act && rows && i8_rows_quantizes(x, y, M, N, K)) {
+    r.x = x; r.gamma = gamma; r.gamma_f32 = gamma_is_f32; r.eps = eps;
+  } else if (!reuse_act && rows && M <= 16) {
+    int rc = i8_quantize(x, gamma, gamma_is_f32, eps, (int)M, (int)M, K, I8Rows((int)M, K), xq, st);
+    if (rc) return rc;
+  } else if (!reuse_act && block_size <= 256) {
+    if (!rows && pl.Kp != K) TPX_CUDA_OK(cudaMemsetAsync(xq, 0, pl.xq_bytes, st));  // the k padding reads as zero, as the weight's
+    int rc = I8Act32::serves(pl.tokp, (int)block_size) ? i8_quantize(x, gamma, gamma_is_f32, eps, (int)M, 32, K, I8Act32(), xq, st)
+                                                       : i8_quantize(x, gamma, gamma_is_f32, eps, (int)M, (int)pl.Mp, K, L, xq, st);
     if (rc) return rc;
   } else if (!reuse_act) {
     const long long warps = (long long)pl.Mp * (K / 512);
     TPX_CUDA_OK(launch_pdl(quantize_act_i8_block512_kernel, dim3((unsigned)((warps + kQbWarps - 1) / kQbWarps)), dim3(kQbWarps * 32), 0, st, x, (int)M, (int)K,
                            (int)pl.Mp, L, xq));
+  }
+  if (rows) {
+    r.t = t;
+    r.w[0] = wq; r.w[1] = wq2; r.swT[0] = swT; r.swT[1] = swT2; r.xq = xq;
+    r.nkb = (int)(K / 64); r.Mp = I8Rows((int)M, K).Mp; r.Kp = (int)pl.Kp; r.Np = (int)pl.Np; r.tiles = (int)(N / 16);
+    return i8_rows_launch(r, wq2 != nullptr, st);
   }
   CUtensorMap mw;
   int rc = make_map_u8(&mw, wq, (uint64_t)pl.Np, (uint64_t)pl.Kp, 128);
@@ -698,8 +683,6 @@ static int i8_linear(const int8_t* wq, const float* swT, const int8_t* wq2, cons
 extern "C" int tpx_qlinear_qint8_tc(const int8_t* wq, const float* swT, const uint16_t* x, const void* gamma, int gamma_is_f32, float eps,
                                     int64_t M, int64_t N, int64_t K, int64_t block_size, int reuse_act, const uint16_t* bias, int act, const uint16_t* mul_in,
                                     const uint16_t* res, float res_scale, uint16_t* y, void* scratch, size_t scratch_bytes, void* stream) {
-  // between 17 and 32 tokens the order of the quantised activations depends on N, which the previous call may have had another of
-  if (block_size == 64 && M > 16 && M <= 32) reuse_act = 0;
   return i8_linear(wq, swT, nullptr, nullptr, x, gamma, gamma_is_f32, eps, M, N, K, block_size, reuse_act, bias, act, mul_in, res, res_scale, y,
                    scratch, scratch_bytes, stream);
 }

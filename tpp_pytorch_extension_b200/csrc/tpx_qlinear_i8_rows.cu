@@ -132,11 +132,13 @@ __global__ void __launch_bounds__(IrCfg<T, MG>::W * 32, 1) qlinear_i8_rows_kerne
   const char* const sb0 = reinterpret_cast<const char*>(p.swT[0] + tile0 * 16);
   const char* const sb1 = DUAL ? reinterpret_cast<const char*>(p.swT[1] + tile0 * 16) : nullptr;
   uint32_t w0 = f0 * row16 + g * p.Kp + t * 16 + turn * 128, s0 = turn * 8 * p.Np + f0 * 64 + lane * 16;
-  const uint32_t xrow = (QUANT ? p.t.M : p.Mp) * 64, xstep = groups * 2 * xrow;
+  constexpr bool STEPS = MG == 4;  // activations I8Act32, as the tcgen05 kernel has them, which serves the same calls of other N
+  constexpr uint32_t kStepScales = 32 * 128, kStep = I8Act32::BYTES;
+  const uint32_t xrow = (QUANT ? p.t.M : p.Mp) * 64, xstep = groups * (STEPS ? kStep : 2 * xrow);
   const uint8_t* const sxb = p.xq + (size_t)p.nkb * xrow;  // a scale is 4 bytes where its 64 values are 64
-  uint32_t x0 = turn * 2 * xrow;
+  uint32_t x0 = turn * (STEPS ? kStep : 2 * xrow);
   const int last = p.t.M - 1;  // QUANT: columns behind the last token repeat it and are not stored
-  const uint32_t xl = (QUANT ? min(g, last) : g) * 64 + t * 16;
+  const uint32_t xl = STEPS ? g * 64 + (t ^ (g >> 1)) * 16 : (QUANT ? min(g, last) : g) * 64 + t * 16;
   const uint32_t xs = tc_smem_u32(ir_smem_raw) + (uint32_t)C::SMEM, fs = xs + p.nkb * xrow;
   pdl_trigger();
 
@@ -163,8 +165,14 @@ __global__ void __launch_bounds__(IrCfg<T, MG>::W * 32, 1) qlinear_i8_rows_kerne
   uint4 xv[2][MG];
   float2 sv[2][MG];
   auto fetch = [&](int z, int td) {
-    const uint32_t x = x0 + (td >> 1) * xstep + (td & 1) * xrow;
-    if constexpr (QUANT) {
+    const uint32_t x = x0 + (td >> 1) * xstep + (STEPS ? 0 : (td & 1) * xrow);
+    if constexpr (STEPS) {
+#pragma unroll
+      for (int m = 0; m < MG; m++) {
+        xv[z][m] = rows_ldg16(p.xq + (x + xl + (td & 1) * 2048 + m * 512));
+        sv[z][m] = rows_ldg8(p.xq + (x + kStepScales + (td & 1) * 128 + t * 8 + m * 32));
+      }
+    } else if constexpr (QUANT) {
       xv[z][0] = rows_lds16(xs + x + xl);
       sv[z][0] = make_float2(rows_lds4(fs + x / 16 + min(2 * t, last) * 4), rows_lds4(fs + x / 16 + min(2 * t + 1, last) * 4));
     } else {

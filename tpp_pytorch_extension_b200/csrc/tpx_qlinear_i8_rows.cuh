@@ -4,12 +4,43 @@
 
 namespace tpx {
 
-// Quantised activations, blocks of 64 values: [K/64][Mp][64] int8, then the scales [K/64][Mp]. The 16 bytes that a lane of the kernel's MMAs
+// The quantised activations of a token tile and k step (128 values) are one run of memory, fetched by one untiled copy: TOK rows of 128
+// bytes, their 16-byte units in the order of the 128-byte swizzle, then the scales of the step's blocks, [1 or 2][TOK] (a block that
+// spans several steps: with its last one). As plain rows of K bytes the 16 pieces of a step lay a power of two apart, and all CTAs
+// asking for them at once was what bounded the kernel (11008 x 4096, 16 tokens: 20 us, 19.4 without any weight traffic).
+struct I8Act {
+  int TOK, ksteps, B, bytes;  // bytes per (token tile, step)
+  __host__ __device__ I8Act(int tok, int ks, int block) : TOK(tok), ksteps(ks), B(block), bytes(tok * 128 + (block == 64 ? 2 : 1) * tok * 4) {}
+  __device__ __forceinline__ uint8_t* step(uint8_t* xq, int tok, int k) const { return xq + ((size_t)(tok / TOK) * ksteps + k / 128) * bytes; }
+  __device__ __forceinline__ uint8_t* value(uint8_t* xq, int tok, int k) const {  // up to the next 16 values
+    const int r = tok % TOK;
+    return step(xq, tok, k) + r * 128 + (((k % 128) / 16) ^ (r & 7)) * 16 + k % 16;
+  }
+  __device__ __forceinline__ float* scale(uint8_t* xq, int tok, int blk) const {
+    const int k = blk * B + B - 1;
+    return reinterpret_cast<float*>(step(xq, tok, k) + TOK * 128) + (B == 64 ? blk & 1 : 0) * TOK + tok % TOK;
+  }
+};
+
+// The same for a tile of 32 tokens in blocks of 64, which the kernel for few tokens reads where N lets it: the 32 rows of 64 bytes of one block, then the
+// other's, in the order of the 64-byte swizzle. The tile is the only one, so that places are found without a division (1 us of a linear of 32 tokens).
+struct I8Act32 {
+  static constexpr int B = 64, BYTES = 32 * 128 + 2 * 32 * 4;  // bytes per step
+  static __host__ __device__ constexpr bool serves(int tok, int block) { return tok == 32 && block == B; }
+  __device__ __forceinline__ uint8_t* value(uint8_t* xq, int tok, int k) const {
+    const uint32_t u = k;
+    return xq + (u / 128 * BYTES + (u % 128 / 64 * 32 + tok) * 64 + ((u % 64 / 16) ^ (((uint32_t)tok >> 1) & 3)) * 16 + u % 16);
+  }
+  __device__ __forceinline__ float* scale(uint8_t* xq, int tok, int blk) const {
+    return reinterpret_cast<float*>(xq + ((uint32_t)blk / 2 * BYTES + 32 * 128)) + (blk & 1) * 32 + tok;
+  }
+};
+
+// Of up to 16 tokens, blocks of 64 values: [K/64][Mp][64] int8, then the scales [K/64][Mp]. The 16 bytes that a lane of the kernel's MMAs
 // takes from a token are one piece, and a warp's 32 pieces (8 tokens) are one run of 512 bytes.
 struct I8Rows {
   int Mp, nkb, B;  // tokens, padded to what a kernel reads; k blocks; B = 64, the scale block, as in I8Act
-  __host__ __device__ I8Rows(int M, int64_t K) : Mp(M <= 8 ? 8 : M <= 16 ? 16 : 32), nkb((int)(K / 64)), B(64) {}
-  __host__ __device__ size_t bytes() const { return (size_t)nkb * Mp * 68; }
+  __host__ __device__ I8Rows(int M, int64_t K) : Mp(M <= 8 ? 8 : 16), nkb((int)(K / 64)), B(64) {}
   __device__ __forceinline__ uint8_t* value(uint8_t* xq, int tok, int k) const { return xq + ((size_t)(k / 64) * Mp + tok) * 64 + k % 64; }
   __device__ __forceinline__ float* scale(uint8_t* xq, int tok, int blk) const {
     return reinterpret_cast<float*>(xq + (size_t)nkb * Mp * 64) + (size_t)blk * Mp + tok;
@@ -61,7 +92,7 @@ struct I8RowsParams {
   TcParams t;                // epilogue fields (bias, act, mul_in, res, res_scale, y, M, N)
   const int8_t* w[2];        // plain int8 weight [Np][Kp]; of a pair: gate, up
   const float* swT[2];       // [K/64][Np]
-  uint8_t* xq;               // I8Rows
+  uint8_t* xq;               // I8Rows; of more than 16 tokens I8Act32
   const uint16_t* x;         // or, if not null: bf16 activations, to be quantised (behind an RMSNorm if gamma is set) and left in xq as well
   const void* gamma;
   int gamma_f32;
