@@ -9,6 +9,10 @@
  *   - bf16 tensors are passed as uint16_t bit patterns, row-major, contiguous;
  *   - every call enqueues work on `stream` (a cudaStream_t passed as void*) and returns without
  *     synchronising; nothing allocates device memory: scratch is passed in by the caller;
+ *   - calls on one stream see each other's results, with one exception: linears of up to 64 tokens start to copy their
+ *     weight (w, wq and its scales) while the kernels of this library in front of them still run, so that a weight which
+ *     one of those has written (tpx_unpack_qint8_tc_bf16, a linear's result) needs a synchronisation or another
+ *     library's kernel in between. Their activations, norm weights, biases and residuals need none;
  *   - return value 0 = success; otherwise a TPX_ERR_* code, with text from tpx_last_error().
  *     The reference aborts the process on its own argument checks (TPP_ASSERT -> exit(1),
  *     src/csrc/utils.h:34-41); this library reports instead.

@@ -162,3 +162,42 @@ def test_result_over_activations(M):
         y = x.clone()
         F.fc_plain(y, w, out=y)
         assert float((y - want).float().norm() / want.float().norm()) < 1e-3  # another group adds the same products
+
+
+@pytest.mark.parametrize("kind", ["mxfp4", "qint8"])
+@pytest.mark.parametrize("M", [1, 2, 8])
+def test_norm_weight_of_the_kernel_before(kind, M, monkeypatch):
+    """A norm's weight that the kernel in front has just written, into a place that held another."""
+    from tpp_pytorch_extension_b200 import _lib
+    from tpp_pytorch_extension_b200._C import _fused_llm_infer as F
+    from tpp_pytorch_extension_b200.llm.llm_common import quantize_weight
+    monkeypatch.setenv("QINT8_BLOCK_SIZE", "64")
+    L = _lib.lib()
+    g = torch.Generator(device="cuda").manual_seed(M)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda").to(torch.bfloat16)
+    D = 2048
+    w, make = quantize_weight(rnd(D, D) * D ** -0.5, kind), rnd(D, D) * D ** -0.5
+    sc = torch.zeros(L.tpx_linear_bf16_tc_scratch_bytes(1, D, D), device="cuda", dtype=torch.uint8)
+    x, seeds, gamma = rnd(M, D), rnd(8, 1, D), torch.empty(1, D, device="cuda", dtype=torch.bfloat16)
+
+    def chain(wait):
+        ys = []
+        for s in seeds:
+            _lib.check(L.tpx_linear_bf16_tc(make.data_ptr(), s.data_ptr(), 1, D, D, None, 0, None, None, 0.0, gamma.data_ptr(), sc.data_ptr(), sc.numel(), _lib.stream()))
+            wait()
+            ys.append(F.fc_plain_norm(x, gamma.view(-1), 1e-5, w))
+            wait()
+        return torch.stack(ys)
+
+    want = chain(torch.cuda.synchronize)
+    assert not torch.equal(want[0], want[1])
+    graph, stream = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        chain(lambda: None)
+        torch.cuda.synchronize()
+        with torch.cuda.graph(graph, stream=stream):
+            got = chain(lambda: None)
+    for _ in range(3):
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(got, want)

@@ -78,7 +78,8 @@ const Knobs& knobs();
 // kernel in the stream may be scheduled and run its prologue while this one works) and calls pdl_wait() before
 // it touches global memory that an earlier kernel may have written or may still read: the wait returns once
 // every earlier grid has completed and its writes are visible, so the memory order is that of plain stream
-// launches and only launch latency and prologues overlap.
+// launches and only launch latency and prologues overlap. The exception are the weights of the linears of up to 64 tokens, whose first copies go out ahead of
+// the wait (a model's weights are not the output of a kernel in flight; the public header says so).
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

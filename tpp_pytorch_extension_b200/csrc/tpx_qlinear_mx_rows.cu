@@ -233,8 +233,10 @@ __global__ void __launch_bounds__(MrCfg<T, MG, MODE>::W * 32, 1) qlinear_mx_rows
       if ((q & 15) == 0) asm volatile("st.shared.f32 [%0], %1;" ::"r"(fs + (uint32_t)((q >> 4) * M + m) * 4), "f"(mr_unscale(f)) : "memory");
     };
     float gm[8], ss[8];
-    if (MODE == kMrNorm && (int)threadIdx.x * 8 < p.t.K) mr_gamma(p.gamma, p.gamma_f32, threadIdx.x, gm);
+    if (MODE == kMrNorm)
+      for (int q = threadIdx.x; q * 8 < p.t.K; q += C::W * 32) rows_prefetch_gamma(p.gamma, p.gamma_f32, q);
     pdl_wait();
+    if (MODE == kMrNorm && (int)threadIdx.x * 8 < p.t.K) mr_gamma(p.gamma, p.gamma_f32, threadIdx.x, gm);
 #pragma unroll
     for (int m = 0; m < 8; m++) ss[m] = 0.0f;
     for (int q0 = 0; q0 < pieces; q0 += C::W * 32) {
@@ -357,6 +359,9 @@ __global__ void __launch_bounds__(kMpThreads) mx_rows_prep_kernel(MxRowsParams p
   constexpr int V = NORM ? kMpVecs : 1;
   const int m = blockIdx.x, q0 = blockIdx.y * kMpThreads + threadIdx.x, pieces = p.steps * 16;
   pdl_trigger();
+  if (NORM)
+    for (int q = q0; q * 8 < p.t.K; q += kMpThreads) rows_prefetch_gamma(p.gamma, p.gamma_f32, q);
+  pdl_wait();
   float gm[V][8];
   if (NORM)
 #pragma unroll
@@ -364,7 +369,6 @@ __global__ void __launch_bounds__(kMpThreads) mx_rows_prep_kernel(MxRowsParams p
       const int q = q0 + v * kMpThreads;
       if (q * 8 < p.t.K) mr_gamma(p.gamma, p.gamma_f32, q, gm[v]);
     }
-  pdl_wait();
   uint4 x[V];
 #pragma unroll
   for (int v = 0; v < V; v++) {
