@@ -183,7 +183,7 @@ int tpx_qlinear_mxfp4_tc_static(const uint8_t* wq, const uint8_t* sfa, int pair,
  * the reference leaves in bf16 unless it is asked to quantize it (examples/llm/run_generation.py:277-282).
  *     y[M][N] = epilogue(x[M][K] . w[N][K]^T + bias[N]),   epilogue as for tpx_qlinear
  * w is the plain row-major weight (nn.Linear.weight), not re-laid out; K a multiple of 8; any M and N. fp32
- * accumulation, one bf16 rounding at the store.
+ * accumulation, one bf16 rounding at the store. y may lie over x for up to 64 tokens and 128 features, else not.
  * The scratch (256-byte aligned; tpx_linear_bf16_tc_scratch_bytes gives its size for M, N and K) holds arrival counters of tiles
  * that are cut along k in its first 64 KiB, with the error word of the bounded waits at byte 65532, and behind them the partial sums
  * of such tiles (up to about 20 MB). The first 64 KiB are zero before the first use and left zero (but for the error word); what lies

@@ -24,7 +24,8 @@ extern "C" {
 enum { TPX_ACT_TANH = 4, TPX_ACT_XIELU = 5, TPX_ACT_CLAMPED_GLU = 6 };
 
 /* y[M][N] = act(x[M][K] . w[N][K]^T + bias[N]); the activation applies to columns n >= act_from. Leading dimensions in
- * elements. bf16 operands run on the tcgen05 kernel and need K, ldx, ldw multiples of 8 and 16-byte aligned bases; fp32
+ * elements. bf16 operands run on the tensor cores and need K, ldx, ldw multiples of 8 and 16-byte aligned bases (their results may lie over x as those of
+ * tpx_linear_bf16_tc may); fp32
  * operands run on the 32-bit kernels: with scratch of tpx_linear_f32_scratch_bytes(M, N, K) many rows run on the tensor cores
  * (every operand as three bf16 terms that hold all its bits; rows of x and weights with an infinity, a NaN or a value of 2^30 and more are
  * computed on the CUDA cores), without it on the CUDA cores. scratch as for tpx_linear_bf16_tc, whatever the operands: its first 64 KiB

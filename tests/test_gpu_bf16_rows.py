@@ -62,3 +62,31 @@ def test_recorded_chain(M):
         graph.replay()
         torch.cuda.synchronize()
         assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("M", [1, 8, 17, 32])
+@pytest.mark.parametrize("N,K", [(16, 16), (128, 128), (128, 4096), (120, 200)])
+def test_result_over_activations(M, N, K):
+    """Up to 128 features: into the activations' own memory, from its start, from its end, with and without the activations' row stride."""
+    from tpp_pytorch_extension_b200 import _lib
+    from tpp_pytorch_extension_b200._C import _hybrid_layers as HL
+    L = _lib.lib()
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    w = (torch.randn(N, K, generator=g, device="cuda") * K ** -0.5).to(torch.bfloat16)
+    x = torch.randn(M, K, generator=g, device="cuda").to(torch.bfloat16)
+    sc = torch.zeros(L.tpx_linear_bf16_tc_scratch_bytes(M, N, K), device="cuda", dtype=torch.uint8)
+    want = x.double() @ w.double().T
+    err = (K // 16 + 40) * 2.0 ** -23 * (x.double().abs() @ w.double().abs().T)
+    for _ in range(4):
+        for at in (0, M * K - M * N):
+            if at < 0:
+                continue
+            buf = x.clone().flatten()
+            y = buf[at:at + M * N].view(M, N)
+            _lib.check(L.tpx_linear_bf16_tc(w.data_ptr(), buf.data_ptr(), M, N, K, None, 0, None, None, 0.0, y.data_ptr(), sc.data_ptr(), sc.numel(), _lib.stream()))
+            assert bool(((y.double() - want).abs() <= 2.0 ** -8 * want.abs() + err).all())
+        buf = torch.empty(M, K + 8, device="cuda", dtype=torch.bfloat16)
+        buf[:, :K] = x
+        y = buf[:, K - min(N, K):K - min(N, K) + N]
+        HL._linear_call(buf[:, :K], w, y)
+        assert bool(((y.double() - want).abs() <= 2.0 ** -8 * want.abs() + err).all())

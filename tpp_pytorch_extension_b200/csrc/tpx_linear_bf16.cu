@@ -406,11 +406,30 @@ static int bf_split_ctas(int64_t M, int64_t N, int64_t K) {
 }
 static size_t bf_split_bytes(int64_t M, int grid) { return (size_t)grid * 2 * (M <= 16 ? 16 : M <= 32 ? 32 : 64) * 128 * 4; }
 
+// Whether rows of x (x_bytes each, x_ld apart) share memory with rows of y; those of one matrix do where their columns do.
+static bool bf_meet(const void* x, size_t x_bytes, size_t x_ld, const void* y, size_t y_bytes, size_t y_ld, int64_t rows) {
+  const uintptr_t a = (uintptr_t)x, b = (uintptr_t)y;
+  if (!y || !y_bytes || a + (rows - 1) * x_ld + x_bytes <= b || b + (rows - 1) * y_ld + y_bytes <= a) return false;
+  if (rows == 1 || x_ld != y_ld) return true;
+  const size_t from = b >= a ? (b - a) % x_ld : (x_ld - (a - b) % x_ld) % x_ld;  // y's first column, in a row of x
+  return from < x_bytes || from + y_bytes > x_ld;
+}
+// Whether the call writes over its own activations, which the CTAs of tpx_linear_bf16_rows.cu read while others already store. Up to 128 features the tcgen05
+// kernel has one tile, whose result is stored when all of x has been read.
+static bool bf_writes_x(const BfParams& p, const void* x, int64_t M, int64_t N, int64_t K, int64_t ldx) {
+  const BfEx& e = p.ex;
+  auto meets = [&](const void* y, int64_t cols, int64_t ld, size_t size) { return bf_meet(x, K * 2, ldx * 2, y, cols * size, ld * size, M); };
+  if (!e.on) return meets(p.t.y, N, N, 2);
+  if (e.x_out) return meets(e.x_out, N, e.ldr, 4) || meets(e.h, N, e.ldh, 2);
+  const bool glu = e.act == TPX_ACT_CLAMPED_GLU;
+  return meets(e.y, glu ? e.act_from : N, e.ldy, e.out_f32 ? 4 : 2) || (glu && meets(e.z, (N - e.act_from) / 2, e.ldz, 2));
+}
+
 // Tiles, tensor maps and launch for a filled epilogue.
 static int bf_run(BfParams& p, const void* w, const void* x, int64_t M, int64_t N, int64_t K, int64_t ldw, int64_t ldx, void* scratch,
                   size_t scratch_bytes, cudaStream_t st) {
   if (bf_pair_serves(p, M, N, K)) return bf_pair_run(p, w, x, M, N, K, ldw, ldx, scratch, scratch_bytes, st);
-  if (bf_rows_serves(M, N, K, ldw)) return bf_rows_run(p, w, x, M, N, K, ldw, ldx, st);
+  if (bf_rows_serves(M, N, K, ldw) && !bf_writes_x(p, x, M, N, K, ldx)) return bf_rows_run(p, w, x, M, N, K, ldw, ldx, st);
   p.ctas = bf_split_ctas(M, N, K);
   if (p.ctas && scratch_bytes < kTcCounterBytes + bf_split_bytes(M, p.ctas)) p.ctas = 0;
   p.t.counters = reinterpret_cast<unsigned*>(scratch);
