@@ -151,6 +151,45 @@ def test_gla_many_heads(cuda, dtype, dim, vdim):
         assert torch.isfinite(got).all()
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("B,dim,vdim", [(2, 64, 128), (2, 32, 64), (60, 32, 64), (60, 64, 128), (2, 20, 28)])  # columns cut, whole heads, the general kernel
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+def test_gla_infinity_and_nan(cuda, dtype, B, dim, vdim, value):
+    """One such value in q, k, v, the gate and the decay, each in a head of its own: nothing before its token and no other head changes."""
+    from tpp_pytorch_extension_b200 import _lib
+    from tpp_pytorch_extension_b200._C import _hybrid_layers as HL
+    S, H, at, ld = 21, 6, 14, 6 * 2 * (dim + vdim)
+    g = torch.Generator(device="cuda").manual_seed(dim)
+    proj = torch.randn(B, S, ld, generator=g, device="cuda").to(dtype)
+    zraw, norm = torch.randn(B, S, H, dim, generator=g, device="cuda"), torch.ones(vdim, device="cuda")
+    first = torch.randn(B, H, dim, vdim, generator=g, device="cuda")
+
+    def call(proj, zraw):
+        state, raw, out = first.clone(), torch.empty(B * S, H * vdim, device="cuda"), torch.zeros(B * S, H * vdim, device="cuda", dtype=dtype)
+        HL._call("tpx_gla", _lib.GlaStruct(
+            proj=proj.data_ptr(), zraw=zraw.data_ptr(), a2=None, a2_bias=None, norm_w=norm.data_ptr(), start=None, dev_len=None, state=state.data_ptr(), raw=raw.data_ptr(),
+            out=out.data_ptr(), B=B, S=S, past=0, ldp=ld, ldo=H * vdim, lda2=0, rank=0, heads=H, dim=dim, vdim=vdim, q_col=0, k_col=H * dim, v_col=2 * H * dim,
+            g_col=2 * H * dim + H * vdim, a1_col=0, tau=16.0, eps=1e-6, f32=int(dtype == torch.float32)))
+        return out.view(B, S, H, vdim), state
+
+    want, end = call(proj, zraw)
+    proj, zraw = proj.clone(), zraw.clone()
+    q, k, v, gate = (proj[1, at, c:c + H * n].view(H, n) for c, n in ((0, dim), (H * dim, dim), (2 * H * dim, vdim), (2 * H * dim + H * vdim, vdim)))
+    q[0, 3] = k[1, 3] = v[2, 3] = gate[3, 3] = value
+    zraw[1, at, 4, 3] = float("nan")  # (an infinity is a decay of one)
+    out, state = call(proj, zraw)
+    for h in range(5):
+        assert not out[1, at, h].isfinite().all()
+    for h in (1, 2, 4):
+        assert not state[1, h].isfinite().all()
+    apart = [0, 1, 3, 4]
+    assert torch.equal(out[1, :at, apart], want[1, :at, apart]) and torch.equal(out[1, :, 5], want[1, :, 5]) and torch.equal(state[1, 5], end[1, 5])
+    back = at if dtype == torch.float32 or dim % 8 else at - at % 4  # bf16 mode: a value's infinity reaches the tokens of its four
+    assert torch.equal(out[1, :back, 2], want[1, :back, 2])
+    others = [b for b in range(B) if b != 1]
+    assert torch.equal(out[others], want[others]) and torch.equal(state[others], end[others])
+
+
 @pytest.mark.parametrize("shift,tau", [(8.0, 16.0), (-60.0, 1.0), (-300.0, 0.5), (0.0, 0.05)])
 def test_gla_decays_at_their_ends(cuda, shift, tau):
     """Decays close to one over a long sequence (what was written far back stays) and decays that vanish within a token."""

@@ -12,7 +12,8 @@
 //                     i.e. 9 operations per state element for four tokens instead of 12, no division by a decay (all factors are
 //                     products of decays, at most 1), and no dependency between lanes. The state stays in registers, in pairs of key channels
 //                     (packed fp32). DP / LPC key channels x CPT columns per thread. In fp32 models the decays and gates take the
-//                     library's functions: 2 x 513 tokens, 16 heads of 64 / 128: 427 us token by token, 60 so.
+//                     library's functions: us, token by token / so, 16 heads of 64 / 128: 2 x 513 tokens 304 / 83, 32 x 513 (whole heads) 2133 / 735; of 32 / 128, 40 x 513 1449 / 416;
+//                     of 128 / 128, 40 x 513 6376 / 1155.
 //   gla_token_kernel  one token: a CTA per (sequence, head) streams the state through once; the low-rank map of the decay is
 //                     computed here as well.
 //   gla_kernel        any size, token by token; a column's key channels on neighbouring lanes.
@@ -307,6 +308,9 @@ struct GfCfg {
   // 16-byte units that a thread copies: rows of DP elements, DP fp32, EC elements; a thread keeps its place in the row
   static constexpr int UD = DP / EU, UZ = DP / 4, UE = EC / EU;
   static_assert(THREADS % UD == 0 && THREADS % UZ == 0 && THREADS % UE == 0, "copies");
+  // CTAs per SM that the compiler leaves registers for: twelve warps of fp32 with up to 32 key channels (left to itself 196 registers and nine: 40 x 513 tokens, 16
+  // heads of 32 / 128 578 us, so 416)
+  static constexpr int BLOCKS = EB == 4 && WHOLE && DP == 32 ? 384 / THREADS : 0;
   static constexpr int OW = EC / 32;  // columns per lane in the output norm
 };
 
@@ -317,7 +321,7 @@ __device__ __forceinline__ void gl_sync() {
 }
 
 template <typename T, int DP, int EC, int LPC, int CPT, int TC, bool WHOLE>
-__global__ void __launch_bounds__(GfCfg<T, DP, EC, LPC, CPT, TC, WHOLE>::THREADS) gla_fast_kernel(TpxGla p) {
+__global__ void __launch_bounds__(GfCfg<T, DP, EC, LPC, CPT, TC, WHOLE>::THREADS, GfCfg<T, DP, EC, LPC, CPT, TC, WHOLE>::BLOCKS) gla_fast_kernel(TpxGla p) {
   using C = GfCfg<T, DP, EC, LPC, CPT, TC, WHOLE>;
   constexpr bool F32 = sizeof(T) == 4;
   constexpr int KV = C::KPT / 4, KP = C::KPT / 2, M = C::M;
@@ -547,7 +551,8 @@ __global__ void __launch_bounds__(GfCfg<T, DP, EC, LPC, CPT, TC, WHOLE>::THREADS
         float w[M];
         gl_ld<M>(rv + (blk * 4 + u) * EC + c0 + c, w);
 #pragma unroll
-        for (int i = 0; i < M; i++) r[i] = fmaf(dd[u], w[i], r[i]);
+        for (int i = 0; i < M; i++)
+          if (!F32 || u <= t) r[i] = fmaf(dd[u], w[i], r[i]);  // an infinity or NaN of a later token stays there; in bf16 mode it reaches the tokens of its four
       }
       if (WHOLE) gl_st_f32<M>(s_o + (blk * 4 + t) * EC + c0 + c, r);
       else if (blk * 4 + t < n && c0 + c < cols) gl_st_f32<M>(p.raw + ((row0 + t0 + blk * 4 + t) * p.heads + head) * vdim + e0 + c0 + c, r);
