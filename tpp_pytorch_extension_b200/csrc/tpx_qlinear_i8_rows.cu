@@ -48,11 +48,6 @@ __device__ __forceinline__ void ir_quantize(const I8RowsParams& p, uint32_t xs, 
       if (r * THREADS + tid < nv) rows_prefetch_gamma(p.gamma, p.gamma_f32, r * THREADS + tid);
   }
   pdl_wait();
-  if (p.gamma) {
-#pragma unroll
-    for (int r = 0; r < 2; r++)
-      if (r * THREADS + tid < nv) i8_gamma(p.gamma, p.gamma_f32, r * THREADS + tid, gm[r]);
-  }
   for (int q0 = 0; q0 < nv; q0 += 2 * THREADS) {  // with the norm (at most 8192 values) once
     uint4 v[2][2];
 #pragma unroll
@@ -64,6 +59,9 @@ __device__ __forceinline__ void ir_quantize(const I8RowsParams& p, uint32_t xs, 
       }
     float inv[2] = {};
     if (p.gamma) {
+#pragma unroll
+      for (int r = 0; r < 2; r++)
+        if (r * THREADS + tid < nv) i8_gamma(p.gamma, p.gamma_f32, r * THREADS + tid, gm[r]);
 #pragma unroll
       for (int m = 0; m < 2; m++) {
         float ss = 0.0f;

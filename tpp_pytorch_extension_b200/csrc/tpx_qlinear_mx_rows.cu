@@ -236,7 +236,6 @@ __global__ void __launch_bounds__(MrCfg<T, MG, MODE>::W * 32, 1) qlinear_mx_rows
     if (MODE == kMrNorm)
       for (int q = threadIdx.x; q * 8 < p.t.K; q += C::W * 32) rows_prefetch_gamma(p.gamma, p.gamma_f32, q);
     pdl_wait();
-    if (MODE == kMrNorm && (int)threadIdx.x * 8 < p.t.K) mr_gamma(p.gamma, p.gamma_f32, threadIdx.x, gm);
 #pragma unroll
     for (int m = 0; m < 8; m++) ss[m] = 0.0f;
     for (int q0 = 0; q0 < pieces; q0 += C::W * 32) {
@@ -245,6 +244,7 @@ __global__ void __launch_bounds__(MrCfg<T, MG, MODE>::W * 32, 1) qlinear_mx_rows
 #pragma unroll
       for (int m = 0; m < 8; m++)
         if (m < M) v[m] = load(q, m);
+      if (MODE == kMrNorm && q0 == 0 && q * 8 < p.t.K) mr_gamma(p.gamma, p.gamma_f32, q, gm);
 #pragma unroll
       for (int m = 0; m < 8; m++)
         if (m < M) {
@@ -362,6 +362,12 @@ __global__ void __launch_bounds__(kMpThreads) mx_rows_prep_kernel(MxRowsParams p
   if (NORM)
     for (int q = q0; q * 8 < p.t.K; q += kMpThreads) rows_prefetch_gamma(p.gamma, p.gamma_f32, q);
   pdl_wait();
+  uint4 x[V];
+#pragma unroll
+  for (int v = 0; v < V; v++) {
+    const int q = q0 + v * kMpThreads;
+    x[v] = q * 8 < p.t.K ? rows_ldg16(p.x + (size_t)m * p.t.K + q * 8) : make_uint4(0, 0, 0, 0);
+  }
   float gm[V][8];
   if (NORM)
 #pragma unroll
@@ -369,12 +375,6 @@ __global__ void __launch_bounds__(kMpThreads) mx_rows_prep_kernel(MxRowsParams p
       const int q = q0 + v * kMpThreads;
       if (q * 8 < p.t.K) mr_gamma(p.gamma, p.gamma_f32, q, gm[v]);
     }
-  uint4 x[V];
-#pragma unroll
-  for (int v = 0; v < V; v++) {
-    const int q = q0 + v * kMpThreads;
-    x[v] = q * 8 < p.t.K ? rows_ldg16(p.x + (size_t)m * p.t.K + q * 8) : make_uint4(0, 0, 0, 0);
-  }
   float inv = 1.0f;
   if (NORM) {
     float ss = 0.0f;
