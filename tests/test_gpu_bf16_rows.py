@@ -1,5 +1,5 @@
 """bf16 linear of few tokens at the edges of its splits: one to twenty tiles per CTA, features and k that end inside a tile, clusters, groups of tokens, padded
-leading dimensions; and a recorded chain of calls. Reference: 64 bits."""
+leading dimensions, every epilogue; a recorded chain of calls; a result over its own activations. Reference: 64 bits."""
 import pytest
 import torch
 
@@ -26,8 +26,51 @@ def test_plain_and_strided(M, N, K):
     bound = 2.0 ** -8 * want.abs() * (1 + 2.0 ** -6) + err * mul.double().abs() + 2.0 ** -22 * (size * mul.double().abs() + res.double().abs())
     assert bool(((y.double() - want).abs() <= bound).all())
     # rows of a wider matrix, fp32 result
-    out = HL.linear(x, wide[:, :K], out_f32=True) if wide.stride(0) % 8 == 0 else HL.linear(x, w, out_f32=True)
+    out = HL.linear(x, wide[:, :K], out_f32=True)
     assert bool(((out.double() - sums).abs() <= err + 2.0 ** -23 * size).all())
+
+
+# 96 features of 4104 values: a cluster cuts k; 2390: the last CTA has few of its own, and the gated units start inside a CTA's tiles
+@pytest.mark.parametrize("M", [1, 8, 9, 17, 32])
+@pytest.mark.parametrize("N,K,act_from", [(96, 4104, 0), (98, 4104, 42), (2390, 200, 1002), (4768, 72, 4766), (7130, 328, 7130), (28400, 128, 10000)])
+def test_gated_units(M, N, K, act_from):
+    from tpp_pytorch_extension_b200._C import _hybrid_layers as HL
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    x, w, bias, limit = rnd(M, K).to(torch.bfloat16), (rnd(N, K) * 3 * K ** -0.5).to(torch.bfloat16), rnd(N), 2.5
+    units = (N - act_from) // 2
+    z = torch.full((M, units + 3), 7.0, device="cuda", dtype=torch.bfloat16)
+    y = HL.linear_glu(x, w, bias, act_from, limit, z)
+    v, err = x.double() @ w.double().T + bias.double(), (K // 16 + 40) * 2.0 ** -23 * (x.double().abs() @ w.double().abs().T + bias.double().abs())
+    assert bool(((y.double() - v[:, :act_from]).abs() <= 2.0 ** -8 * v[:, :act_from].abs() + err[:, :act_from] * 2).all())
+    a, b, ea, eb = v[:, act_from::2], v[:, act_from + 1::2], err[:, act_from::2], err[:, act_from + 1::2]
+    gate, up = a.clamp(max=limit), b.clamp(-limit, limit) + 1
+    act = gate * torch.sigmoid(1.702 * gate)  # its slope is below 1.1; fast exponential and division, 2^-18 of the value
+    want = act * up
+    bound = 2.0 ** -8 * want.abs() * (1 + 2.0 ** -6) + (1.1 * ea + 2.0 ** -18 * act.abs()) * up.abs() + (act.abs() + 1.1 * ea) * eb
+    assert bool(((z[:, :units].double() - want).abs() <= bound).all())
+    assert bool((z[:, units:] == 7).all())
+
+
+@pytest.mark.parametrize("M", [1, 8, 9, 17, 32])
+@pytest.mark.parametrize("N,K", [(96, 4104), (100, 4104), (2390, 200), (4768, 72), (28400, 128)])
+@pytest.mark.parametrize("extra", [False, True])
+def test_residual_and_norm(M, N, K, extra):
+    from tpp_pytorch_extension_b200._C import _hybrid_layers as HL
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    x, w = rnd(M, K).to(torch.bfloat16), (rnd(N, K) * K ** -0.5).to(torch.bfloat16)
+    res, add, nw, nb, alpha = rnd(M, N), rnd(N) if extra else None, rnd(N), rnd(N), 0.7
+    s, h = HL.linear_residual(x, w, res, add, (alpha, nw, nb))
+    v = x.double() @ w.double().T
+    want = res.double() + v + (add.double() if extra else 0)
+    err = (K // 16 + 40) * 2.0 ** -23 * (x.double().abs() @ w.double().abs().T) + 2.0 ** -23 * (res.double().abs() + v.abs() + (add.double().abs() if extra else 0))
+    assert bool(((s.double() - want).abs() <= err).all())
+    t = torch.tanh(alpha * want)
+    want = t * nw.double() + nb.double()
+    # tanh to 2^-21, its slope at most 1, the product and sum rounded once
+    bound = 2.0 ** -8 * want.abs() * (1 + 2.0 ** -6) + (alpha * err + 2.0 ** -21) * nw.double().abs() + 2.0 ** -23 * want.abs()
+    assert bool(((h.double() - want).abs() <= bound).all())
 
 
 @pytest.mark.parametrize("M", [1, 16, 24])
