@@ -746,7 +746,7 @@ def run_ours(args):
                 M = SWEEP[mi]
                 wg, wu, wd = sets[counter[0] % N_COPIES]
                 counter[0] += 1
-                # the public ops take the pinned host buffers themselves: the activation-split kernel reads X across
+                # the public ops take the pinned host buffers themselves: the kernel that converts the activations reads X across
                 # the bus, the down projection's epilogue writes Y to host memory (no separate copies in the stream)
                 F.fc_plain(F.fc_gate_up(xs_host[M], wg, wu), wd, out=ys_host[M])
         eb.record(cur)
@@ -806,7 +806,7 @@ def run_ours(args):
                          "achieved": dom_gbs, "peak": pk["hbm_gbs"], "unit": "GB/s", "frac": dom_gbs / pk["hbm_gbs"],
                          "peak_src": pk["src"], "traffic": NCU_TRAFFIC.get(SWEEP[dom]),
                          "traffic_src": "ncu capture summarised under profiles/, not measured in this run",
-                         "duration": "CUDA events around K back-to-back launches of the op (activation-split kernel + GEMM kernel each), divided by K"},
+                         "duration": "CUDA events around K back-to-back launches of the op (the GEMM, with the conversion of the activations in it or in a kernel in front), divided by K"},
             "kernels": kernels,
             "e2e": {"value": e2e_value, "unit": "GB/s",
                     "h2d_bytes_per_step": sum(SWEEP[i] * D_MODEL * 2 for i in dec),

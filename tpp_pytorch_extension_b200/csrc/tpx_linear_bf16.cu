@@ -20,7 +20,7 @@
 // cut are added in the order of k by the CTA that finishes last (fp32 partials and an arrival counter in the scratch; no
 // CTA waits for another). Two accumulators in tensor memory: the
 // epilogue of a tile runs under the MMAs of the next. Up to 32 tokens it has only the largest weights: the others stream
-// through the warps' own rings (tpx_linear_bf16_rows.cu), where a call of 4096 x 4096 takes 7.2 us instead of 13.6.
+// through the warps' own rings (tpx_linear_bf16_rows.cu), where a call of 4096 x 4096 takes 6.9 us instead of 13.2.
 #include "tpx_bf16_pair.cuh"
 
 namespace tpx {

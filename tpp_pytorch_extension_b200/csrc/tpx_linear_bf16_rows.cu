@@ -1,13 +1,14 @@
 // bf16 linear of few tokens: the weight streams through private rings of every warp, mma.sync beside it. Same results as linear_bf16_kernel
 // (tpx_linear_bf16.cu) up to the order of its fp32 sums, all its epilogues.
 //
-// Bound by HBM. A CTA has T tiles of 16 features (T: one round of CTAs) and all of K; its KG groups of warps take the 64-wide k blocks (a 128-byte line of a row) in
+// A large weight comes at 0.88 to 0.94 of HBM's rate at one token, 0.80 to 0.88 at 16; a small one (4096 x 4096 0.74, 2048 x 2048 0.43) is a launch's start and end in the chain and
+// the wait for the first activations. A CTA has T tiles of 16 features (T: one round of CTAs) and all of K; its KG groups of warps take the 64-wide k blocks (a 128-byte line of a row) in
 // turn, H warps of a group N tiles each. A lane copies (cp.async) exactly the 16-byte pieces that it feeds to its MMAs, k being permuted inside a block
 // for both operands: no barrier in the loop, 25 instructions per 2 KB. Activations come straight from L2 to registers, a block ahead. The tcgen05 form streams a
 // large weight as fast, but a decode step is a chain of small ones, and there it pays for tensor memory, tensor maps, tiles of 128 features cut between CTAs and put
-// together over memory. Chains of calls, us, tcgen05 / here (floor), 1 and 16 tokens:
-// 2048 x 2048 8.4 / 3.2 and 8.4 / 4.2 (1.3), 4096 x 4096 13.6 / 7.2 and 13.5 / 8.3 (5.2), 4096 x 14336 26.8 / 20.7 and 27.9 / 22.5 (18.1), 14336 x 4096 27.1 / 21.9
-// and 26.6 / 24.8, 32000 x 4096 48.5 / 45.6 (40.3); 24 tokens 4096 x 4096 18.4 / 9.8.
+// together over memory. Recorded chains of calls, us, tcgen05 / here (floor), 1 and 16 tokens: 2048 x 2048 8.2 / 3.0 and 8.2 / 3.8 (1.3), 4096 x 4096 13.2 / 6.9 and
+// 13.4 / 8.1 (5.1), 4096 x 14336 25.6 / 19.2 and 25.5 / 21.1 (18.0), 14336 x 4096 25.2 / 20.4 and 25.4 / 22.5, 32000 x 4096 44.9 / 42.6 and 45.3 / 45.5 (40.1); 24 tokens
+// 4096 x 4096 18.0 / 9.5.
 #include "tpx_bf16_pair.cuh"
 #include "tpx_rows.cuh"
 

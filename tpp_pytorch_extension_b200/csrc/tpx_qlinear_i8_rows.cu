@@ -2,15 +2,16 @@
 //
 // Arithmetic of qlinear_i8_kernel (tpx_qlinear_i8.cu): int8 x int8 -> int32 per block of 64 k values, times s_x * s_w, added in fp32.
 //
-// Bound by HBM up to 16 tokens (every weight byte is used once), above by the instructions per weight byte. A CTA has T tiles of 16 features
+// Every weight byte is read once, which is 0.73 of a call of 11008 x 4096 at one token, 0.55 at 16 and 0.44 at 32 (7.3 us of HBM); the rest is a launch's start and end
+// in the chain, the wait for the activations and, above 16 tokens, the instructions per weight byte (43 % of issue slots at 32). A CTA has T tiles of 16 features
 // and all of K; its groups of warps take the 64-wide k blocks in turn, two neighbours (128 bytes of a row) at a time. A warp's weights come by
 // cp.async into a ring of its own, each lane copying exactly the 16-byte pieces that it feeds to its MMAs: no barrier of the CTA in the loop,
 // 100 to 200 KB per SM on the way, the first of them before the wait for the previous kernel. k is permuted inside a block (a lane's MMA slots
 // are 16 consecutive values), which both operands share, so the plain row-major weight needs no repacking. Quantised activations come straight
 // from L2 to registers, a block ahead; one or two tokens every CTA quantises for itself. The tcgen05 form has a chain per 256 k values (copies, MMAs, drain of int32 accumulators from tensor memory)
 // on whole tiles of 128 features; here the drain is three packed fp32 operations per two sums in the registers where the MMA left them.
-// With the quantisation of x, a chain of calls on one B200, tcgen05 form / here: 11008 x 4096 (7.4 us of HBM) 1 token 16.4 / 11.8 us, 16: 16.4 / 13.6,
-// 32: 18.8 / 17.4; 4096 x 4096 10.2 / 5.7 at 1, 12.6 / 8.9 at 32; the pair 2 x 11008 x 4096 at 1 token 31.8 / 19.4 (one kernel instead of two).
+// With the quantisation of x, recorded chains of calls on one B200, tcgen05 form / here: 11008 x 4096 1 token 15.6 / 10.0 us, 16: 15.8 / 13.2, 32: 18.1 / 16.7; 4096 x 4096
+// 9.8 / 5.4 at 1, 12.2 / 8.5 at 32; the pair 2 x 11008 x 4096 at 1 token 30.7 / 16.8 (one kernel instead of two).
 #include "tpx_qlinear_i8_rows.cuh"
 #include "tpx_rows.cuh"
 
@@ -18,7 +19,7 @@ namespace tpx {
 
 constexpr int kIrSlot = 1088;  // 16 features x 64 values and the 16 scales
 // A warp's ring holds D k blocks of its tiles: every address in the loop over D blocks is a constant offset. Sixteen warps hide the latencies (with eight, 11008 x 4096 took 18.4 us at
-// 16 tokens, now 14.1); above 16 tokens the sums and the activations of the next block need the registers of twelve (18.2 / 17.2 us).
+// 16 tokens, with sixteen 14.1); above 16 tokens the sums and the activations of the next block need the registers of twelve (18.2 / 17.2 us).
 template <int T, int MG>
 struct IrCfg : RowsSplit<T, MG, MG == 4 ? 12 : 16, MG == 4 ? 3 : 4> {
   using S0 = RowsSplit<T, MG, MG == 4 ? 12 : 16, MG == 4 ? 3 : 4>;
@@ -286,9 +287,11 @@ bool i8_rows_serves(int64_t M, int64_t N, int64_t block, bool pair) {
   return block == 64 && (M <= 16 || (M <= 32 && !pair && rows_tiles(N / 16) < 7));
 }
 
-// One and two tokens: in every CTA, which costs less than the launch in front. Generation of 40 tokens behind 64, 8 layers of 4096 x 11008: 1 token 24.0 ms, from
-// 26.2 with a kernel in front; 2 tokens 26.5 (26.7 with only the norms in here, 27.9 with none). Calls in a chain at 1 token, without a norm: 11008 x 4096 11.9 -> 10.6 us, 4096 x
-// 11008 11.9 -> 11.5, 4096 x 4096 5.7 -> 5.9; at 2 tokens 11.8 -> 11.2, 12.1 -> 12.8, 5.7 -> 6.3. A norm in front is a kernel of 5 us, in here of about one.
+// One and two tokens: in every CTA. Recorded chains of calls, us, a kernel in front / in here. 1 token: 4096 x 4096 5.3 / 5.4, 6144 x 4096 8.1 / 7.1, 11008 x 4096
+// 11.5 / 10.1, 4096 x 11008 11.4 / 10.8, the pair of 11008 x 4096 18.2 / 16.8; behind a norm 7.4 / 6.8, 10.3 / 8.0, 13.8 / 11.2, the pair 21.0 / 18.0. 2 tokens: 6144 x 4096 8.2 / 7.5,
+// 11008 x 4096 11.3 / 10.5, the pair 18.3 / 17.3, behind a norm 7.6 / 7.3, 10.3 / 8.6, 13.6 / 11.7, 20.9 / 18.5; only with two tiles per CTA and no norm is the kernel in front
+// ahead, 4096 x 4096 5.4 / 5.9, 4096 x 11008 11.5 / 12.0, by less than a launch costs a caller of single linears: a generation of two sequences, 8 layers of 4096 x 11008,
+// takes 26.8 ms either way.
 bool i8_rows_quantizes(const void* x, const void* y, int64_t M, int64_t N, int64_t K) {
   return M <= 2 && M * K <= kIrStaged && rows_shared_x(x, (size_t)M * K * 2, y, (size_t)M * N * 2);
 }

@@ -421,10 +421,12 @@ static int mr_launch_mode(const MxRowsParams& p, cudaStream_t st) {
 
 template <int T, bool DUAL>
 static int mr_launch(MxRowsParams p, uint8_t* scratch, cudaStream_t st) {
-  // By every CTA while that costs about what the launch in front would, which a caller of single linears pays for as well: one weight up to 20480 values (4096 x
-  // 4096 at 1, 4 and 8 tokens 4.7, 5.3 and 6.2 us, by a kernel in front 5.0, 5.0, 5.1; 4096 x 14336 at 4 tokens 12.4 / 9.8), a pair of more than eight tiles 8 tokens
-  // of 4096 (14336 x 4096 at 1 and 8 tokens 14.7 and 16.8, 15.9 and 16.0), behind a norm 2 tokens of 4096 (the same pair 15.9 and 20.8, 15.8 and 16.3). Activations in the
-  // host's memory are read once, and those that the result replaces before it is written.
+  // By every CTA while that costs about what the launch in front does, which a caller of single linears pays for as well: one weight up to 20480 values, a pair of more than
+  // eight tiles 8 tokens of 4096, behind a norm 2 tokens of 4096. Recorded chains, us, a kernel in front / by every CTA: 4096 x 4096 at 1, 2, 4 and 5 tokens 4.7 / 4.4, 4.5 / 4.7,
+  // 4.6 / 5.0 and 4.6 / 5.2, 6144 x 4096 5.6 / 5.1, 5.6 / 5.3, 5.7 / 5.7 and 5.7 / 5.9, 2048 x 2048 3.2 / 2.4, 3.3 / 2.6, 3.3 / 3.0 and 3.1 / 3.1, 4096 x 14336 at 1 token
+  // 9.6 / 10.5; the pair of 14336 x 4096 at 1, 4 and 8 tokens 14.4 / 13.7, 14.7 / 14.5 and 15.3 / 15.9, behind a norm at 1 and 2 tokens 15.7 / 15.0 and 15.8 / 15.6. Launched one by
+  // one, the launches count for more: an MLP of 8 tokens 29.5 / 27.5 us, a generation of 40 tokens on the Llama-3 shape 21.3 / 20.8 ms with limits after the recorded chains
+  // (12288 values, 4096 with two tiles per CTA, 20480 of a pair). Activations in the host's memory are read once, and those that the result replaces before it is written.
   const long long values = (long long)p.steps * 128 * p.t.M;
   if (p.t.M <= (p.gamma ? 2 : 8) && values <= (p.gamma ? 8192 : T > 8 ? 32768 : 20480) &&
       rows_shared_x(p.x, (size_t)p.t.M * p.t.K * 2, p.t.y, (size_t)p.t.M * p.t.N * 2))

@@ -1,4 +1,4 @@
-// What the kernels for few tokens share (tpx_qlinear_i8_rows.cu, tpx_qlinear_mx_rows.cu): weights copied by each warp into a ring of its own, activations
+// What the kernels for few tokens share (tpx_qlinear_i8_rows.cu, tpx_qlinear_mx_rows.cu, tpx_linear_bf16_rows.cu): weights copied by each warp into a ring of its own, activations
 // straight from L2, tiles of 16 features.
 #pragma once
 #include "tpx_tc_ptx.cuh"
