@@ -195,7 +195,7 @@ int tpx_linear_bf16_tc(const uint16_t* w, const uint16_t* x, int64_t M, int64_t 
                        size_t scratch_bytes, void* stream);
 
 /* ---------------------------------------------------------------- int8 linear on the tcgen05 tensor cores
- * Any number of tokens (blocks of 64 and up to 32 tokens: a kernel that streams the weight
+ * Any number of tokens (blocks of 64 and up to 32 tokens: at most sizes a kernel that streams the weight
  * through registers; else tiles of 16, 32, 64 or 128 tokens x 128 features) with the reference's own int8 arithmetic
  * (TppBlockedQInt8LinearW, src/csrc/fused_gemm.h:1075-1341):
  * the activations are quantised on the fly to int8 with one scale per (token, K block) (:1249), each K block is an

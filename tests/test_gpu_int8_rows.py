@@ -19,9 +19,11 @@ def _weight(N, K, g):
     return q, s, wq, sw
 
 
-# 16 features: a cluster of eight where K allows it; 149, 297, ... tiles: the last CTA has one of its own; 1037 tiles: two rounds
+# 16 features: a cluster of eight where K allows it; 149, 297, ... tiles: the last CTA has one of its own; 1037 and 1193 tiles: two rounds; the last five
+# as long as five, six and seven tiles per CTA and two rounds have to be for more than 8 and 16 tokens
 @pytest.mark.parametrize("M", [1, 8, 9, 16, 17, 32])
-@pytest.mark.parametrize("N,K", [(16, 64), (16, 16448), (1040, 1024), (2384, 192), (4752, 2112), (7120, 320), (9488, 576), (11856, 448), (14224, 704), (16592, 1024)])
+@pytest.mark.parametrize("N,K", [(16, 64), (16, 16448), (1040, 1024), (2384, 192), (4752, 2112), (7120, 320), (9488, 576), (11856, 448), (14224, 704), (16592, 1024), (9488, 1600),
+                                 (11856, 3136), (14224, 4160), (19088, 320), (19088, 1600)])
 def test_linear_and_pair(M, N, K):
     from tpp_pytorch_extension_b200 import _lib
     L = _lib.lib()
@@ -130,9 +132,9 @@ def test_result_over_activations(M, monkeypatch):
         assert torch.equal(y, want)
 
 
-# 272 and 14224 features: 17 and 889 tiles of 16, which different kernels take at 17 to 32 tokens; 320: half a step of 128 k values left over
+# 272, 14224 and 17408 features: 17, 889 and 1088 tiles of 16, which different kernels take above 8, 16 and 2 tokens; 320: half a step of 128 k values left over
 @pytest.mark.parametrize("M", [1, 2, 8, 16, 17, 24, 32, 33])
-@pytest.mark.parametrize("first,second", [(272, 14224), (14224, 272), (272, 272)])
+@pytest.mark.parametrize("first,second", [(272, 14224), (14224, 272), (272, 17408), (17408, 272), (272, 272)])
 @pytest.mark.parametrize("K", [320, 4096])
 def test_reuse_across_sizes(M, first, second, K):
     from tpp_pytorch_extension_b200 import _lib

@@ -294,7 +294,7 @@ qlinear_i8_kernel(const __grid_constant__ CUtensorMap tmW, I8Params p) {
     // ------------------------------------------------------------ MMA issuer
     // kind::i8: D = S32 (2), A = B = S8 (1), both K-major, N = TOK, M = 128
     constexpr uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TOK >> 3) << 17) | ((128u >> 4) << 24);
-    constexpr bool HALF = I8Act32::serves(TOK, BS * 32);  // the B operand has a block's rows of 64 bytes
+    constexpr bool HALF = I8Act64::serves(TOK, BS * 32);  // the B operand has a block's rows of 64 bytes
     const uint64_t desc0 = tc_smem_desc(smem_base), bdesc0 = HALF ? tc_smem_desc64(smem_base + C::A_BYTES) : tc_smem_desc(smem_base + C::A_BYTES);
     int s = 0, g = 0;  // g: groups handed out
     uint32_t phase = 0;
@@ -528,9 +528,8 @@ static int i8_launch(const CUtensorMap& w, I8Params p, int tiles, cudaStream_t s
 
 template <int BS>
 static int i8_launch_tok(int tokp, const CUtensorMap& w, const I8Params& p, int tiles, cudaStream_t st) {
-  if constexpr (BS > 2)  // up to 16 tokens, blocks of 64 are tpx_qlinear_i8_rows.cu's
-    if (tokp == 16) return i8_launch<16, BS>(w, p, tiles, st);
   switch (tokp) {
+    case 16: return i8_launch<16, BS>(w, p, tiles, st);
     case 32: return i8_launch<32, BS>(w, p, tiles, st);
     case 64: return i8_launch<64, BS>(w, p, tiles, st);
     default: return i8_launch<128, BS>(w, p, tiles, st);
@@ -626,7 +625,7 @@ static int i8_linear(const int8_t* wq, const float* swT, const int8_t* wq2, cons
               scratch_bytes);
   TPX_REQUIRE(!gamma || (K <= 8192 && block_size <= 256 && ((uintptr_t)gamma & 15) == 0), TPX_ERR_UNSUPPORTED,
               "qlinear_qint8_tc: the fused RMSNorm takes rows of up to 8192 values, blocks of up to 256 and a 16-byte aligned gamma");
-  if (wq2 && !i8_rows_serves(M, N, block_size, true)) {
+  if (wq2 && !i8_rows_serves(M, N, K, block_size, true)) {
     int rc = i8_linear(wq, swT, nullptr, nullptr, x, gamma, gamma_is_f32, eps, M, N, K, block_size, reuse_act, bias, act, nullptr, nullptr, 1.0f, y,
                        scratch, scratch_bytes, stream);
     if (rc) return rc;
@@ -640,19 +639,17 @@ static int i8_linear(const int8_t* wq, const float* swT, const int8_t* wq2, cons
   t.bias = bias; t.mul_in = mul_in; t.res = res; t.res_scale = res_scale; t.y = y; t.act = act;
   t.M = (int)M; t.N = (int)N; t.K = (int)K; t.cluster = pl.cluster;
   t.err = reinterpret_cast<unsigned*>(sc + kTcCounterBytes - 4);
-  const bool rows = i8_rows_serves(M, N, block_size, wq2 != nullptr);
+  const bool rows = i8_rows_serves(M, N, K, block_size, wq2 != nullptr);
   I8RowsParams r = {};
   // The order of the quantised activations depends on M, K and block_size alone, so that a call that reuses them may be of another N, and another kernel's.
   const I8Act L(pl.tokp, pl.ksteps, (int)block_size);
   if (!reuse_act && rows && i8_rows_quantizes(x, y, M, N, K)) {
     r.x = x; r.gamma = gamma; r.gamma_f32 = gamma_is_f32; r.eps = eps;
-  } else if (!reuse_act && rows && M <= 16) {
-    int rc = i8_quantize(x, gamma, gamma_is_f32, eps, (int)M, (int)M, K, I8Rows((int)M, K), xq, st);
-    if (rc) return rc;
   } else if (!reuse_act && block_size <= 256) {
     if (!rows && pl.Kp != K) TPX_CUDA_OK(cudaMemsetAsync(xq, 0, pl.xq_bytes, st));  // the k padding reads as zero, as the weight's
-    int rc = I8Act32::serves(pl.tokp, (int)block_size) ? i8_quantize(x, gamma, gamma_is_f32, eps, (int)M, 32, K, I8Act32(), xq, st)
-                                                       : i8_quantize(x, gamma, gamma_is_f32, eps, (int)M, (int)pl.Mp, K, L, xq, st);
+    int rc = I8Act64::serves(pl.tokp, (int)block_size)
+                 ? i8_quantize(x, gamma, gamma_is_f32, eps, (int)M, rows ? (int)M : pl.tokp, K, I8Act64{(uint32_t)pl.tokp}, xq, st)
+                 : i8_quantize(x, gamma, gamma_is_f32, eps, (int)M, (int)pl.Mp, K, L, xq, st);
     if (rc) return rc;
   } else if (!reuse_act) {
     const long long warps = (long long)pl.Mp * (K / 512);
@@ -662,7 +659,7 @@ static int i8_linear(const int8_t* wq, const float* swT, const int8_t* wq2, cons
   if (rows) {
     r.t = t;
     r.w[0] = wq; r.w[1] = wq2; r.swT[0] = swT; r.swT[1] = swT2; r.xq = xq;
-    r.nkb = (int)(K / 64); r.Mp = I8Rows((int)M, K).Mp; r.Kp = (int)pl.Kp; r.Np = (int)pl.Np; r.tiles = (int)(N / 16);
+    r.nkb = (int)(K / 64); r.Kp = (int)pl.Kp; r.Np = (int)pl.Np; r.tiles = (int)(N / 16);
     return i8_rows_launch(r, wq2 != nullptr, st);
   }
   CUtensorMap mw;

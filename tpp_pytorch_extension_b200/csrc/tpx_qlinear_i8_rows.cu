@@ -105,8 +105,9 @@ __device__ __forceinline__ void ir_quantize(const I8RowsParams& p, uint32_t xs, 
         asm volatile("st.shared.v2.u32 [%0], {%1,%2};" ::"r"(xs + (uint32_t)((blk * M + m) * 64 + (q & 7) * 8)), "r"(o.x), "r"(o.y) : "memory");
         if ((q & 7) == 0) asm volatile("st.shared.f32 [%0], %1;" ::"r"(fs + (uint32_t)(blk * M + m) * 4), "f"(scale) : "memory");
         if (blockIdx.x == 0) {
-          *reinterpret_cast<uint2*>(p.xq + ((size_t)blk * p.Mp + m) * 64 + (q & 7) * 8) = o;
-          if ((q & 7) == 0) reinterpret_cast<float*>(p.xq + (size_t)p.nkb * p.Mp * 64)[(size_t)blk * p.Mp + m] = scale;
+          const I8Act64 L = {16};
+          *reinterpret_cast<uint2*>(L.value(p.xq, m, q * 8)) = o;
+          if ((q & 7) == 0) *L.scale(p.xq, m, blk) = scale;
         }
       }
   }
@@ -136,13 +137,11 @@ __global__ void __launch_bounds__(IrCfg<T, MG>::W * 32, 1) qlinear_i8_rows_kerne
   const char* const sb0 = reinterpret_cast<const char*>(p.swT[0] + tile0 * 16);
   const char* const sb1 = DUAL ? reinterpret_cast<const char*>(p.swT[1] + tile0 * 16) : nullptr;
   uint32_t w0 = f0 * row16 + g * p.Kp + t * 16 + turn * 128, s0 = turn * 8 * p.Np + f0 * 64 + lane * 16;
-  constexpr bool STEPS = MG == 4;  // activations I8Act32, as the tcgen05 kernel has them, which serves the same calls of other N
-  constexpr uint32_t kStepScales = 32 * 128, kStep = I8Act32::BYTES;
-  const uint32_t xrow = (QUANT ? p.t.M : p.Mp) * 64, xstep = groups * (STEPS ? kStep : 2 * xrow);
-  const uint8_t* const sxb = p.xq + (size_t)p.nkb * xrow;  // a scale is 4 bytes where its 64 values are 64
-  uint32_t x0 = turn * (STEPS ? kStep : 2 * xrow);
+  constexpr uint32_t TOK = MG == 4 ? 32 : 16;
+  const uint32_t xrow = p.t.M * 64, xpair = QUANT ? 2 * xrow : I8Act64::bytes(TOK), xstep = groups * xpair;  // QUANT: rows in shared memory, a block's after another's
+  uint32_t x0 = turn * xpair;
   const int last = p.t.M - 1;  // QUANT: columns behind the last token repeat it and are not stored
-  const uint32_t xl = STEPS ? g * 64 + (t ^ (g >> 1)) * 16 : (QUANT ? min(g, last) : g) * 64 + t * 16;
+  const uint32_t xl = QUANT ? min(g, last) * 64 + t * 16 : g * 64 + (t ^ (g >> 1)) * 16;
   const uint32_t xs = tc_smem_u32(ir_smem_raw) + (uint32_t)C::SMEM, fs = xs + p.nkb * xrow;
   pdl_trigger();
 
@@ -169,21 +168,16 @@ __global__ void __launch_bounds__(IrCfg<T, MG>::W * 32, 1) qlinear_i8_rows_kerne
   uint4 xv[2][MG];
   float2 sv[2][MG];
   auto fetch = [&](int z, int td) {
-    const uint32_t x = x0 + (td >> 1) * xstep + (STEPS ? 0 : (td & 1) * xrow);
-    if constexpr (STEPS) {
-#pragma unroll
-      for (int m = 0; m < MG; m++) {
-        xv[z][m] = rows_ldg16(p.xq + (x + xl + (td & 1) * 2048 + m * 512));
-        sv[z][m] = rows_ldg8(p.xq + (x + kStepScales + (td & 1) * 128 + t * 8 + m * 32));
-      }
-    } else if constexpr (QUANT) {
-      xv[z][0] = rows_lds16(xs + x + xl);
-      sv[z][0] = make_float2(rows_lds4(fs + x / 16 + min(2 * t, last) * 4), rows_lds4(fs + x / 16 + min(2 * t + 1, last) * 4));
+    const uint32_t x = x0 + (td >> 1) * xstep;
+    if constexpr (QUANT) {
+      const uint32_t xb = x + (td & 1) * xrow;
+      xv[z][0] = rows_lds16(xs + xb + xl);
+      sv[z][0] = make_float2(rows_lds4(fs + xb / 16 + min(2 * t, last) * 4), rows_lds4(fs + xb / 16 + min(2 * t + 1, last) * 4));
     } else {
 #pragma unroll
       for (int m = 0; m < MG; m++) {
-        xv[z][m] = rows_ldg16(p.xq + (x + xl + m * 512));
-        sv[z][m] = rows_ldg8(sxb + (x / 16 + t * 8 + m * 32));
+        xv[z][m] = rows_ldg16(p.xq + (x + xl + (td & 1) * (TOK * 64) + m * 512));
+        sv[z][m] = rows_ldg8(p.xq + (x + TOK * 128 + (td & 1) * (TOK * 4) + t * 8 + m * 32));
       }
     }
   };
@@ -281,10 +275,26 @@ static int ir_launch_t(const I8RowsParams& p, bool pair, int tf, cudaStream_t st
   }
 }
 
-// Blocks of 64, up to 32 tokens; a pair up to 16 (its two sums do not fit in registers above). Seven tiles per CTA leave too few warps per tile above 16
-// tokens: 14336 x 4096 at 32 tokens 21.0 us here, 19.7 on the tcgen05 kernel; six tiles (12288 x 4096) 18.7 / 19.3, one (2048 x 8192) 10.1 / 14.0.
-bool i8_rows_serves(int64_t M, int64_t N, int64_t block, bool pair) {
-  return block == 64 && (M <= 16 || (M <= 32 && !pair && rows_tiles(N / 16) < 7));
+// Blocks of 64, up to 32 tokens; a pair up to 16 (its two sums do not fit in registers above), where two tcgen05 linears never win. One weight: where the tcgen05 kernel's
+// tiles of 128 features fill its one wave of CTAs, it takes the same time for the largest N as for the smallest and for 16 tokens as for one, this kernel more with each. Chains, us,
+// tcgen05 / here:
+// up to 8 tokens only that wave's last part, which is two rounds here: 4 tokens of 18944 x 3584 15.9 / 17.5, of 17408 x 2048 11.0 / 11.3; 1 token 15.9 / 14.7 and 11.2 / 10.5, of 17408 x 256
+//   4.5 / 6.1; with two waves again 27392 x 4096 31.4 / 23.5, 37888 x 4096 34.3 / 32.0 (8 tokens);
+// 9 to 16 tokens: up to five tiles per CTA from 256 values on (11008 x 256 4.2 / 4.0, 9408 x 128 4.1 / 5.6), more tiles from 4096 on (14080 x 2048 9.9 / 10.7, 14336 x 2048 10.1 / 10.6,
+//   14336 x 4096 16.2 / 15.6, 15360 x 4096 16.6 / 16.2, 16384 x 4096 17.0 / 18.4; 12 tokens);
+// 17 to 32 tokens, fewer groups of warps: four tiles from 256 values on (9408 x 128 4.5 / 6.1, x 256 6.5 / 5.8), five from 1536 (11008 x 1024 7.4 / 8.2, x 1536 9.3 / 9.2), six from 3072
+//   (14080 x 2048 11.6 / 12.0, x 3072 14.9 / 14.8, 12288 x 4096 18.1 / 17.2), seven nowhere (14336 x 4096 19.7 / 21.0); more rounds where waves are badly filled (25600 x 5120, 200 tiles:
+//   42.0 / 36.6; 32000 x 4096, 250: 36.5 / 36.6; 37888 x 4096, 296: 38.6 / 45.4).
+bool i8_rows_serves(int64_t M, int64_t N, int64_t K, int64_t block, bool pair) {
+  if (block != 64 || M > 32) return false;
+  if (pair) return M <= 16;
+  const int64_t sms = sm_count(), tiles = N / 16, big = (N + 127) / 128, waves = (big + sms - 1) / sms;
+  const int T = rows_tiles(tiles);
+  const bool rounds = tiles > 7 * sms;
+  if (M <= 8) return !rounds || waves > 1 || (M <= 2 && K >= 1024);
+  if (M <= 16) return rounds ? waves > 1 : T <= 5 ? K >= 256 : K >= 4096 && 2 * tiles <= 13 * sms;
+  if (rounds) return T < 7 && 10 * big < 7 * waves * sms && K >= 1536;
+  return T <= 4 ? K >= 256 : T == 5 ? K >= 1536 : T == 6 && K >= 3072;
 }
 
 // One and two tokens: in every CTA. Recorded chains of calls, us, a kernel in front / in here. 1 token: 4096 x 4096 5.3 / 5.4, 6144 x 4096 8.1 / 7.1, 11008 x 4096

@@ -22,28 +22,20 @@ struct I8Act {
   }
 };
 
-// The same for a tile of 32 tokens in blocks of 64, which the kernel for few tokens reads where N lets it: the 32 rows of 64 bytes of one block, then the
-// other's, in the order of the 64-byte swizzle. The tile is the only one, so that places are found without a division (1 us of a linear of 32 tokens).
-struct I8Act32 {
-  static constexpr int B = 64, BYTES = 32 * 128 + 2 * 32 * 4;  // bytes per step
-  static __host__ __device__ constexpr bool serves(int tok, int block) { return tok == 32 && block == B; }
+// The same for up to 32 tokens in blocks of 64, one tile of TOK = 16 or 32, which the kernel for few tokens reads where the call is its: the TOK rows of 64 bytes of
+// one block, then the other's, in the order of the 64-byte swizzle, then the scales [2][TOK]. The 16 bytes that a lane of that kernel's MMAs takes from a token are one unit, and a
+// warp's 32 units (8 tokens) one run of 512 bytes; places are found without a division (1 us of a linear of 32 tokens).
+struct I8Act64 {
+  static constexpr int B = 64;
+  uint32_t TOK;
+  static __host__ __device__ constexpr bool serves(int tok, int block) { return tok <= 32 && block == B; }
+  static __host__ __device__ constexpr uint32_t bytes(uint32_t tok) { return tok * 136; }  // per step
   __device__ __forceinline__ uint8_t* value(uint8_t* xq, int tok, int k) const {
     const uint32_t u = k;
-    return xq + (u / 128 * BYTES + (u % 128 / 64 * 32 + tok) * 64 + ((u % 64 / 16) ^ (((uint32_t)tok >> 1) & 3)) * 16 + u % 16);
+    return xq + (u / 128 * bytes(TOK) + (u % 128 / 64 * TOK + tok) * 64 + ((u % 64 / 16) ^ (((uint32_t)tok >> 1) & 3)) * 16 + u % 16);
   }
   __device__ __forceinline__ float* scale(uint8_t* xq, int tok, int blk) const {
-    return reinterpret_cast<float*>(xq + ((uint32_t)blk / 2 * BYTES + 32 * 128)) + (blk & 1) * 32 + tok;
-  }
-};
-
-// Of up to 16 tokens, blocks of 64 values: [K/64][Mp][64] int8, then the scales [K/64][Mp]. The 16 bytes that a lane of the kernel's MMAs
-// takes from a token are one piece, and a warp's 32 pieces (8 tokens) are one run of 512 bytes.
-struct I8Rows {
-  int Mp, nkb, B;  // tokens, padded to what a kernel reads; k blocks; B = 64, the scale block, as in I8Act
-  __host__ __device__ I8Rows(int M, int64_t K) : Mp(M <= 8 ? 8 : 16), nkb((int)(K / 64)), B(64) {}
-  __device__ __forceinline__ uint8_t* value(uint8_t* xq, int tok, int k) const { return xq + ((size_t)(k / 64) * Mp + tok) * 64 + k % 64; }
-  __device__ __forceinline__ float* scale(uint8_t* xq, int tok, int blk) const {
-    return reinterpret_cast<float*>(xq + (size_t)nkb * Mp * 64) + (size_t)blk * Mp + tok;
+    return reinterpret_cast<float*>(xq + ((uint32_t)blk / 2 * bytes(TOK) + TOK * 128)) + (blk & 1) * TOK + tok;
   }
 };
 
@@ -92,15 +84,15 @@ struct I8RowsParams {
   TcParams t;                // epilogue fields (bias, act, mul_in, res, res_scale, y, M, N)
   const int8_t* w[2];        // plain int8 weight [Np][Kp]; of a pair: gate, up
   const float* swT[2];       // [K/64][Np]
-  uint8_t* xq;               // I8Rows; of more than 16 tokens I8Act32
+  uint8_t* xq;               // I8Act64
   const uint16_t* x;         // or, if not null: bf16 activations, to be quantised (behind an RMSNorm if gamma is set) and left in xq as well
   const void* gamma;
   int gamma_f32;
   float eps;
-  int nkb, Mp, Kp, Np, tiles;  // tiles: N / 16
+  int nkb, Kp, Np, tiles;  // k blocks; N / 16
 };
 
-bool i8_rows_serves(int64_t M, int64_t N, int64_t block, bool pair);
+bool i8_rows_serves(int64_t M, int64_t N, int64_t K, int64_t block, bool pair);
 bool i8_rows_quantizes(const void* x, const void* y, int64_t M, int64_t N, int64_t K);  // whether the launch takes x instead of xq
 int i8_rows_launch(I8RowsParams p, bool pair, cudaStream_t st);  // sets t.cluster
 
