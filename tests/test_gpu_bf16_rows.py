@@ -6,9 +6,11 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-# 16 and 100 features: clusters; 2390 and more: 150, 300, ... tiles, the last CTA with few of its own; 47200: twenty per CTA
+# 16 and 100 features: clusters; 2390 and more: 150, 300, ... tiles, the last CTA with few of its own; 47200: twenty per CTA; 1032 values: as long
+# as five to eight tiles per CTA have to be above 16 tokens
 @pytest.mark.parametrize("M", [1, 8, 9, 16, 17, 32])
-@pytest.mark.parametrize("N,K", [(16, 8), (100, 4104), (2390, 200), (4768, 72), (7130, 328), (9504, 136), (11872, 64), (14240, 192), (18950, 248), (28400, 128), (47200, 40)])
+@pytest.mark.parametrize("N,K", [(16, 8), (100, 4104), (2390, 200), (4768, 72), (7130, 328), (9504, 136), (11872, 64), (14240, 192), (18950, 248), (28400, 128), (47200, 40),
+                                 (9500, 1032), (11872, 1032), (14240, 1032), (17000, 1032)])
 def test_plain_and_strided(M, N, K):
     from tpp_pytorch_extension_b200 import _lib
     from tpp_pytorch_extension_b200._C import _fused_llm_infer as F

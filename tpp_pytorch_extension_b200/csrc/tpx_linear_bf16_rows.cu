@@ -247,10 +247,17 @@ static int br_launch_t(const BrParams& p, cudaStream_t st) {
   else return N == 3 ? br_launch<4, 3, MG>(p, st) : N == 4 ? br_launch<4, 4, MG>(p, st) : br_launch<4, 5, MG>(p, st);
 }
 
-// As many tiles per CTA as this kernel streams no slower than the tcgen05 one, which needs no more time for 16 tokens than for one: 40976 x 4096 (18 tiles) at 1 token
-// 56.9 us / 60.0, at 16 61.6 / 60.2; 20608 x 4096 (9) at 16 34.2 / 35.3, at 32 39.2 / 38.4; 14336 x 4096 (7) at 32 28.8 / 31.9.
+// As many tiles per CTA as this kernel streams no slower than the tcgen05 one, which needs no more time for 16 tokens than for one. Chains, us, tcgen05 / here: 1 token 40960 x 4096
+// (18 tiles) 55.9 / 54.1, the longest weights even (24192 x 11584, 11 tiles, 88.4 / 89.3; at 8 tokens 88.6 / 92.3); 16 tokens 20608 x 4096 (9) 32.0 / 30.4, 25600 x 5120 (11) 46.1 / 45.1, but 24192 x 8192 65.1 / 68.9; 32 tokens
+// 16384 x 8192 (7) 54.1 / 52.5, but 16384 x 512 7.4 / 8.2, 11008 x 512 (5) 6.4 / 6.8 (x 1024 17.2 / 9.3), 8192 x 20480 (4) 62.5 / 65.4 (x 14336 47.7 / 43.9). Where the tcgen05
+// kernel has a tile for every SM, so that none is cut, it is the faster one above 8 tokens: 18944 x 3584 at 8, 16 and 32 tokens 23.4 / 22.8, 23.3 / 24.6 and 25.1 / 28.2.
 bool bf_rows_serves(int64_t M, int64_t N, int64_t K, int64_t ldw) {
-  return M <= 32 && (N + 15) / 16 <= (M <= 8 ? 20LL : M <= 16 ? 12LL : 8LL) * sm_count() && 336 * ldw + K < (1ll << 31);
+  const int64_t sms = sm_count(), T = ((N + 15) / 16 + sms - 1) / sms;
+  if (M > 32 || T > 20 || 336 * ldw + K >= (1ll << 31)) return false;
+  if (M <= 8) return true;
+  if ((N + 127) / 128 == sms) return false;
+  if (M <= 16) return T <= 8 || (T <= 12 && K <= 6144);
+  return T <= 3 || (T <= 8 && K <= 16384 && (T <= 4 || K >= 1024));
 }
 
 int bf_rows_run(const BfParams& b, const void* w, const void* x, int64_t M, int64_t N, int64_t K, int64_t ldw, int64_t ldx, cudaStream_t st) {
